@@ -134,7 +134,10 @@ struct TraceTuning {
     int blocks_per_sm = 16;
     int sm_count = 148;
     int shade_shape = 1;  // ris_shade launch shape, 0 .. kShadeShapes - 1 (256 x 2: fastest at 1080p)
-    int shadow_shape = 1; // shadow-BVH walk register budget, 0 .. kShadowShapes - 1: 64 / 80 / 90 registers
+    // shadow-BVH walk register budget, 0 .. kShadowShapes - 1: 64 / 80 / 90 registers. With one ray
+    // in registers the walk fits 64, and 8 resident blocks hide its loads best (1080p terrain
+    // shadow rays 3.47 ms at 64, 3.84 at 80; 56 and 48 registers spill: 3.66, 4.23)
+    int shadow_shape = 0;
 };
 // ris_shade launch shapes: (threads per block, minimum resident blocks per SM)
 // = (256, 1), (256, 2), (128, 3), (128, 4)
@@ -200,13 +203,9 @@ int launch_ris_wavefront(const DeviceScene &s, const CameraD &cam, int frame_ind
                          GBufferView gb, ReservoirView rv, WaveBuffers wb, float4 *color, int trace_level,
                          unsigned *err, cudaStream_t st, const TraceTuning &tune, cudaEvent_t *ev_begin = nullptr,
                          cudaEvent_t *ev_end = nullptr);
-// The same launchers with the closures' texture overrides compiled in
+// The shading launchers with the closures' texture overrides compiled in
 // (wavefront_tex.cu); the ones above leave them out, for scenes without textures.
 namespace textured {
-int launch_shadow_queue(const DeviceScene &s, const float4 *q, const int *count, int *fetch, unsigned char *occ,
-                        const TraceTuning &tune, unsigned *err, cudaStream_t st);
-int launch_wave_trace(const DeviceScene &s, WaveBuffers wb, const TraceTuning &tune, unsigned *err, cudaStream_t st,
-                      cudaEvent_t *ev_begin = nullptr, cudaEvent_t *ev_end = nullptr);
 int launch_winner_visibility(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
                              GBufferView gb, ReservoirView rv, WaveBuffers wb, float4 *color, unsigned *err,
                              cudaStream_t st, const TraceTuning &tune);

@@ -91,6 +91,11 @@ HDR_HD V3 m4f_transform(const float *m, V3 v) {
     const float inv = (w != 0.0f) ? 1.0f / w : 1.0f;
     return V3{inv * x, inv * y, inv * z};
 }
+// The same for a matrix whose last column is (0, 0, 0, 1) and a finite v: w is 1.
+HDR_HD V3 m4f_transform_affine(const float *m, V3 v) {
+    return V3{v.x * m[0] + v.y * m[4] + v.z * m[8] + m[12], v.x * m[1] + v.y * m[5] + v.z * m[9] + m[13],
+              v.x * m[2] + v.y * m[6] + v.z * m[10] + m[14]};
+}
 // GfMatrix4f::TransformDir (upper 3x3, row vector).
 HDR_HD V3 m4f_transform_dir(const float *m, V3 v) {
     return V3{v.x * m[0] + v.y * m[4] + v.z * m[8], v.x * m[1] + v.y * m[5] + v.z * m[9],

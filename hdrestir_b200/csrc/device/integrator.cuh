@@ -97,7 +97,7 @@ struct TracedResults {
     __device__ __forceinline__ bool closest(int slot, V3 o, V3 d, Hit &h, unsigned &) const {
         if (trace_level < (slot > 0 ? kTraceAllBsdfRays : kTraceBounceRay)) return false;
         const float4 r = hits[slot];
-        const HitId id{r.x, fbits(r.y), fbits(r.z), r.w, hit_v[slot]};
+        const HitId id{r.x, fbits(r.y), hit_tri(fbits(r.z)), r.w, hit_v[slot]};
         if (id.inst < 0) return false;
         h = make_hit(*s, o, d, id);
         return true;

@@ -6,13 +6,27 @@
 // IntersectTriangle (bvh.cpp:8-30, restated in tri_test) returns t < limit for
 // it in its instance's space, which is the same arithmetic on the same records
 // whatever tree finds it. The trees only cull, so their box tests are made
-// conservative: the near and far slab distances are computed with the
-// reciprocal direction shrunk and grown by 2^-20 and offset by 2^-20 of the
-// origin term, which covers the rounding of the fused form
+// conservative: bounds are rounded outward on the node's grid, the near and far slab
+// distances are computed with the reciprocal direction shrunk and grown by 2^-20 and
+// offset by 2^-20 of the origin term, which covers the rounding of
 // t = bound * (1/d) - o * (1/d), so a box is never skipped when a ray hits a
 // triangle inside it. (The reference culls with its own rounded slab tests on
 // its own boxes; it can miss a hit that grazes a box face by an ulp, which no
 // tree change reproduces. Such rays are counted by the tests.)
+//
+// What bounds the walk, on the 14.5 M shadow rays of a 1080p terrain frame (1.03 M
+// triangles, 2001 instances; 6.93 ms before, 3.47 ms now):
+//  * L1's data stage. A divergent load takes a pass for nearly every line it touches.
+//    112-byte float nodes in seven 128-bit loads kept the stage 62 % busy next to an issue
+//    rate of 63 % (93 % once the instructions were halved); 64-byte nodes of byte bounds in
+//    two 256-bit loads leave it at 60 %.
+//  * Instructions: 379 warp instructions per ray before, 200 now. The ray's own order of the
+//    children does not shorten a shadow walk (22.9 steps either way), so children are tried as
+//    they stand; entries need no decoding; near and far bounds share the two halves of
+//    packed multiply-adds; three-operand min and max; an end marker instead of a test at
+//    every pop.
+//  * Registers: one ray at a time (the world ray is read again after an instance) fits 64
+//    without spills in the loop, 8 resident blocks of 128 instead of 6.
 #pragma once
 
 #include "gf.cuh"
@@ -20,64 +34,131 @@
 
 namespace hdr {
 
-constexpr int kSh4Tlas = 0, kSh4Blas = 1, kSh4Inst = 2, kSh4Leaf = 3;
 constexpr unsigned kErrShadowStack = 16u;
 
-// A ray prepared for the 4-child box tests.
-struct Sh4Ray {
-    float inx, iny, inz;  // near bounds: 1/d shrunk by 2^-20
-    float ifx, ify, ifz;  // far bounds: 1/d grown by 2^-20
-    float onx, ony, onz;  // near offsets: -o/d, conservatively lowered
-    float ofx, ofy, ofz;  // far offsets: -o/d, conservatively raised
-    int sgn;              // bit k: direction component k is negative (its near bound is the box max)
-};
+// The walk's entry in hand: a child entry of sh4_layout.h, or one of these (their
+// instance bit is set, so one comparison tells a node from everything else).
+constexpr int kSh4World = 0x7ffffffb;  // back from an instance to the world ray
+constexpr int kSh4Hit = 0x7ffffffc;    // shadow walk over: a triangle blocks the ray
+constexpr int kSh4Done = 0x7ffffffd;   // walk over
+constexpr int kSh4Idle = 0x7ffffffe;   // lane without a ray
 
-__device__ __forceinline__ void sh4_axis(float o, float d, float &in, float &iff, float &on, float &of, int &neg) {
-    const float dd = fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d);
-    const float inv = __frcp_rn(dd);  // IEEE reciprocal, rounded to nearest
-    in = inv * (1.0f - 9.5367431640625e-07f);
-    iff = inv * (1.0f + 9.5367431640625e-07f);
-    const float oi = -o * inv;
-    const float e = fabsf(oi) * 9.5367431640625e-07f;
-    on = -o * in - e;
-    of = -o * iff + e;
-    neg = dd < 0.0f ? 1 : 0;
+__device__ __forceinline__ bool sh4_is_node(int e) { return (unsigned)e < (unsigned)kSh4InstBit; }
+__device__ __forceinline__ bool sh4_is_leaf(int e) { return e < 0; }
+__device__ __forceinline__ bool sh4_is_switch(int e) { return e >= kSh4InstBit && e <= kSh4World; }
+__device__ __forceinline__ bool sh4_is_over(int e) { return e == kSh4Hit || e == kSh4Done; }
+
+// Two floats in one 64-bit register: fma.rn.f32x2 and add.rn.f32x2 work on both in one
+// instruction, each half rounded as the scalar form rounds it.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
-
-__device__ __forceinline__ Sh4Ray sh4_ray(V3 o, V3 d) {
-    Sh4Ray r;
-    int nx, ny, nz;
-    sh4_axis(o.x, d.x, r.inx, r.ifx, r.onx, r.ofx, nx);
-    sh4_axis(o.y, d.y, r.iny, r.ify, r.ony, r.ofy, ny);
-    sh4_axis(o.z, d.z, r.inz, r.ifz, r.onz, r.ofz, nz);
-    r.sgn = nx | (ny << 1) | (nz << 2);
+__device__ __forceinline__ void f2_get(F2 v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
 
-// The four child boxes of node `np` against the ray: bit k of the result is set
-// when child k's box overlaps [0, limit] along the ray; tn[k] its entry distance.
-__device__ __forceinline__ unsigned sh4_children(const float4 *np, const Sh4Ray &r, float limit, float tn[4],
-                                                 int4 &code) {
-    const int sx = r.sgn & 1, sy = (r.sgn >> 1) & 1, sz = (r.sgn >> 2) & 1;
-    const float4 nx = __ldg(np + sx), fx = __ldg(np + 1 - sx);
-    const float4 ny = __ldg(np + 2 + sy), fy = __ldg(np + 3 - sy);
-    const float4 nz = __ldg(np + 4 + sz), fz = __ldg(np + 5 - sz);
-    const float4 c = __ldg(np + 6);
-    code = make_int4(__float_as_int(c.x), __float_as_int(c.y), __float_as_int(c.z), __float_as_int(c.w));
-    const float n_x[4] = {nx.x, nx.y, nx.z, nx.w}, f_x[4] = {fx.x, fx.y, fx.z, fx.w};
-    const float n_y[4] = {ny.x, ny.y, ny.z, ny.w}, f_y[4] = {fy.x, fy.y, fy.z, fy.w};
-    const float n_z[4] = {nz.x, nz.y, nz.z, nz.w}, f_z[4] = {fz.x, fz.y, fz.z, fz.w};
-    unsigned mask = 0;
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// A ray prepared for the 4-child box tests: near and far values side by side.
+struct Sh4Axis {
+    F2 inv;         // 1/d shrunk by 2^-20 | grown by 2^-20
+    F2 off;         // -o/d, conservatively lowered | raised
+    unsigned pick;  // byte selector of the near bounds in (minima, maxima): the minima, or the
+                    // maxima where the direction is negative
+};
+struct Sh4Ray {
+    Sh4Axis x, y, z;
+};
+
+__device__ __forceinline__ Sh4Axis sh4_axis(float o, float d) {
+    const float dd = fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d);
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(dd));  // within one unit in the last place
+    const float in = inv * (1.0f - 9.5367431640625e-07f), inf = inv * (1.0f + 9.5367431640625e-07f);
+    const float e = fabsf(o * inv) * 9.5367431640625e-07f;
+    Sh4Axis a;
+    a.inv = f2(in, inf);
+    a.off = f2(-o * in - e, -o * inf + e);
+    a.pick = dd < 0.0f ? 0x7654u : 0x3210u;
+    return a;
+}
+
+__device__ __forceinline__ Sh4Ray sh4_ray(V3 o, V3 d) {
+    return Sh4Ray{sh4_axis(o.x, d.x), sh4_axis(o.y, d.y), sh4_axis(o.z, d.z)};
+}
+
+// max(a, b, c) / min(a, b, c) in one instruction, NaN operands ignored like fmaxf / fminf
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3f(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// 32 bytes in one load (as four 64-bit words: the assembler of CUDA 12.9 crashes on the form
+// with eight 32-bit words in the larger kernels)
+__device__ __forceinline__ void load_256(unsigned long long at, unsigned v[8]) {
+    unsigned long long w[4];
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(at));
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float t0 = fmaxf(fmaxf(__fmaf_rn(n_x[k], r.inx, r.onx), __fmaf_rn(n_y[k], r.iny, r.ony)),
-                               fmaxf(__fmaf_rn(n_z[k], r.inz, r.onz), 0.0f));
-        const float t1 = fminf(fminf(__fmaf_rn(f_x[k], r.ifx, r.ofx), __fmaf_rn(f_y[k], r.ify, r.ofy)),
-                               fminf(__fmaf_rn(f_z[k], r.ifz, r.ofz), limit));
-        tn[k] = t0;
-        mask |= (t0 <= t1 ? 1u : 0u) << k;
+        v[2 * k] = (unsigned)w[k];
+        v[2 * k + 1] = (unsigned)(w[k] >> 32);
     }
-    return mask;
+}
+
+// Entry and exit distances of the four children along one axis: a bound is 1 + byte / 32768
+// (the byte put into a float's mantissa) times scale, plus origin. Near and far go through
+// each instruction together.
+__device__ __forceinline__ void sh4_slabs(unsigned minima, unsigned maxima, unsigned origin, unsigned scale,
+                                          const Sh4Axis &a, float near[4], float far[4]) {
+    const float s = __uint_as_float(scale), o = __uint_as_float(origin);
+    const F2 s2 = f2_mul(f2(s, s), a.inv), o2 = f2_fma(f2(o, o), a.inv, a.off);
+    const unsigned n = __byte_perm(minima, maxima, a.pick), f = __byte_perm(maxima, minima, a.pick);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const unsigned at = 0x7604u | (unsigned)k << 4;
+        const F2 q = f2(__uint_as_float(__byte_perm(n, 0x3f800000u, at)),
+                        __uint_as_float(__byte_perm(f, 0x3f800000u, at)));
+        f2_get(f2_fma(q, s2, o2), near[k], far[k]);
+    }
+}
+
+// The four child boxes of a node against the ray: child k's box overlaps [0, limit]
+// along the ray exactly when t0[k] <= t1[k]; t0[k] is its entry distance.
+__device__ __forceinline__ void sh4_children(const float4 *nodes, int idx, const Sh4Ray &r, float limit, float t0[4],
+                                             float t1[4], int code[4]) {
+    const unsigned long long node = (unsigned long long)nodes + 64ull * (unsigned)idx;
+    const unsigned turn = ((unsigned)idx << 4) & 32u;  // sh4_slot_of
+    unsigned a[8], b[8];
+    load_256(node | turn, a);
+    load_256(node | (turn ^ 32u), b);
+    float nx[4], ny[4], nz[4], fx[4], fy[4], fz[4];
+    sh4_slabs(a[6], a[7], a[0], a[3], r.x, nx, fx);
+    sh4_slabs(b[0], b[1], a[1], a[4], r.y, ny, fy);
+    sh4_slabs(b[2], b[3], a[2], a[5], r.z, nz, fz);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        code[k] = (int)b[4 + k];
+        t0[k] = fmaxf(max3f(nx[k], ny[k], nz[k]), 0.0f);
+        t1[k] = fminf(min3f(fx[k], fy[k], fz[k]), limit);
+    }
 }
 
 // IntersectTriangle (bvh.cpp:8-30) on a tri_geo record, as tri_test.
@@ -100,166 +181,212 @@ __device__ __forceinline__ bool sh4_tri_blocks(V3 o, V3 d, const float4 *g, floa
     return t > 1e-4f && t < limit;
 }
 
+// Where a walk finds its world ray again when it leaves an instance.
+struct Sh4RayValue {
+    V3 o, d;
+    __device__ __forceinline__ void get(V3 &wo, V3 &wd) const { wo = o, wd = d; }
+};
+struct Sh4RayRecord {  // a ray queue entry: origin.xyz, slot | direction.xyz, limit
+    const float4 *at;
+    __device__ __forceinline__ void get(V3 &wo, V3 &wd) const {
+        const float4 a = __ldg(at), b = __ldg(at + 1);
+        wo = V3{a.x, a.y, a.z}, wd = V3{b.x, b.y, b.z};
+    }
+};
 
-// Phases of a shadow walk: the entry in hand is a TLAS or BLAS node, a BLAS
-// leaf's triangles, or an instance to enter; or the walk is over.
-enum : int { kSh4ModeNode = 0, kSh4ModeLeaf = 1, kSh4ModeInst = 2, kSh4ModeDone = 3, kSh4ModeIdle = 4 };
-
-// The walk as a resumable state machine. Entries are (payload << 2) | tag:
-// nodes (TLAS / BLAS node index), instances (instance index) and BLAS leaves
-// ((first triangle << 2) | (count - 1)). The entry in hand is `cur`; its tag
-// sets the mode. A node step tests the node's four child boxes, takes a hit
-// leaf (or else the nearest hit child) into hand and pushes the other hits,
-// the nearest last. Leaf and instance entries are served in their own phases,
-// so the node steps of a warp stay in step.
-template <class Stk>
-struct Shadow4Walk {
-    V3 o, d, oo, od;
-    Sh4Ray wr, br;
-    float limit;
-    int sp, cur, mode;
-    bool blocked;
+// What both walks share: a resumable state machine over one ray at a time, the world
+// ray or, inside an instance, its object-space ray (keeping both cost 19 registers and
+// spills). `cur` is the entry in hand; the caller serves it by kind: a node step tests
+// the node's four child boxes, takes one hit child into hand and pushes the others;
+// leaves and ray switches (into an instance, or back) are served in their own phases,
+// so that the node steps of a warp stay in step.
+template <class Stk, class Src>
+struct Walk4Base {
+    V3 oo, od;
+    Sh4Ray r;
+    int cur;
     Stk stack;
+    Src src;
 
-    __device__ __forceinline__ void take(int e) {
-        cur = e;
-        const int tag = e & 3;
-        mode = e < 0 ? kSh4ModeDone : (tag == kSh4Leaf ? kSh4ModeLeaf : (tag == kSh4Inst ? kSh4ModeInst : kSh4ModeNode));
+    // an end marker stands at the bottom of the stack, so popping needs no test
+    __device__ __forceinline__ void begin(const DeviceScene &s, V3 o, V3 d) {
+        oo = o;
+        od = d;
+        r = sh4_ray(o, d);
+        stack.reset(kSh4Done);
+        cur = s.has_tlas ? 0 : kSh4Done;
     }
-    __device__ __forceinline__ void next() { take(sp > 0 ? stack.get(--sp) : -1); }
+    __device__ __forceinline__ void next() { cur = stack.pop(); }
 
-    __device__ __forceinline__ void start(const DeviceScene &s, V3 ro, V3 rd, float lim) {
-        o = ro;
-        d = rd;
-        oo = ro;
-        od = rd;
+    // the hit children in order: the first in hand, the others pushed so that the next comes out first
+    template <class Hit>
+    __device__ __forceinline__ void take(const int code[4], Hit hit, unsigned &err) {
+        int in_hand = kSh4Done;
+        bool any = false;
+        if (stack.fast(4)) {  // the pushes and the pop stay in the fast part of the stack
+#pragma unroll
+            for (int k = 3; k >= 0; --k) {
+                const bool h = hit(k);
+                stack.push_fast_if(h && any, in_hand);
+                if (h) in_hand = code[k];
+                any = any || h;
+            }
+            cur = any ? in_hand : stack.pop_fast();
+            return;
+        }
+        if (!stack.room(4)) {
+            err |= kErrShadowStack;
+            cur = kSh4Done;
+            return;
+        }
+#pragma unroll
+        for (int k = 3; k >= 0; --k)
+            if (hit(k)) {
+                if (any) stack.push(in_hand);
+                in_hand = code[k];
+                any = true;
+            }
+        cur = any ? in_hand : stack.pop();
+    }
+
+    // enter an instance (returns its index), or go back to the world ray (-1)
+    __device__ __forceinline__ int switch_ray(const DeviceScene &s) {
+        const int e = cur;
+        V3 o, d;
+        src.get(o, d);
+        int ii = -1;
+        if (e != kSh4World) {
+            ii = e & (kSh4InstBit - 1);
+            const float4 *ip = s.instances + 8 * (size_t)ii;
+            const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2), m3 = __ldg(ip + 3);
+            const float inv[16] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w,
+                                   m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z, m3.w};
+            // GfMatrix4f::Transform divides by w; an affine matrix makes it 1 and the division exact
+            if (m0.w == 0.0f && m1.w == 0.0f && m2.w == 0.0f && m3.w == 1.0f)
+                oo = m4f_transform_affine(inv, o);
+            else
+                oo = m4f_transform(inv, o);
+            od = m4f_transform_dir(inv, d);
+            if (!stack.bottom()) stack.push(kSh4World);
+            cur = __ldg(&s.sh4_inst_root[ii]);
+        } else {
+            oo = o;
+            od = d;
+            next();
+        }
+        r = sh4_ray(oo, od);
+        return ii;
+    }
+};
+
+// The shadow walk. The children of a node stand in the order they are tried.
+template <class Stk, class Src>
+struct Shadow4Walk : Walk4Base<Stk, Src> {
+    using B = Walk4Base<Stk, Src>;
+    float limit;
+
+    __device__ __forceinline__ void start(const DeviceScene &s, V3 o, V3 d, float lim) {
         limit = lim;
-        wr = sh4_ray(ro, rd);
-        br = wr;
-        sp = 0;
-        blocked = false;
-        take(s.has_tlas ? ((0 << 2) | kSh4Tlas) : -1);
+        B::begin(s, o, d);
     }
-    __device__ __forceinline__ void finish(bool hit) {
-        blocked = hit;
-        sp = 0;
-        cur = -1;
-        mode = kSh4ModeDone;
-    }
+    __device__ __forceinline__ bool blocked() const { return B::cur == kSh4Hit; }
 
-    // one node entry (mode kSh4ModeNode)
+    // one node entry
     template <class St>
     __device__ __forceinline__ void node_step(const DeviceScene &s, unsigned &err, St &st) {
         st.pop();
-        const int tag = cur & 3, idx = cur >> 2;
-        const bool blas = tag == kSh4Blas;
-        float tn[4];
-        int4 code;
-        const unsigned hits = sh4_children(s.sh4_nodes + 7 * (size_t)idx, blas ? br : wr, limit, tn, code);
-        if (!hits) {
-            next();
-            return;
-        }
-        if (sp + 4 > Stk::kCapacity) {
-            err |= kErrShadowStack;
-            finish(false);
-            return;
-        }
-        const int codes[4] = {code.x, code.y, code.z, code.w};
-        int ent[4];
-        int pick = -1;
-        float t_pick = 3.402823466e+38f;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int c = codes[k];
-            ent[k] = c >= 0 ? ((c << 2) | tag) : (blas ? (((~c) << 2) | kSh4Leaf) : ((((~c) >> 2) << 2) | kSh4Inst));
-            if (!((hits >> k) & 1u)) continue;
-            // a leaf first (its triangles may end the walk), else the nearest child
-            const float key = (c < 0 && blas) ? -1.0f : tn[k];
-            if (key < t_pick) {
-                t_pick = key;
-                pick = k;
-            }
-        }
-        // the other hits, the nearest of them pushed last
-        int second = -1;
-        float t_second = 3.402823466e+38f;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (k != pick && ((hits >> k) & 1u) && tn[k] < t_second) {
-                t_second = tn[k];
-                second = k;
-            }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (k != pick && k != second && ((hits >> k) & 1u)) stack.set(sp++, ent[k]);
-        if (second >= 0) stack.set(sp++, ent[second]);
-        take(ent[pick]);
+        float t0[4], t1[4];
+        int code[4];
+        sh4_children(s.sh4_nodes, B::cur, B::r, limit, t0, t1, code);
+        B::take(code, [&](int k) { return t0[k] <= t1[k]; }, err);
     }
 
-    // a BLAS leaf's triangles (mode kSh4ModeLeaf)
+    // a leaf's triangles
     template <class St>
     __device__ __forceinline__ void leaf(const DeviceScene &s, St &st) {
-        const int p = cur >> 2, first = p >> 2, cnt = (p & 3) + 1;
+        const int p = ~B::cur, first = p >> 2, cnt = (p & 3) + 1;
         st.leaf();
         for (int q = 0; q < cnt; ++q) {
             st.tri();
-            if (sh4_tri_blocks(oo, od, s.sh4_tris + 3 * (size_t)(first + q), limit)) {
-                finish(true);
+            if (sh4_tri_blocks(B::oo, B::od, s.sh4_tris + 3 * (size_t)(first + q), limit)) {
+                B::cur = kSh4Hit;
                 return;
             }
         }
-        next();
-    }
-
-    // enter an instance (mode kSh4ModeInst): its ray, then its BLAS root
-    template <class St>
-    __device__ __forceinline__ void inst(const DeviceScene &s, St &st) {
-        const int ii = cur >> 2;
-        st.leaf();
-        const float4 *ip = s.instances + 8 * (size_t)ii;
-        const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2), m3 = __ldg(ip + 3);
-        const float inv[16] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w,
-                               m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z, m3.w};
-        oo = m4f_transform(inv, o);
-        od = m4f_transform_dir(inv, d);
-        br = sh4_ray(oo, od);
-        take((__ldg(&s.sh4_inst_root[ii]) << 2) | kSh4Blas);
+        B::next();
     }
 
     template <class St>
-    __device__ __forceinline__ void step(const DeviceScene &s, unsigned &err, St &st) {
-        if (mode == kSh4ModeNode)
-            node_step(s, err, st);
-        else if (mode == kSh4ModeLeaf)
-            leaf(s, st);
-        else if (mode == kSh4ModeInst)
-            inst(s, st);
+    __device__ __forceinline__ void switch_ray(const DeviceScene &s, St &st) {
+        if (B::cur != kSh4World) st.leaf();
+        (void)B::switch_ray(s);
     }
 };
 
 // Entries below kShared in this thread's column of a shared-memory array, the
-// rest (up to kSh4Stack) in a per-thread local array.
+// rest (up to kSh4Stack) in a per-thread local array. The stack pointer of the
+// column is its shared-memory address.
 template <int kShared, int kThreads>
 struct Sh4SplitStack {
-    static constexpr int kCapacity = kSh4Stack;
-    int *col;
+    static constexpr unsigned kStride = 4u * kThreads;
+    unsigned base, sp;  // address of entry 0, of the next free entry
     int *deep;
-    __device__ __forceinline__ int get(int k) const { return k < kShared ? col[k * kThreads] : deep[k - kShared]; }
-    __device__ __forceinline__ void set(int k, int v) {
-        if (k < kShared)
-            col[k * kThreads] = v;
-        else
-            deep[k - kShared] = v;
+    __device__ __forceinline__ void bind(int *col, int *deep_entries) {
+        base = (unsigned)__cvta_generic_to_shared(col);
+        sp = base;
+        deep = deep_entries;
+    }
+    __device__ __forceinline__ int depth() const { return (int)((sp - base) / kStride); }
+    __device__ __forceinline__ bool fast(int n) const { return sp <= base + (unsigned)(kShared - n) * kStride; }
+    __device__ __forceinline__ bool room(int n) const { return depth() + n <= kSh4Stack; }
+    __device__ __forceinline__ bool bottom() const { return sp == base + kStride; }
+    __device__ __forceinline__ void push_fast_if(bool want, int v) {
+        asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p st.shared.s32 [%0], %1;\n}" ::"r"(sp), "r"(v),
+                     "r"((int)want));
+        sp += want ? kStride : 0u;
+    }
+    __device__ __forceinline__ int pop_fast() {
+        sp -= kStride;
+        int v;
+        asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(sp));
+        return v;
+    }
+    __device__ __forceinline__ void push(int v) {
+        if (fast(1))
+            push_fast_if(true, v);
+        else {
+            deep[depth() - kShared] = v;
+            sp += kStride;
+        }
+    }
+    __device__ __forceinline__ int pop() {
+        if (fast(0)) return pop_fast();
+        sp -= kStride;
+        return deep[depth() - kShared];
+    }
+    __device__ __forceinline__ void reset(int end) {
+        sp = base;
+        push_fast_if(true, end);
     }
 };
 
 template <class T, int kCap>
 struct Sh4LocalStack {
-    static constexpr int kCapacity = kCap;
     T e[kCap];
-    __device__ __forceinline__ T get(int k) const { return e[k]; }
-    __device__ __forceinline__ void set(int k, T v) { e[k] = v; }
+    int sp;
+    __device__ __forceinline__ bool fast(int n) const { return sp + n <= kCap; }
+    __device__ __forceinline__ bool room(int n) const { return sp + n <= kCap; }
+    __device__ __forceinline__ bool bottom() const { return sp == 1; }
+    __device__ __forceinline__ void push(T v) { e[sp++] = v; }
+    __device__ __forceinline__ T pop() { return e[--sp]; }
+    __device__ __forceinline__ void push_fast_if(bool want, T v) {
+        if (want) push(v);
+    }
+    __device__ __forceinline__ T pop_fast() { return pop(); }
+    __device__ __forceinline__ void reset(T end) {
+        e[0] = end;
+        sp = 1;
+    }
 };
 
 // Closest-hit walk over the same trees (IntersectScene, scene.cpp:409-535), with
@@ -268,159 +395,146 @@ struct Sh4LocalStack {
 // instance's space, and among hits at equal t the smallest (instance position in
 // the reference TLAS's leaf order, triangle index in the reference BLAS order)
 // wins, the hit the reference's left-first walks meet first with their strict
-// `<`. Same phases as the shadow walk.
-template <class Stk>
-struct Closest4Walk {
-    V3 o, d, oo, od;
-    Sh4Ray wr, br;
-    float best_t, best_u, best_v;
-    int best_inst, best_tri, best_rank;
-    int cur_inst, cur_rank;
-    int sp, cur, mode;
-    Stk stack;
+// `<`. The nearest hit child is taken into hand, the others are pushed as they stand
+// (sorting them too saves 1 % of the node steps).
+//
+// second_t is the nearest hit of any other triangle seen. Boxes are culled 2^-18 of
+// the way beyond the closest t, so every triangle hit up to 15 units in the last place
+// (less than 2^-19) beyond it has been tested: bound() is the distance up to which no
+// other hit exists.
+constexpr float kSh4CullPast = 1.0f + 3.814697265625e-06f;
+constexpr int kSh4BoundUlps = 15;
 
-    __device__ __forceinline__ void take(int e) {
-        cur = e;
-        const int tag = e & 3;
-        mode = e < 0 ? kSh4ModeDone : (tag == kSh4Leaf ? kSh4ModeLeaf : (tag == kSh4Inst ? kSh4ModeInst : kSh4ModeNode));
-    }
-    __device__ __forceinline__ void next() { take(sp > 0 ? stack.get(--sp) : -1); }
+template <class Stk, class Src>
+struct Closest4Walk : Walk4Base<Stk, Src> {
+    using B = Walk4Base<Stk, Src>;
+    float best_t, second_t, best_u, best_v;
+    int best_rec;   // triangle record of the hit, -1 = none
+    int best_inst;  // its instance, -1 = the opened one of its mesh
+    int cur_inst;   // the instance the ray is in, -1 = the world
 
-    __device__ __forceinline__ void start(const DeviceScene &s, V3 ro, V3 rd) {
-        o = ro;
-        d = rd;
-        oo = ro;
-        od = rd;
-        wr = sh4_ray(ro, rd);
-        br = wr;
+    __device__ __forceinline__ void start(const DeviceScene &s, V3 o, V3 d) {
         best_t = 1e30f;  // IntersectScene's initial closest distance
+        second_t = 1e30f;
         best_u = best_v = 0.0f;
-        best_inst = best_tri = -1;
-        best_rank = 0x7fffffff;
-        cur_inst = -1;
-        cur_rank = 0x7fffffff;
-        sp = 0;
-        take(s.has_tlas ? ((0 << 2) | kSh4Tlas) : -1);
+        best_rec = best_inst = cur_inst = -1;
+        B::begin(s, o, d);
     }
+    __device__ __forceinline__ bool found() const { return best_rec >= 0; }
+    __device__ __forceinline__ static int rec_inst(const DeviceScene &s, int rec, int inst) {
+        return inst >= 0 ? inst : __ldg(&s.sh4_mesh_world[__float_as_int(__ldg(&s.sh4_tris[3 * (size_t)rec + 2].z))]);
+    }
+    __device__ __forceinline__ static int rec_tri(const DeviceScene &s, int rec) {
+        return __float_as_int(__ldg(&s.sh4_tris[3 * (size_t)rec + 2].y));
+    }
+    __device__ __forceinline__ int hit_inst(const DeviceScene &s) const {
+        return found() ? rec_inst(s, best_rec, best_inst) : -1;
+    }
+    __device__ __forceinline__ int hit_tri(const DeviceScene &s) const { return found() ? rec_tri(s, best_rec) : -1; }
+    // units in the last place of best_t up to which no other hit lies
+    __device__ __forceinline__ int bound_ulps() const {
+        const int u = __float_as_int(second_t) - __float_as_int(best_t);
+        return u < kSh4BoundUlps ? u : kSh4BoundUlps;
+    }
+    __device__ __forceinline__ float bound() const { return __int_as_float(__float_as_int(best_t) + bound_ulps()); }
 
     template <class St>
     __device__ __forceinline__ void node_step(const DeviceScene &s, unsigned &err, St &st) {
         st.pop();
-        const int tag = cur & 3, idx = cur >> 2;
-        const bool blas = tag == kSh4Blas;
-        float tn[4];
-        int4 code;
-        const unsigned hits = sh4_children(s.sh4_nodes + 7 * (size_t)idx, blas ? br : wr, best_t, tn, code);
-        if (!hits) {
-            next();
-            return;
-        }
-        if (sp + 4 > Stk::kCapacity) {
-            err |= kErrShadowStack;
-            sp = 0;
-            take(-1);
-            return;
-        }
-        const int codes[4] = {code.x, code.y, code.z, code.w};
-        int ent[4];
-        int pick = -1, second = -1;
-        float t_pick = 3.402823466e+38f, t_second = 3.402823466e+38f;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int c = codes[k];
-            ent[k] = c >= 0 ? ((c << 2) | tag) : (blas ? (((~c) << 2) | kSh4Leaf) : ((((~c) >> 2) << 2) | kSh4Inst));
-            if (!((hits >> k) & 1u)) continue;
-            if (tn[k] < t_pick) {
-                t_second = t_pick;
-                second = pick;
-                t_pick = tn[k];
-                pick = k;
-            } else if (tn[k] < t_second) {
-                t_second = tn[k];
-                second = k;
-            }
-        }
-        // the nearest in hand, the next nearest pushed last (taken next), the others below it
+        float t0[4], t1[4];
+        int code[4];
+        sh4_children(s.sh4_nodes, B::cur, B::r, best_t * kSh4CullPast, t0, t1, code);
+        // entry distances are >= 0: their bits order like the values; the slot breaks ties
+        unsigned key[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (k != pick && k != second && ((hits >> k) & 1u)) stack.set(sp++, ent[k]);
-        if (second >= 0) stack.set(sp++, ent[second]);
-        take(ent[pick]);
+            key[k] = t0[k] <= t1[k] ? ((__float_as_uint(t0[k]) & ~3u) | (unsigned)k) : 0xffffffffu;
+        const unsigned nearest = umin(umin(key[0], key[1]), umin(key[2], key[3]));
+        const int first = nearest & 3u;
+        // the nearest child moved to the front, the others as they stand
+        const int moved[4] = {first == 0 ? code[0] : (first == 1 ? code[1] : (first == 2 ? code[2] : code[3])),
+                              first == 1 ? code[0] : code[1], first == 2 ? code[0] : code[2],
+                              first == 3 ? code[0] : code[3]};
+        const bool hit0 = key[0] != 0xffffffffu;
+        const bool hits[4] = {nearest != 0xffffffffu, first == 1 ? hit0 : key[1] != 0xffffffffu,
+                              first == 2 ? hit0 : key[2] != 0xffffffffu, first == 3 ? hit0 : key[3] != 0xffffffffu};
+        B::take(moved, [&](int k) { return hits[k]; }, err);
     }
 
     template <class St>
     __device__ __forceinline__ void leaf(const DeviceScene &s, St &st) {
-        const int p = cur >> 2, first = p >> 2, cnt = (p & 3) + 1;
+        const int p = ~B::cur, first = p >> 2, cnt = (p & 3) + 1;
         st.leaf();
         for (int q = 0; q < cnt; ++q) {
             st.tri();
-            const float4 *g = s.sh4_tris + 3 * (size_t)(first + q);
+            const int rec = first + q;
             float t, u, v;
-            if (!tri_test(oo, od, g, t, u, v)) continue;
-            const int tri = __float_as_int(__ldg(&g[2].y));
-            if (t < best_t || (t == best_t && (cur_rank < best_rank || (cur_rank == best_rank && tri < best_tri)))) {
+            if (!tri_test(B::oo, B::od, s.sh4_tris + 3 * (size_t)rec, t, u, v)) continue;
+            bool better = t < best_t;
+            if (t == best_t && found()) {
+                const int ra = __ldg(&s.sh4_inst_rank[rec_inst(s, rec, cur_inst)]);
+                const int rb = __ldg(&s.sh4_inst_rank[rec_inst(s, best_rec, best_inst)]);
+                better = ra < rb || (ra == rb && rec_tri(s, rec) < rec_tri(s, best_rec));
+            }
+            if (better) {
+                second_t = best_t;
                 best_t = t;
                 best_u = u;
                 best_v = v;
+                best_rec = rec;
                 best_inst = cur_inst;
-                best_rank = cur_rank;
-                best_tri = tri;
+            } else {
+                second_t = fminf(second_t, t);
             }
         }
-        next();
+        B::next();
     }
 
     template <class St>
-    __device__ __forceinline__ void inst(const DeviceScene &s, St &st) {
-        const int ii = cur >> 2;
-        st.leaf();
-        const float4 *ip = s.instances + 8 * (size_t)ii;
-        const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2), m3 = __ldg(ip + 3);
-        const float inv[16] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w,
-                               m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z, m3.w};
-        oo = m4f_transform(inv, o);
-        od = m4f_transform_dir(inv, d);
-        br = sh4_ray(oo, od);
-        cur_inst = ii;
-        cur_rank = __ldg(&s.sh4_inst_rank[ii]);
-        take((__ldg(&s.sh4_inst_root[ii]) << 2) | kSh4Blas);
+    __device__ __forceinline__ void switch_ray(const DeviceScene &s, St &st) {
+        if (B::cur != kSh4World) st.leaf();
+        cur_inst = B::switch_ray(s);
     }
-
-    template <class St>
-    __device__ __forceinline__ void step(const DeviceScene &s, unsigned &err, St &st) {
-        if (mode == kSh4ModeNode)
-            node_step(s, err, st);
-        else if (mode == kSh4ModeLeaf)
-            leaf(s, st);
-        else if (mode == kSh4ModeInst)
-            inst(s, st);
-    }
-    __device__ __forceinline__ bool found() const { return best_inst >= 0; }
 };
 
-// One ray's answer (callers outside the wavefront trace kernels).
+// One ray's walk to its end (callers outside the wavefront trace kernels).
+template <class W, class St>
+__device__ __forceinline__ void walk4_ray(const DeviceScene &s, W &w, unsigned &err, St &st) {
+    for (;;) {
+        while (sh4_is_node(w.cur)) w.node_step(s, err, st);
+        if (sh4_is_leaf(w.cur))
+            w.leaf(s, st);
+        else if (sh4_is_switch(w.cur))
+            w.switch_ray(s, st);
+        else
+            return;
+    }
+}
+
 template <class St>
 __device__ inline bool shadow4_ray(const DeviceScene &s, V3 o, V3 d, float limit, unsigned &err, St &st) {
-    Shadow4Walk<Sh4LocalStack<int, kSh4Stack>> w;
+    Shadow4Walk<Sh4LocalStack<int, kSh4Stack>, Sh4RayValue> w;
+    w.src = Sh4RayValue{o, d};
     w.start(s, o, d, limit);
-    while (w.mode != kSh4ModeDone) w.step(s, err, st);
-    return w.blocked;
+    walk4_ray(s, w, err, st);
+    return w.blocked();
 }
 
-}  // namespace hdr
-
-namespace hdr {
-// Closest hit of one ray (callers outside the wavefront trace kernels).
+// Closest hit of one ray; bound: the distance up to which no other hit lies.
 template <class St>
-__device__ inline bool closest4_ray(const DeviceScene &s, V3 o, V3 d, HitId &hit, unsigned &err, St &st) {
-    Closest4Walk<Sh4LocalStack<int, kSh4Stack>> w;
+__device__ inline bool closest4_ray(const DeviceScene &s, V3 o, V3 d, HitId &hit, float &bound, unsigned &err,
+                                    St &st) {
+    Closest4Walk<Sh4LocalStack<int, kSh4Stack>, Sh4RayValue> w;
+    w.src = Sh4RayValue{o, d};
     w.start(s, o, d);
-    while (w.mode != kSh4ModeDone) w.step(s, err, st);
+    walk4_ray(s, w, err, st);
     hit.t = w.best_t;
-    hit.inst = w.best_inst;
-    hit.tri = w.best_tri;
+    hit.inst = w.hit_inst(s);
+    hit.tri = w.hit_tri(s);
     hit.u = w.best_u;
     hit.v = w.best_v;
+    bound = w.bound();
     return w.found();
 }
+
 }  // namespace hdr

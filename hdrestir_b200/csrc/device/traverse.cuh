@@ -61,20 +61,18 @@ struct DeviceScene {
     int has_textures;          // 1: some material has a texture (closures read uv and tangents)
     // shadow-ray BVH (host/shadow_bvh.h): 4-wide SAH trees over the same triangles,
     // walked for "hit nearer than the limit" queries when sh4 is 1
-    const float4 *sh4_nodes;   // 7 per node
+    const float4 *sh4_nodes;   // 8 per node
     const float4 *sh4_tris;    // 3 per triangle (tri_geo records in leaf order)
     const int *sh4_inst_root;  // per instance: its mesh's root node, -1 = no triangles
     const int *sh4_inst_rank;  // per instance: its position in the reference TLAS's leaf order
+    const int *sh4_mesh_world; // per mesh: the instance whose nodes are opened into the top-level tree, -1 = none
     int sh4;                   // 1: shadow queries walk the 4-wide SAH trees
     // closest hits: 0 walk the reference trees; 1 walk the SAH trees (HDR_CTX_SAH_CLOSEST);
     // 2 walk the SAH trees and check each hit against the reference walk (ref_reaches),
     // which then walks the reference trees for the rare ray whose answer it cannot vouch for
     int sh4_closest;
-    // parent links of the reference trees for that check
-    // path records, 2 float4 per node: (box min, parent index bits, -1 at a root), (box max, 0)
-    const float4 *ref_tlas_path;  // per TLAS node
+    // where the check finds a hit's boxes in the reference trees
     const int *ref_inst_leaf;     // per instance: its TLAS leaf
-    const float4 *ref_blas_path;  // per BLAS node of all meshes, mesh-local parents
     const int *ref_tri_leaf;      // per triangle record: its mesh-local leaf
     // This struct's own copy in device memory. Kernels take the scene by value
     // (parameter space); a non-inlined callee gets this pointer instead of the
@@ -196,6 +194,13 @@ struct HitId {
     int tri;   // triangle index local to the instance's mesh
     float u, v;
 };
+
+// The triangle field of a wavefront hit slot: the index, and in the four bits above it
+// (the upload limits a scene to 2^27 triangles) how many units in the last place beyond
+// t the SAH walk found no other hit (Closest4Walk::bound).
+__device__ __forceinline__ int hit_pack(int tri, int bound_ulps) { return tri | (bound_ulps << 27); }
+__device__ __forceinline__ int hit_tri(int packed) { return packed & 0x07ffffff; }
+__device__ __forceinline__ int hit_bound_ulps(int packed) { return packed >> 27; }
 
 // Closest hit (kAnyHit = false), or "closest t < t_limit" test (kAnyHit = true).
 //
@@ -779,50 +784,38 @@ namespace hdr {
 
 // The check of a closest hit found on the 4-wide SAH trees (DeviceScene::sh4_closest
 // == 2). The reference's walk (scene.cpp:414-510, bvh.cpp:243-305) skips a node only
-// when its slab test fails or its entry distance exceeds the running closest t. No
-// triangle lies nearer than the SAH walk's nearest hit t, so that running t never
-// drops below t before the hit's triangle is tested. Hence, if every box on the way
-// from the TLAS root down to the instance's leaf, and from the instance's BLAS root
-// down to the triangle's leaf (object-space ray, BLAS thresholds), passes the
-// reference's slab test with an entry distance no farther than t, the reference walk
-// tests the triangle and takes it: the same IntersectTriangle arithmetic gives the
-// same t, and the SAH walk breaks ties in the reference's walk order. A hit that
-// grazes a box the reference's rounding rejects fails the check.
-__device__ __noinline__ static bool ref_reaches(const DeviceScene *s, V3 o, V3 d, int inst, int tri, float t) {
-    const SlabRay wr = make_slab_ray<false>(o, d);
+// when its slab test fails or its entry distance exceeds the running closest t. The
+// SAH walk reports `bound` (Closest4Walk::bound): no hit of the scene but this one lies
+// in [t, bound), so the running t does not drop below `bound` before the hit's triangle
+// is tested. Hence, if every box on the way from the TLAS root down to the instance's
+// leaf, and from the instance's BLAS root down to the triangle's leaf (object-space
+// ray, BLAS thresholds), passes the reference's slab test with an entry distance no
+// farther than `bound`, the reference walk tests the triangle and takes it: the same
+// IntersectTriangle arithmetic gives the same t, and the SAH walk breaks ties in the
+// reference's walk order. A hit that grazes a box the reference's rounding rejects
+// fails the check.
+//
+// Only the two leaves are tested. Every node's box is the exact union of its
+// children's, and the rounded products (bound - o) * inv are monotone in the bound:
+// an ancestor's per-axis entry is no later and its exit no earlier, an axis below the
+// threshold that holds the origin still holds it, so what the leaf passes every
+// ancestor passes, and enters no later (tests/test_leaf_check.py). Climbing both
+// paths level by level took 0.47 ms of the 12.7 ms of nine dome views at depth 16,
+// and most of a one-ray walk's check.
+__device__ __noinline__ static bool ref_reaches(const DeviceScene *s, V3 o, V3 d, int inst, int tri, float bound) {
     const float4 *ip = s->instances + 8 * (size_t)inst;
+    const int node_base = fbits(__ldg(&ip[4].w)), tri_base = fbits(__ldg(&ip[5].w));
+    const int nt = __ldg(&s->ref_inst_leaf[inst]), nb = __ldg(&s->ref_tri_leaf[tri_base + tri]);
+    if (nt < 0 || nb < 0) return false;  // in no leaf of the reference's trees: its walk decides
+    const float4 *tp = s->tlas_nodes + 2 * (size_t)nt, *bp = s->blas_nodes + 2 * (size_t)(node_base + nb);
+    const float4 tlo = __ldg(tp), thi = __ldg(tp + 1), blo = __ldg(bp), bhi = __ldg(bp + 1);
+    float ta;
+    if (!slab_test(make_slab_ray<false>(o, d), tlo, thi, ta) || ta > bound) return false;
     const float4 m0 = __ldg(ip), m1 = __ldg(ip + 1), m2 = __ldg(ip + 2), m3 = __ldg(ip + 3);
     const float inv[16] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w,
                            m2.x, m2.y, m2.z, m2.w, m3.x, m3.y, m3.z, m3.w};
     const SlabRay br = make_slab_ray<true>(m4f_transform(inv, o), m4f_transform_dir(inv, d));
-    const int node_base = fbits(__ldg(&ip[4].w)), tri_base = fbits(__ldg(&ip[5].w));
-    // The boxes on these paths are reachable ones, so DeviceScene::proper_boxes lets
-    // the walks' regular slab test stand in for the full one, as in the walks.
-    const bool wreg = s->proper_boxes && !wr.any_small, breg = s->proper_boxes && !br.any_small;
-    // Both paths are climbed together, one level of each per iteration: every level
-    // reads one 32-byte record (the box and the link up), and the two records'
-    // loads are issued together so that their latencies overlap. A finished path
-    // re-reads its last record (in bounds) and tests nothing.
-    int nt = __ldg(&s->ref_inst_leaf[inst]), nb = __ldg(&s->ref_tri_leaf[tri_base + tri]);
-    if (nt < 0 || nb < 0) return false;  // in no leaf of the reference's trees: its walk decides
-    int lt = nt, lb = nb;
-    while (nt >= 0 || nb >= 0) {
-        const float4 *tp = s->ref_tlas_path + 2 * (size_t)(nt >= 0 ? nt : lt);
-        const float4 *bp = s->ref_blas_path + 2 * (size_t)(node_base + (nb >= 0 ? nb : lb));
-        const float4 tlo = __ldg(tp), thi = __ldg(tp + 1), blo = __ldg(bp), bhi = __ldg(bp + 1);
-        float ta;
-        if (nt >= 0) {
-            if (!(wreg ? slab_test_regular(wr, tlo, thi, ta) : slab_test(wr, tlo, thi, ta)) || ta > t) return false;
-            lt = nt;
-            nt = __float_as_int(tlo.w);
-        }
-        if (nb >= 0) {
-            if (!(breg ? slab_test_regular(br, blo, bhi, ta) : slab_test(br, blo, bhi, ta)) || ta > t) return false;
-            lb = nb;
-            nb = __float_as_int(blo.w);
-        }
-    }
-    return true;
+    return slab_test(br, blo, bhi, ta) && !(ta > bound);
 }
 
 // The reference walk for a ray whose SAH hit the check could not vouch for.
@@ -847,8 +840,9 @@ __device__ __forceinline__ bool trace_ray(const DeviceScene &s, V3 o, V3 d, floa
                                           unsigned &err) {
     if (!kAnyHit && s.sh4_closest) {
         NoStats ns;
-        const bool found = closest4_ray(s, o, d, hit, err, ns);
-        if (s.sh4_closest == 2 && found && !ref_reaches(s.dev, o, d, hit.inst, hit.tri, hit.t)) {
+        float bound;
+        const bool found = closest4_ray(s, o, d, hit, bound, err, ns);
+        if (s.sh4_closest == 2 && found && !ref_reaches(s.dev, o, d, hit.inst, hit.tri, bound)) {
             const RefClosest r = reference_closest(s.dev, o, d);
             hit = r.hit;
             err |= r.err;

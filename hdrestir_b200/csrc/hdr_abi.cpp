@@ -95,8 +95,9 @@ struct SceneStore {
     // the reference trees' parent links for exact SAH closest hits (closest_mode 2); they
     // describe the uploaded TLAS, so moving instances on the device clears this
     bool ref_links = false;
-    std::vector<int> sh4_inst_root;
-    int sh4_tlas_capacity = 0, sh4_blas_depth = 0;
+    // its host copy, from which hdr_scene_set_instance_transforms rebuilds the top-level tree
+    // (nodes, roots and mesh table; the triangles are dropped after the upload)
+    hdr::ShadowBvh sh4_host;
     // the scene's arrays by DeviceScene field name, for hdr_scene_array
     std::map<std::string, std::pair<const void *, size_t>> arrays;
     // hdr_ris_path_trace_batch's shared ray queues and result slots: one grow-only set per
@@ -638,31 +639,18 @@ namespace {
 // The check's path records: per TLAS node and per BLAS node, 8 floats (32 B, one
 // sector): the node's box min, its parent's index bits (-1 at a root), its box max, 0.
 struct RefLinks {
-    std::vector<float> tlas_path, blas_path;
     std::vector<int> inst_leaf, tri_leaf;
 };
-void set_path_record(std::vector<float> &path, size_t n, const float *rec, int parent) {
-    float *p = &path[8 * n];
-    p[0] = rec[0];
-    p[1] = rec[1];
-    p[2] = rec[2];
-    std::memcpy(&p[3], &parent, sizeof(int));
-    p[4] = rec[4];
-    p[5] = rec[5];
-    p[6] = rec[6];
-    p[7] = 0.0f;
-}
 int float_bits(float v) {
     int i;
     std::memcpy(&i, &v, sizeof(i));
     return i;
 }
-// The TLAS half of the links: a path record per node (n_tlas of the 8-float nodes)
-// and each instance's leaf, from a walk of the tree as it is now. False when the
-// tree does not fit the records or names an instance outside the scene.
+// The TLAS half of the links: each instance's leaf, from a walk of the tree as it is now
+// (n_tlas of the 8-float nodes). False when the tree does not fit them or names an
+// instance outside the scene.
 bool tlas_links(const float *nodes, size_t n_tlas, const int *tlas_inst, size_t n_tlas_inst, int num_instances,
-                std::vector<float> &path, std::vector<int> &inst_leaf) {
-    std::vector<int> parent(n_tlas, -1);
+                std::vector<int> &inst_leaf) {
     inst_leaf.assign((size_t)num_instances, -1);
     std::vector<int> todo{0};
     while (!todo.empty()) {
@@ -673,7 +661,6 @@ bool tlas_links(const float *nodes, size_t n_tlas, const int *tlas_inst, size_t 
         if (left >= 0) {
             for (int ch : {left, left + 1}) {
                 if ((size_t)ch >= n_tlas) return false;
-                parent[(size_t)ch] = n;
                 todo.push_back(ch);
             }
         } else {
@@ -686,8 +673,6 @@ bool tlas_links(const float *nodes, size_t n_tlas, const int *tlas_inst, size_t 
             }
         }
     }
-    path.assign(8 * n_tlas, 0.0f);
-    for (size_t n = 0; n < n_tlas; ++n) set_path_record(path, n, &nodes[8 * n], parent[n]);
     return true;
 }
 // blas_nodes: every mesh's BLAS nodes (8 floats each, the host build's or a copy of the device
@@ -695,11 +680,9 @@ bool tlas_links(const float *nodes, size_t n_tlas, const int *tlas_inst, size_t 
 bool build_ref_links(const hdr::FlatScene &f, const std::vector<float> &blas_nodes, size_t n_tri, RefLinks &L) {
     if (blas_nodes.empty() || f.tlas_nodes.empty() || f.num_instances <= 0) return false;
     const size_t n_tlas = f.tlas_nodes.size() / 8, n_blas = blas_nodes.size() / 8;
-    std::vector<int> blas_parent(n_blas, -1);
     L.tri_leaf.assign(n_tri, -1);
     auto ibits = float_bits;
-    if (!tlas_links(f.tlas_nodes.data(), n_tlas, f.tlas_inst.data(), f.tlas_inst.size(), f.num_instances, L.tlas_path,
-                    L.inst_leaf))
+    if (!tlas_links(f.tlas_nodes.data(), n_tlas, f.tlas_inst.data(), f.tlas_inst.size(), f.num_instances, L.inst_leaf))
         return false;
     std::vector<int> todo;
     std::vector<char> done_mesh(n_blas + 1, 0);
@@ -719,7 +702,6 @@ bool build_ref_links(const hdr::FlatScene &f, const std::vector<float> &blas_nod
             if (left >= 0) {
                 for (int ch : {left, left + 1}) {
                     if ((size_t)node_base + (size_t)ch >= n_blas) return false;
-                    blas_parent[(size_t)node_base + (size_t)ch] = m;
                     todo.push_back(ch);
                 }
             } else {
@@ -732,8 +714,6 @@ bool build_ref_links(const hdr::FlatScene &f, const std::vector<float> &blas_nod
             }
         }
     }
-    L.blas_path.assign(8 * n_blas, 0.0f);
-    for (size_t n = 0; n < n_blas; ++n) set_path_record(L.blas_path, n, &blas_nodes[8 * n], blas_parent[n]);
     return true;
 }
 
@@ -913,10 +893,8 @@ hdr_status hdr_scene_upload(hdr_ctx *c, const hdr_scene_desc *desc) {
         UP(sb.tris, sh4_tris);
         UP(sb.inst_root, sh4_inst_root);
         UP(sb.inst_rank, sh4_inst_rank);
+        UP(sb.mesh_world, sh4_mesh_world);
         store->sh4 = true;
-        store->sh4_inst_root = sb.inst_root;
-        store->sh4_tlas_capacity = sb.tlas_capacity;
-        store->sh4_blas_depth = sb.blas_depth;
         RefLinks links;  // exact closest hits on the SAH trees (closest_mode 2)
         std::vector<float> dev_nodes;  // a device build's BLAS nodes, copied back for the links
         if (device_build && f.num_blas_nodes > 0) {
@@ -927,9 +905,7 @@ hdr_status hdr_scene_upload(hdr_ctx *c, const hdr_scene_desc *desc) {
         }
         if (build_ref_links(f, device_build ? dev_nodes : f.blas_nodes,
                             device_build ? (size_t)f.num_triangles : f.tri_geo.size() / 12, links)) {
-            UP(links.tlas_path, ref_tlas_path);
             UP(links.inst_leaf, ref_inst_leaf);
-            UP(links.blas_path, ref_blas_path);
             UP(links.tri_leaf, ref_tri_leaf);
             store->ref_links = true;
         }
@@ -1004,6 +980,10 @@ hdr_status hdr_scene_upload(hdr_ctx *c, const hdr_scene_desc *desc) {
     }
     s.dev = store->desc_dev + desc_index(s);
     const cudaError_t sync_err = cudaStreamSynchronize(c->stream);
+    if (sb.ok) {
+        std::vector<float>().swap(sb.tris);
+        store->sh4_host = std::move(sb);
+    }
     c->scene_store = store;  // owns the buffers from here on, also on the error path below
     c->scene_bytes_accounted = store->bytes;
     if (sync_err != cudaSuccess) return fail(HDR_ECUDA, "scene upload: %s", cudaGetErrorString(sync_err));
@@ -1502,50 +1482,47 @@ hdr_status hdr_scene_set_instance_transforms(hdr_ctx *c, const float *transforms
     s.proper_boxes = (store->blas_proper && !info[3]) ? 1 : 0;
     s.shallow = (store->max_blas_depth + info[1] + 4 <= hdr::kShallowStack) ? 1 : 0;
     if (store->sh4) {  // the shadow BVH's TLAS over the moved instances' world boxes
-        std::vector<float> b9((size_t)num_instances * 9), b6((size_t)num_instances * 6);
+        std::vector<float> b9((size_t)num_instances * 9), b6((size_t)num_instances * 6),
+            records((size_t)num_instances * 32);
         HDR_CUDA(cudaMemcpyAsync(b9.data(), store->inst_bounds, b9.size() * sizeof(float), cudaMemcpyDeviceToHost,
                                  c->stream));
-        HDR_CUDA(cudaStreamSynchronize(c->stream));
-        for (int i = 0; i < num_instances; ++i)
-            for (int k = 0; k < 6; ++k) b6[6 * (size_t)i + k] = b9[9 * (size_t)i + k];
-        std::vector<float> tlas;
-        int depth = 0;
+        HDR_CUDA(cudaMemcpyAsync(records.data(), s.instances, records.size() * sizeof(float), cudaMemcpyDeviceToHost,
+                                 c->stream));
         // closest-hit tie-breaks follow the rebuilt reference TLAS's instance order
         std::vector<int> tlas_inst((size_t)num_instances), rank;
         HDR_CUDA(cudaMemcpyAsync(tlas_inst.data(), s.tlas_inst, tlas_inst.size() * sizeof(int),
                                  cudaMemcpyDeviceToHost, c->stream));
         HDR_CUDA(cudaStreamSynchronize(c->stream));
+        for (int i = 0; i < num_instances; ++i)
+            for (int k = 0; k < 6; ++k) b6[6 * (size_t)i + k] = b9[9 * (size_t)i + k];
         hdr::shadow_ranks(tlas_inst, num_instances, rank);
-        if (hdr::rebuild_shadow_tlas(b6, store->sh4_inst_root, store->sh4_blas_depth, tlas, store->sh4_tlas_capacity,
-                                     depth)) {
-            HDR_CUDA(cudaMemcpyAsync(const_cast<float4 *>(s.sh4_nodes), tlas.data(), tlas.size() * sizeof(float),
+        hdr::ShadowBvh &sb = store->sh4_host;
+        if (hdr::rebuild_shadow_tlas(b6.data(), records.data(), sb)) {
+            HDR_CUDA(cudaMemcpyAsync(const_cast<float4 *>(s.sh4_nodes), sb.nodes.data(),
+                                     (size_t)sb.tlas_capacity * hdr::kSh4NodeFloats * sizeof(float),
                                      cudaMemcpyHostToDevice, c->stream));
+            HDR_CUDA(cudaMemcpyAsync(const_cast<int *>(s.sh4_mesh_world), sb.mesh_world.data(),
+                                     sb.mesh_world.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
             HDR_CUDA(cudaMemcpyAsync(const_cast<int *>(s.sh4_inst_rank), rank.data(), rank.size() * sizeof(int),
                                      cudaMemcpyHostToDevice, c->stream));
-            HDR_CUDA(cudaStreamSynchronize(c->stream));  // `tlas` and `rank` are host buffers
+            HDR_CUDA(cudaStreamSynchronize(c->stream));  // host buffers
         } else {
             store->sh4 = false;  // too deep for the shadow walk's stack: the reference trees serve shadow rays
         }
     }
-    // the reference TLAS changed on the device: its path records are rebuilt from it (the BLAS
-    // ones still hold); if the new tree does not fit them, closest hits go back to the reference
-    // walk for this scene
+    // the reference TLAS changed on the device: the instances' leaves are found again in it (the
+    // triangles' still hold); if that fails, closest hits go back to the reference walk
     if (store->ref_links && store->sh4) {
-        const size_t n_rec = store->arrays["ref_tlas_path"].second / 32;
-        const size_t n_nodes = std::min(n_rec, (size_t)store->tlas_capacity);
-        std::vector<float> nodes(8 * n_nodes);
+        std::vector<float> nodes(8 * (size_t)store->tlas_capacity);
         std::vector<int> tlas_inst((size_t)num_instances), inst_leaf;
-        std::vector<float> path;
         HDR_CUDA(cudaMemcpyAsync(nodes.data(), s.tlas_nodes, nodes.size() * sizeof(float), cudaMemcpyDeviceToHost,
                                  c->stream));
         HDR_CUDA(cudaMemcpyAsync(tlas_inst.data(), s.tlas_inst, tlas_inst.size() * sizeof(int),
                                  cudaMemcpyDeviceToHost, c->stream));
         HDR_CUDA(cudaStreamSynchronize(c->stream));
-        store->ref_links =
-            tlas_links(nodes.data(), n_nodes, tlas_inst.data(), tlas_inst.size(), num_instances, path, inst_leaf);
+        store->ref_links = tlas_links(nodes.data(), (size_t)store->tlas_capacity, tlas_inst.data(), tlas_inst.size(),
+                                      num_instances, inst_leaf);
         if (store->ref_links) {
-            HDR_CUDA(cudaMemcpyAsync(const_cast<float4 *>(s.ref_tlas_path), path.data(), path.size() * sizeof(float),
-                                     cudaMemcpyHostToDevice, c->stream));
             HDR_CUDA(cudaMemcpyAsync(const_cast<int *>(s.ref_inst_leaf), inst_leaf.data(),
                                      inst_leaf.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
             HDR_CUDA(cudaStreamSynchronize(c->stream));  // host buffers

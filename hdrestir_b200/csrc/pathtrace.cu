@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256) pt_sample_kernel(const __grid_constant__ 
         const float4 ro4 = B.ray_o[i], rd4 = B.ray_d[i];
         const SpectralCtx sc = make_spectral_ctx(ro4.w);
         const float4 hr = B.hits[i];
-        const HitId id{hr.x, __float_as_int(hr.y), __float_as_int(hr.z), hr.w, B.hit_v[i]};
+        const HitId id{hr.x, __float_as_int(hr.y), hit_tri(__float_as_int(hr.z)), hr.w, B.hit_v[i]};
         const V3 ro = v3(ro4), rd = v3(rd4);
         const Hit bh = make_hit(s, ro, rd, id);
         Closure c = get_closure(s, bh);
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) pt_connect_kernel(const __grid_constant__
             cn.has_hit = false;
             if (cn.b.ok) {
                 const float4 hr = B.hits[i];
-                const HitId id{hr.x, __float_as_int(hr.y), __float_as_int(hr.z), hr.w, B.hit_v[i]};
+                const HitId id{hr.x, __float_as_int(hr.y), hit_tri(__float_as_int(hr.z)), hr.w, B.hit_v[i]};
                 if (id.inst >= 0) {
                     cn.hit = make_hit(s, cn.b.origin, cn.b.dir, id);
                     cn.has_hit = true;

@@ -126,7 +126,7 @@ __global__ void trace_stats_kernel(DeviceScene s, const float *rays, const float
         case 2: r = trace_ray_binary<true>(s, o, d, lim, h, e, st) && h.t < lim; break;
         case 3: r = trace_ray_wide<true>(s, o, d, lim, h, e, st) && h.t < lim; break;
         case 4: r = shadow4_ray(s, o, d, lim, e, st); break;
-        default: r = closest4_ray(s, o, d, h, e, st); break;
+        default: { float bound; r = closest4_ray(s, o, d, h, bound, e, st); break; }
     }
     out[k] = make_int4(st.pops, st.leaves, st.tris, r ? 1 : 0);
     if (e) atomicOr(err, e);

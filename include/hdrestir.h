@@ -594,8 +594,8 @@ hdr_status hdr_trace_rays(hdr_ctx *ctx, const float *rays, const float *tmax, in
  * shade_shape: launch shape of the resampling kernel: 0 = 256 threads with the
  * register file of one block per SM, 1 (default) = 256 threads for two blocks,
  * 2 / 3 = 128 threads for three / four blocks (no effect on results).
- * shadow_shape: register budget of the shadow-BVH walk kernel: 0 = 64 registers
- * (8 resident blocks of 128 threads), 1 (default) = 80 (6 blocks), 2 = 90 (5 blocks). */
+ * shadow_shape: register budget of the SAH-tree walk kernels: 0 (default) = 64 registers
+ * (8 resident blocks of 128 threads), 1 = 80 (6 blocks), 2 = 90 (5 blocks). */
 typedef struct hdr_trace_tuning {
     int32_t node_quorum;
     int32_t blocks_per_sm;
