@@ -66,6 +66,7 @@ struct RisParamsD {
     int render_ibl_background;
     float roulette;
     int m_cap;
+    int trace_all;  // HDR_RIS_TRACE_ALL_RAYS
     int spatial_neighbors;
     float spatial_radius;
     ReprojD reproj;
@@ -98,9 +99,13 @@ struct WaveBuffers {
                           // redoes (nullptr exactly when the queue has no entries)
     float4 *hits;         // pixels * n_closest: t, instance bits, triangle bits, u
     float *hit_v;         // pixels * n_closest
-    unsigned char *occ;   // pixels * n_shadow
+    unsigned char *occ;   // n_shadow planes of pixels
+    // n_shadow planes of pixels: each light candidate's resampling weight if its shadow ray is
+    // unoccluded (float with a reservoir, double without; nee_weight_bits)
+    void *nee_weight;
     uint4 *rng_state;     // 3 planes of pixels: stream state at the end of candidate generation
-    unsigned char *done;  // pixels: 1 = no GBuffer hit, colour already written
+                          // (store_stream_from)
+    unsigned char *done;  // pixels: kPixel* bits of wavefront.cu (no GBuffer hit, ...)
     size_t pixels;
     int n_closest, n_shadow;
     // added to the result slots the generate kernel writes into the queues: a
@@ -133,14 +138,14 @@ struct TraceTuning {
     int node_quorum = 12;  // best for the SAH-tree walks (16 for the reference-tree ones)
     int blocks_per_sm = 16;
     int sm_count = 148;
-    int shade_shape = 1;  // ris_shade launch shape, 0 .. kShadeShapes - 1 (256 x 2: fastest at 1080p)
+    int shade_shape = 3;  // ris_resample launch shape, 0 .. kShadeShapes - 1 (128 x 8: fastest at 1080p)
     // shadow-BVH walk register budget, 0 .. kShadowShapes - 1: 64 / 80 / 90 registers. With one ray
     // in registers the walk fits 64, and 8 resident blocks hide its loads best (1080p terrain
     // shadow rays 3.47 ms at 64, 3.84 at 80; 56 and 48 registers spill: 3.66, 4.23)
     int shadow_shape = 0;
 };
-// ris_shade launch shapes: (threads per block, minimum resident blocks per SM)
-// = (256, 1), (256, 2), (128, 3), (128, 4)
+// ris_resample launch shapes: (threads per block, minimum resident blocks per SM)
+// = (256, 2), (256, 4), (128, 5), (128, 8)
 constexpr int kShadeShapes = 4;
 // The trace kernels over the queues of the last ris_generate: closest hits, then
 // shadow queries; with checked SAH closest hits (s.sh4_closest == 2) also the

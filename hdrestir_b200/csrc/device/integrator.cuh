@@ -67,25 +67,67 @@ __device__ __noinline__ static unsigned occluded_call(const DeviceScene *s, V3 o
 // the k-th generated BSDF candidate, shadow slot j the j-th NEE candidate.
 // TraceNow traverses at the call (one thread per pixel); TracedResults reads
 // what the wavefront trace kernels wrote for the pixel's slots.
+//
+// Rays that cannot matter are not cast in either form. A generated BSDF candidate contributes
+// only when its ray meets light geometry or an environment; in a scene with neither it is
+// invalid whatever it hits. Without emission either, the bounce of a path's last vertex weighs
+// 0 whatever it hits (480 x 270 boxes, 16 candidates, depth 4: 7 of 16 rays per vertex, 2.53
+// -> 1.62 ms a frame).
 struct TraceNow {
+    static constexpr bool kNeeWeights = false;
     const DeviceScene *s;
+    bool trace_all;  // cast them all the same
+    // the closest-hit slot of the bounce at the path's last vertex; -1: not cast
+    __device__ __forceinline__ int last_bounce_slot() const {
+        return trace_all || s->bsdf_lights || s->emissive ? 0 : -1;
+    }
     __device__ __forceinline__ bool fresh_bsdf_empty() const { return false; }
     __device__ __forceinline__ bool shadow(int, V3 o, V3 d, float limit, unsigned &err) const {
         return occluded(*s, o, d, limit, err);
     }
-    __device__ __forceinline__ bool closest(int, V3 o, V3 d, Hit &h, unsigned &err) const {
+    __device__ __forceinline__ bool closest(int slot, V3 o, V3 d, Hit &h, unsigned &err) const {
+        if (slot != 0 && (slot < 0 || !(trace_all || s->bsdf_lights))) return false;
         return intersect(*s, o, d, h, err);
     }
     __device__ __forceinline__ bool winner_shadow(V3 o, V3 d, float limit, unsigned &err) const {
         return occluded(*s, o, d, limit, err);
     }
+    template <class T>
+    __device__ __forceinline__ T nee_weight(int) const {
+        return T(0);
+    }
 };
 
+// A candidate's weight is mis * target / pdf; an occluded one has target 0 and so weight 0,
+// except that 0 times an infinite or undefined mis is a NaN, which the reference lets into the
+// reservoir's sum. Such a weight is stored with all its lower bits set and stays when the
+// candidate is occluded; any other NaN is stored with one bit set.
+__device__ __forceinline__ bool nee_weight_stays(float w) { return __float_as_uint(w) == 0x7fffffffu; }
+__device__ __forceinline__ bool nee_weight_stays(double w) {
+    return (unsigned long long)__double_as_longlong(w) == 0x7fffffffffffffffull;
+}
+template <class T>
+__device__ __forceinline__ T nee_weight_bits(double w, bool stays);
+template <>
+__device__ __forceinline__ float nee_weight_bits<float>(double w, bool stays) {
+    return stays ? __uint_as_float(0x7fffffffu) : (isnan((float)w) ? __uint_as_float(0x7fc00000u) : (float)w);
+}
+template <>
+__device__ __forceinline__ double nee_weight_bits<double>(double w, bool stays) {
+    return __longlong_as_double(stays ? 0x7fffffffffffffffll
+                                      : (isnan(w) ? 0x7ff8000000000000ll : __double_as_longlong(w)));
+}
+
 struct TracedResults {
+    static constexpr bool kNeeWeights = true;  // the generate kernel evaluated the light candidates
+    __device__ __forceinline__ int last_bounce_slot() const { return 0; }
     const DeviceScene *s;
     const float4 *hits;        // this pixel's closest-hit slots: t, instance bits, triangle bits, u
     const float *hit_v;        // and v
-    const unsigned char *occ;  // this pixel's shadow slots
+    const unsigned char *occ;  // this pixel's shadow slots, `plane` apart
+    const void *weight;        // and its light candidates' weights (WaveBuffers::nee_weight)
+    size_t plane;
+    bool skip_vis;             // no shadow rays were cast
     int trace_level;           // kTrace*: which closest-hit slots were cast (the others cannot matter)
     float4 *q_winner;          // non-null: the winner's shadow ray is queued (answer fixed up later)
     int *winner_count;
@@ -93,7 +135,16 @@ struct TracedResults {
     // Every generated BSDF candidate is invalid whatever it samples: its ray was
     // not cast because the scene has no light geometry and no environment.
     __device__ __forceinline__ bool fresh_bsdf_empty() const { return trace_level < kTraceAllBsdfRays; }
-    __device__ __forceinline__ bool shadow(int slot, V3, V3, float, unsigned &) const { return occ[slot] != 0; }
+    __device__ __forceinline__ bool shadow(int slot, V3, V3, float, unsigned &) const {
+        return occ[plane * (size_t)slot] != 0;
+    }
+    // the weight of light candidate j, visibility included
+    template <class T>
+    __device__ __forceinline__ T nee_weight(int j) const {
+        const T w = ((const T *)weight)[plane * (size_t)j];
+        if (w == T(0) || nee_weight_stays(w) || skip_vis) return w;  // no ray, or none that counts
+        return occ[plane * (size_t)j] != 0 ? T(0) : w;
+    }
     __device__ __forceinline__ bool closest(int slot, V3 o, V3 d, Hit &h, unsigned &) const {
         if (trace_level < (slot > 0 ? kTraceAllBsdfRays : kTraceBounceRay)) return false;
         const float4 r = hits[slot];
@@ -373,21 +424,47 @@ __device__ inline RisContrib ris_evaluate_light_sample(const DeviceScene &s, con
     return r;
 }
 
-// The shadow ray _evaluateLightSample would cast for a fresh NEE sample, or
-// false when its early-outs (or skipVisibility) mean none is cast.
-__device__ __forceinline__ bool ris_nee_shadow_ray(const DeviceScene &s, const Surface &sf, int li,
-                                                   const LightSampleD &ls, bool skip_vis, V3 &o, V3 &d,
-                                                   float &limit) {
+struct RisNeeRay {  // a light candidate as the generate kernel leaves it
+    bool cast;         // its shadow ray is to be cast
+    V3 o, d;
+    float limit;
+    double weight;     // RISLightCandidate::risWeight if the ray is unoccluded (or not cast)
+    bool stays;        // the weight is a NaN that occlusion does not clear (nee_weight_bits)
+};
+
+// A light candidate's shadow ray and its weight (_generateNEECandidates, :553-589, with
+// _evaluateLightSample, :628-673): the values ris_nee_candidate computes after the trace.
+// A candidate that the early-outs drop weighs 0 whatever its densities are, unless the
+// light's density squared overflows (mis is then undefined): only then are they evaluated.
+__device__ __forceinline__ RisNeeRay ris_nee_ray(const DeviceScene &s, const Surface &sf, int li,
+                                                 const LightSampleD &ls, const RisStrategy &strat,
+                                                 const SpectralCtx &sc) {
+    RisNeeRay r;
     const float n_l = dot(sf.sn, ls.dir);
     const float dist2 = ls.dist * ls.dist;
     const float cos_y = smaxf(0.0f, dot(-ls.dir, ls.normal));
     const float p_nee = pdf_to_solid_angle(ls.pdf, ls.pdf_solid_angle, dist2, smaxf(cos_y, 1e-6f));
     const bool delta = light_is_delta(s, li);
-    if (n_l <= 0.0f || p_nee <= 0.0f || (cos_y <= 0.0f && !delta) || skip_vis) return false;
-    o = sf.hit.position + sf.sn * 1e-4f;
-    d = ls.dir;
-    limit = ls.dist - 1e-3f;
-    return true;
+    const bool dropped = n_l <= 0.0f || p_nee <= 0.0f || (cos_y <= 0.0f && !delta);
+    r.cast = !dropped && !strat.skip_vis;
+    r.o = sf.hit.position + sf.sn * 1e-4f;
+    r.d = ls.dir;
+    r.limit = ls.dist - 1e-3f;
+    r.weight = 0.0;
+    r.stays = false;
+    if (dropped && (delta || !isinf(p_nee * p_nee))) return r;
+    const V3 wo = -sf.ray_d;
+    const float mis = delta ? 1.0f
+                            : power_heuristic3(p_nee, strat.n_nee, 0.0f, strat.n_sky,
+                                               ggx_pdf_f(sf.g, sf.sn, wo, ls.dir), strat.n_bsdf);
+    float target = 0.0f;
+    if (!dropped) {
+        const V3 bval = ggx_eval_f(sf.g, sf.sn, wo, ls.dir);
+        target = spectrum_luminance(light_emission(s, li, ls.color, sc) * rgb_to_spectrum(bval * n_l, sc.up), sc.cie);
+    }
+    r.weight = (double)(mis * target) / ((double)p_nee + 1e-9);
+    r.stays = !isfinite(mis);
+    return r;
 }
 
 // _reEvaluateForTemporalReuse (:675-691)
@@ -459,73 +536,46 @@ struct RisCtx {
     int max_refl, max_refr;
 };
 
-// Candidate j of allCandidates: NEE (sampler), then sky NEE, then BSDF.
-// kFull = false only advances the stream exactly like the full generation.
-// HDR_CANDIDATE_INLINE: how the including kernels take it (a call returns the
+// HDR_CANDIDATE_INLINE: how the including kernels take the candidates (a call returns the
 // candidate through local memory, about 20 stores and loads per candidate).
 #ifndef HDR_CANDIDATE_INLINE
 #define HDR_CANDIDATE_INLINE
 #endif
-template <bool kFull, class RP>
-__device__ HDR_CANDIDATE_INLINE Cand ris_candidate(const RisCtx<RP> &x, int j, MtStream &rng, unsigned &err) {
+// _generateNEECandidates (:553-589), candidate j
+template <class RP>
+__device__ HDR_CANDIDATE_INLINE Cand ris_nee_candidate(const RisCtx<RP> &x, int j, MtStream &rng, unsigned &err) {
     const DeviceScene &s = *x.s;
     const Surface &sf = *x.sf;
     const SpectralCtx &sc = *x.sc;
     Cand c = cand_none();
-    if (j < x.strat.n_nee) {
-        // _generateNEECandidates (:553-589)
-        if (!kFull) {
-            skip_propose_candidate(s, rng);
-            return c;
-        }
-        int li;
-        LightSampleD ls;
-        if (!propose_candidate(s, sf.hit.position, rng, li, ls)) return c;
-        const RisContrib nee = ris_evaluate_light_sample(s, *x.rp, j, sf, li, ls, x.strat.skip_vis, sc, err);
-        const Spec contribution = nee.emission * nee.tmul;
-        const float target = spectrum_luminance(contribution, sc.cie);
-        const float mis = nee.use_mis ? power_heuristic3(nee.p_nee, x.strat.n_nee, 0.0f, x.strat.n_sky, nee.p_bsdf,
-                                                         x.strat.n_bsdf)
-                                      : 1.0f;
-        c.valid = true;
-        c.has_lc = true;
-        c.light = li;
-        c.ls = ls;
-        c.origin = 0;
-        c.tp = contribution;
-        c.ris_weight = (double)(mis * target) / ((double)nee.p_nee + 1e-9);
-        c.target = target;
-        c.vis_tested = nee.vis_tested;
-        return c;
-    }
-    j -= x.strat.n_nee;
-    if (j < x.strat.n_sky) {
-        // sky NEE (:445-475): the environment outside the light sampler is the physical
-        // sky, whose SampleLight is the sun and draws nothing; every sky candidate is
-        // the same sample, so they share one shadow slot (index n_nee of the pixel's)
-        if (!kFull) return c;
-        LightSampleD ls;
-        if (!sky_sun_sample(s, ls)) return c;
-        const int li = sky_light_index(s);
-        const RisContrib nee =
-            ris_evaluate_light_sample(s, *x.rp, x.strat.n_nee, sf, li, ls, x.strat.skip_vis, sc, err);
-        const Spec contribution = nee.emission * nee.tmul;
-        const float target = spectrum_luminance(contribution, sc.cie);
-        const float mis = nee.use_mis ? power_heuristic3(nee.p_nee, x.strat.n_sky, 0.0f, x.strat.n_nee, nee.p_bsdf,
-                                                         x.strat.n_bsdf)
-                                      : 1.0f;
-        c.valid = true;
-        c.has_lc = true;
-        c.light = li;
-        c.ls = ls;
-        c.origin = 1;
-        c.tp = contribution;
-        c.ris_weight = (double)(mis * target) / ((double)nee.p_nee + 1e-9);
-        c.target = target;
-        c.vis_tested = nee.vis_tested;
-        return c;
-    }
-    j -= x.strat.n_sky;
+    int li;
+    LightSampleD ls;
+    if (!propose_candidate(s, sf.hit.position, rng, li, ls)) return c;
+    const RisContrib nee = ris_evaluate_light_sample(s, *x.rp, j, sf, li, ls, x.strat.skip_vis, sc, err);
+    const Spec contribution = nee.emission * nee.tmul;
+    const float target = spectrum_luminance(contribution, sc.cie);
+    const float mis = nee.use_mis ? power_heuristic3(nee.p_nee, x.strat.n_nee, 0.0f, x.strat.n_sky, nee.p_bsdf,
+                                                     x.strat.n_bsdf)
+                                  : 1.0f;
+    c.valid = true;
+    c.has_lc = true;
+    c.light = li;
+    c.ls = ls;
+    c.origin = 0;
+    c.tp = contribution;
+    c.ris_weight = (double)(mis * target) / ((double)nee.p_nee + 1e-9);
+    c.target = target;
+    c.vis_tested = nee.vis_tested;
+    return c;
+}
+
+// BSDF candidate j: the caller's connection first, then the generated ones.
+template <bool kFull, class RP>
+__device__ HDR_CANDIDATE_INLINE Cand ris_bsdf_candidate(const RisCtx<RP> &x, int j, MtStream &rng, unsigned &err) {
+    const DeviceScene &s = *x.s;
+    const Surface &sf = *x.sf;
+    const SpectralCtx &sc = *x.sc;
+    Cand c = cand_none();
     // _generateBSDFSamplingCandidates (:396-551)
     if (x.conn_cand && j == 0) {
         if (!kFull) return c;
@@ -605,6 +655,50 @@ __device__ HDR_CANDIDATE_INLINE Cand ris_candidate(const RisCtx<RP> &x, int j, M
     return c;
 }
 
+// Candidate j of allCandidates: NEE (sampler), then sky NEE, then BSDF.
+// kFull = false only advances the stream exactly like the full generation.
+template <bool kFull, class RP>
+__device__ HDR_CANDIDATE_INLINE Cand ris_candidate(const RisCtx<RP> &x, int j, MtStream &rng, unsigned &err) {
+    const DeviceScene &s = *x.s;
+    const Surface &sf = *x.sf;
+    const SpectralCtx &sc = *x.sc;
+    Cand c = cand_none();
+    if (j < x.strat.n_nee) {
+        if (kFull) return ris_nee_candidate(x, j, rng, err);
+        skip_propose_candidate(s, rng);
+        return c;
+    }
+    j -= x.strat.n_nee;
+    if (j < x.strat.n_sky) {
+        // sky NEE (:445-475): the environment outside the light sampler is the physical
+        // sky, whose SampleLight is the sun and draws nothing; every sky candidate is
+        // the same sample, so they share one shadow slot (index n_nee of the pixel's)
+        if (!kFull) return c;
+        LightSampleD ls;
+        if (!sky_sun_sample(s, ls)) return c;
+        const int li = sky_light_index(s);
+        const RisContrib nee =
+            ris_evaluate_light_sample(s, *x.rp, x.strat.n_nee, sf, li, ls, x.strat.skip_vis, sc, err);
+        const Spec contribution = nee.emission * nee.tmul;
+        const float target = spectrum_luminance(contribution, sc.cie);
+        const float mis = nee.use_mis ? power_heuristic3(nee.p_nee, x.strat.n_sky, 0.0f, x.strat.n_nee, nee.p_bsdf,
+                                                         x.strat.n_bsdf)
+                                      : 1.0f;
+        c.valid = true;
+        c.has_lc = true;
+        c.light = li;
+        c.ls = ls;
+        c.origin = 1;
+        c.tp = contribution;
+        c.ris_weight = (double)(mis * target) / ((double)nee.p_nee + 1e-9);
+        c.target = target;
+        c.vis_tested = nee.vis_tested;
+        return c;
+    }
+    j -= x.strat.n_sky;
+    return ris_bsdf_candidate<kFull>(x, j, rng, err);
+}
+
 struct Reservoir {  // WeightedReservoir<RISLightCandidate>
     Cand chosen;    // chosen.valid == ChosenSample engaged
     float wsum;
@@ -612,11 +706,14 @@ struct Reservoir {  // WeightedReservoir<RISLightCandidate>
     float w;
 };
 
-__device__ __forceinline__ void reservoir_update(Reservoir &r, const Cand &c, float weight, MtStream &rng) {
+// true when the candidate replaced the chosen one
+__device__ __forceinline__ bool reservoir_update(Reservoir &r, const Cand &c, float weight, MtStream &rng) {
     ++r.m;
-    if (weight <= 0.0f) return;
+    if (weight <= 0.0f) return false;
     r.wsum += weight;
-    if (rng.next_float() <= weight / r.wsum) r.chosen = c;
+    if (!(rng.next_float() <= weight / r.wsum)) return false;
+    r.chosen = c;
+    return true;
 }
 
 __device__ __forceinline__ void reservoir_finalize(Reservoir &r, int cpf) {
@@ -675,6 +772,7 @@ struct RisRun {
     bool use_reservoir;
     bool skip_vis;
     int m_cap;       // extension: 0 = unbounded (reference)
+    bool trace_all;  // cast the rays that cannot matter too (one-kernel form)
     ReprojD reproj;  // extension: mode 0 = the reference's same-pixel history
 };
 
@@ -752,12 +850,29 @@ __device__ HDR_BOUNCE_INLINE Spec ris_direct_li(const DeviceScene &s, const RP &
         r.wsum = 0.0f;
         r.m = 0;
         r.w = 0.0f;
-        for (int j = 0; j < n_eval; ++j) {
+        int winner = -1;  // a light candidate chosen by its weight, evaluated once the choice stands
+        // (a stream past draw 311 at the end of generation is replayed candidate by candidate)
+        const bool stored = RP::kNeeWeights && gen_end_state != nullptr;
+        if (stored) {
+            for (int j = 0; j < x.strat.n_nee; ++j) {
+                ++r.m;
+                const float w = rp.template nee_weight<float>(j);
+                if (w <= 0.0f) continue;
+                r.wsum += w;
+                if (upd.next_float() <= w / r.wsum) winner = j;
+            }
+        }
+        MtStream nee_start = rng;
+        if (stored) {
+            if (!skip_fresh) skip_candidates(s, x.strat.n_nee, rng);
+        }
+        for (int j = stored ? x.strat.n_nee : 0; j < n_eval; ++j) {
             const Cand c = ris_candidate<true>(x, j, rng, err);
-            if (c.valid)
-                reservoir_update(r, c, (float)c.ris_weight, upd);
-            else
+            if (c.valid) {
+                if (reservoir_update(r, c, (float)c.ris_weight, upd)) winner = -1;
+            } else {
                 ++r.m;  // CountMiss
+            }
         }
         if (skip_fresh) {
             r.m += x.n_total - n_eval;  // CountMiss of each generated BSDF candidate
@@ -791,9 +906,16 @@ __device__ HDR_BOUNCE_INLINE Spec ris_direct_li(const DeviceScene &s, const RP &
                 r.m += prev.m;
                 if (mw > 0.0f) {
                     r.wsum += mw;
-                    if (rng.next_float() <= mw / r.wsum) r.chosen = prev.chosen;
+                    if (rng.next_float() <= mw / r.wsum) {
+                        r.chosen = prev.chosen;
+                        winner = -1;
+                    }
                 }
             }
+        }
+        if (winner >= 0) {  // the light candidate from its own draws
+            skip_candidates(s, winner, nee_start);
+            r.chosen = ris_nee_candidate(x, winner, nee_start, err);
         }
         reservoir_finalize(r, x.n_total);
         // winner visibility (:309-321)
@@ -816,14 +938,26 @@ __device__ HDR_BOUNCE_INLINE Spec ris_direct_li(const DeviceScene &s, const RP &
     const MtStream start = rng;
     double weights[kMaxPlainRisCandidates];
     double wsum = 0.0;
-    for (int j = 0; j < n_eval; ++j) {
-        const Cand c = ris_candidate<true>(x, j, rng, err);
+    if constexpr (RP::kNeeWeights) {
+        for (int j = 0; j < x.strat.n_nee; ++j) {
+            const double w = rp.template nee_weight<double>(j);
+            if (w > 0.0) wsum += w;
+        }
+        if (!skip_fresh) skip_candidates(s, x.strat.n_nee, rng);
+    }
+    for (int j = RP::kNeeWeights ? x.strat.n_nee : 0; j < n_eval; ++j) {
+        const Cand c = RP::kNeeWeights ? ris_bsdf_candidate<true>(x, j - x.strat.n_nee - x.strat.n_sky, rng, err)
+                                       : ris_candidate<true>(x, j, rng, err);
         const double w = c.valid ? c.ris_weight : 0.0;
         weights[j] = w;
         if (w > 0.0) wsum += w;
     }
-    if (skip_fresh) {  // the generated BSDF candidates weigh nothing; the stream continues after them
-        for (int j = n_eval; j < x.n_total; ++j) weights[j] = 0.0;
+    auto weight_of = [&](int j) -> double {
+        if constexpr (RP::kNeeWeights)
+            if (j < x.strat.n_nee) return rp.template nee_weight<double>(j);
+        return j < n_eval ? weights[j] : 0.0;  // a generated BSDF candidate that is not replayed weighs nothing
+    };
+    if (skip_fresh) {  // the stream continues after the generated BSDF candidates
         uint64_t *const spill = rng.spill;
         rng = *gen_end_state;
         rng.spill = spill;
@@ -832,7 +966,7 @@ __device__ HDR_BOUNCE_INLINE Spec ris_direct_li(const DeviceScene &s, const RP &
     double remaining = (double)rng.next_float() * wsum;
     int chosen = -1;
     for (int j = 0; j < x.n_total; ++j) {
-        const double w = weights[j];
+        const double w = weight_of(j);
         if (w <= 0.0) continue;
         remaining -= w;
         if (remaining <= 0.0) {
@@ -875,7 +1009,7 @@ __device__ Spec path_li_continue(const DeviceScene &s, Spec total, Spec tp, V3 r
                                  BounceState st, const SpectralCtx &sc, MtStream &rng, const PathRun &pr,
                                  const RisRun &ris, const ReservoirView &rv, size_t pixel, int first_bounce,
                                  unsigned &err) {
-    const TraceNow now{&s};
+    const TraceNow now{&s, ris.trace_all};
     for (int bounce = first_bounce; bounce < pr.max_depth; ++bounce) {
         if (!has_next) break;
         const Hit bh = next;
@@ -890,7 +1024,8 @@ __device__ Spec path_li_continue(const DeviceScene &s, Spec total, Spec tp, V3 r
         const bool inside = dot(c.normal, rd) > 0.0f;
         beer_absorption(tp, c, bh.depth, inside, sc);
         const Surface sf = make_surface(s, ro, rd, bh, c, inside);
-        const Connection cn = sample_bounce_with_connection(now, 0, sf, pr.max_refl, pr.max_refr, st, sc, rng, err);
+        const int slot = kRis && bounce + 1 >= pr.max_depth ? now.last_bounce_slot() : 0;
+        const Connection cn = sample_bounce_with_connection(now, slot, sf, pr.max_refl, pr.max_refr, st, sc, rng, err);
         total = total + tp * direct_li<kRis>(s, now, sf, cn.b.ok, cn, sc, rng, false, ris, rv, pixel, nullptr, err);
         if (!cn.b.ok) break;
         tp = tp * cn.b.tmul;
@@ -918,7 +1053,8 @@ __device__ Spec path_li_shaded(const DeviceScene &s, const RP &rp, const Surface
     Spec total = rgb_to_spectrum(sf0.c.emission, sc.up);
     Spec tp = spec(1.0f);
     BounceState st{0, 0};
-    const Connection first = sample_bounce_with_connection(rp, 0, sf0, pr.max_refl, pr.max_refr, st, sc, rng, err);
+    const int slot = kRis && pr.max_depth <= 1 ? rp.last_bounce_slot() : 0;
+    const Connection first = sample_bounce_with_connection(rp, slot, sf0, pr.max_refl, pr.max_refr, st, sc, rng, err);
     total = total + direct_li<kRis>(s, rp, sf0, first.b.ok, first, sc, rng, true, ris, rv, pixel, gen_end_state, err);
     if (!first.b.ok) return total;
     if (kDirectOnly) return total;  // maxDepth 1: the loop below would not run

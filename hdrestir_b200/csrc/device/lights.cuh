@@ -282,6 +282,14 @@ __device__ __forceinline__ void skip_propose_candidate(const DeviceScene &s, MtS
     const int n = light_sample_draws(s, (int)idx);
     for (int k = 0; k < n; ++k) (void)rng.next_raw();
 }
+// The draws of n candidates.
+__device__ __forceinline__ void skip_candidates(const DeviceScene &s, int n, MtStream &rng) {
+    if (s.num_lights <= 0) return;
+    if (s.nee_draws > 0)
+        rng.skip((uint32_t)(n * s.nee_draws));
+    else
+        for (int j = 0; j < n; ++j) skip_propose_candidate(s, rng);
+}
 // UniformLightSampler::EvalPdf: every scene light is in the sampler's set.
 __device__ __forceinline__ float light_select_pdf(const DeviceScene &s) {
     return s.num_lights <= 0 ? 0.0f : 1.0f / (float)s.num_lights;

@@ -80,6 +80,18 @@ struct MtStream {
         new0 = 0;
     }
 
+    // init() for a seed whose word s[156], the only costly one, is known
+    HDR_HD void init_from(uint32_t s, uint64_t s156, uint64_t *spill_buf) {
+        seed = s;
+        spill = spill_buf;
+        k = 0;
+        a = (uint64_t)s;
+        b = mt_seed_step(a, 1);
+        c = s156;
+        d = 0;
+        new0 = 0;
+    }
+
     HDR_HD uint64_t next_raw() {
         uint64_t r;
         if (k < 156) {
@@ -123,6 +135,17 @@ struct MtStream {
     }
 
     HDR_HD float next_float() { return mt_to_float(next_raw()); }
+
+    // n draws without their values
+    HDR_HD void skip(uint32_t n) {
+        for (; n > 0 && k < 155; --n) {
+            a = b;
+            b = mt_seed_step(b, k + 2);
+            c = mt_seed_step(c, k + 157);
+            ++k;
+        }
+        for (; n > 0; --n) (void)next_raw();
+    }
 };
 
 // A stream in three uint4 planes of n entries (entry i): the state of a
@@ -143,6 +166,27 @@ __device__ __forceinline__ MtStream load_stream(const uint4 *st, size_t i, size_
     r.k = w.z;
     r.seed = w.w;
     r.spill = nullptr;
+    return r;
+}
+
+
+// The same with the stream's own start and one draw index of the pixel's: s156 stands in the
+// place of b, which is the step after a, and k0 in the place of the seed, which the pixel and
+// the frame give. (Seeding again takes 155 dependent steps.)
+__device__ __forceinline__ void store_stream_from(uint4 *st, size_t i, size_t n, const MtStream &r, uint64_t s156,
+                                                  uint32_t k0) {
+    MtStream x = r;
+    x.b = s156;
+    x.seed = k0;
+    store_stream(st, i, n, x);
+}
+__device__ __forceinline__ MtStream load_stream_from(const uint4 *st, size_t i, size_t n, uint32_t seed,
+                                                     uint64_t &s156, uint32_t &k0) {
+    MtStream r = load_stream(st, i, n);
+    s156 = r.b;
+    k0 = r.seed;
+    r.b = mt_seed_step(r.a, r.k + 1);
+    r.seed = seed;
     return r;
 }
 

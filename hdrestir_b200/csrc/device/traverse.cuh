@@ -39,6 +39,7 @@ struct DeviceScene {
     int num_instances;
     int num_materials;
     int num_lights;
+    int nee_draws;             // random numbers a proposed light candidate draws, 0 = not the same for all lights
     int env_light;             // the first dome light (the environment unless `sky`), -1 = none
     // PhysicalSky (sky.cuh): the environment when `sky` is 1. Its sun is light index
     // num_lights for reservoirs and the delta-light test, outside the light sampler.
@@ -58,6 +59,8 @@ struct DeviceScene {
     int wide;                  // 1: walk the wide trees, 0: the binary ones (same results)
     int proper_boxes;          // 1: no node box of any tree is empty (min > max on some axis)
     int shallow;               // 1: the binary walk's stack never exceeds kShallowStack entries
+    int bsdf_lights;           // 1: a BSDF ray can meet light: some instance is a light's geometry, or an environment
+    int emissive;              // 1: some material emits
     int has_textures;          // 1: some material has a texture (closures read uv and tangents)
     // shadow-ray BVH (host/shadow_bvh.h): 4-wide SAH trees over the same triangles,
     // walked for "hit nearer than the limit" queries when sh4 is 1

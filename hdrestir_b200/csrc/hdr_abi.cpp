@@ -153,8 +153,6 @@ struct hdr_ctx {
     hdr::DeviceScene scene{};
     bool has_scene = false;
     bool scene_opaque = true;          // every material has opacity >= 0.999 (no stochastic pass-through)
-    bool scene_light_geometry = false; // some instance is a light's geometry (GetLightAtHit can succeed)
-    bool scene_emissive = false;       // some material emits
     // camera of the last RIS frame with HDR_RIS_REPROJECT (its hit points are in "__prev_pos_depth")
     bool reproj_valid = false;
     int reproj_w = 0, reproj_h = 0;
@@ -744,11 +742,13 @@ int closest_mode(uint32_t flags, bool sh4, bool links) {
     return links ? 2 : 0;
 }
 
+// Bytes per light candidate of WaveBuffers::nee_weight.
+size_t nee_weight_size(const hdr_ris_params *p) { return p->use_reservoir ? sizeof(float) : sizeof(double); }
 // Which closest-hit rays the wavefront RIS pass casts (hdr::kTrace*).
 int ris_trace_level(const hdr_ctx *c, const hdr_ris_params *p) {
-    if ((p->flags & HDR_RIS_TRACE_ALL_RAYS) || c->scene_light_geometry || c->scene.env_light >= 0 || c->scene.sky)
+    if ((p->flags & HDR_RIS_TRACE_ALL_RAYS) || c->scene.bsdf_lights)
         return hdr::kTraceAllBsdfRays;
-    return c->scene_emissive ? hdr::kTraceBounceRay : hdr::kTraceNoBsdfRays;
+    return c->scene.emissive ? hdr::kTraceBounceRay : hdr::kTraceNoBsdfRays;
 }
 // Closest-hit slots per pixel of the wavefront RIS queues: only the rays the trace
 // level casts get one (the resampling kernel reads no other slot), so a frame whose
@@ -941,6 +941,17 @@ hdr_status hdr_scene_upload(hdr_ctx *c, const hdr_scene_desc *desc) {
     s.num_materials = f.num_materials;
     s.num_lights = f.num_lights;
     s.env_light = f.env_light;
+    {  // as light_sample_draws: rect, triangle and the environment's dome draw two numbers, others none
+        bool two = true, none = true;
+        for (int i = 0; i < desc->num_lights; ++i) {
+            const int32_t type = desc->lights[i].type;
+            const bool draws = type == HDR_LIGHT_RECT || type == HDR_LIGHT_TRIANGLE ||
+                               (type == HDR_LIGHT_DOME && f.dome_width > 0 && i == f.env_light);
+            two = two && draws;
+            none = none && !draws;
+        }
+        s.nee_draws = two ? 3 : (none ? 1 : 0);
+    }
     s.sky = desc->enable_physical_sky ? 1 : 0;
     s.blackbody = 0;
     for (int i = 0; i < desc->num_lights; ++i) s.blackbody |= desc->lights[i].temperature > 0.0f ? 1 : 0;
@@ -960,6 +971,13 @@ hdr_status hdr_scene_upload(hdr_ctx *c, const hdr_scene_desc *desc) {
     s.proper_boxes = (store->blas_proper && tlas_boxes_proper(f)) ? 1 : 0;
     s.shallow = (f.max_blas_depth + f.max_tlas_depth + 4 <= hdr::kShallowStack) ? 1 : 0;
     s.has_textures = f.textures.empty() ? 0 : 1;
+    s.bsdf_lights = (f.env_light >= 0 || desc->enable_physical_sky) ? 1 : 0;
+    for (int i = 0; i < desc->num_instances; ++i)
+        if (desc->instances[i].light >= 0) s.bsdf_lights = 1;
+    s.emissive = 0;
+    for (int i = 0; i < desc->num_materials; ++i)  // the closure's emission, as the scene builder computes it
+        for (int k = 0; k < 3; ++k)
+            if (!(desc->materials[i].emission_color[k] * desc->materials[i].emission == 0.0f)) s.emissive = 1;
     s.sh4 = store->sh4 ? 1 : 0;
     s.sh4_closest = closest_mode(c->flags, store->sh4, store->ref_links);
     // the descriptor itself, for callees that are not inlined into a kernel
@@ -993,13 +1011,6 @@ hdr_status hdr_scene_upload(hdr_ctx *c, const hdr_scene_desc *desc) {
     c->scene_opaque = true;
     for (int i = 0; i < desc->num_materials; ++i)
         if (!(desc->materials[i].opacity >= 0.999f)) c->scene_opaque = false;
-    c->scene_light_geometry = false;
-    for (int i = 0; i < desc->num_instances; ++i)
-        if (desc->instances[i].light >= 0) c->scene_light_geometry = true;
-    c->scene_emissive = false;
-    for (int i = 0; i < desc->num_materials; ++i)  // the closure's emission, as the scene builder computes it
-        for (int k = 0; k < 3; ++k)
-            if (!(desc->materials[i].emission_color[k] * desc->materials[i].emission == 0.0f)) c->scene_emissive = true;
     return HDR_OK;
 }
 
@@ -1224,6 +1235,7 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
     d.render_ibl_background = p->path.render_ibl_background;
     d.roulette = p->path.roulette_aggressiveness;
     d.m_cap = p->m_cap;
+    d.trace_all = (p->flags & HDR_RIS_TRACE_ALL_RAYS) ? 1 : 0;
     d.spatial_neighbors = p->spatial_neighbors;
     d.spatial_radius = p->spatial_radius;
     hdr::CameraD cd = make_camera(cam);
@@ -1294,6 +1306,9 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         wb.hit_v = (float *)q;
         if ((st = ensure_buffer(c, "__wave_occ", count * wb.n_shadow, &q)) != HDR_OK) return st;
         wb.occ = (unsigned char *)q;
+        if ((st = ensure_scratch(c, "__wave_nee_weight", count * wb.n_shadow * nee_weight_size(p), &q)) != HDR_OK)
+            return st;
+        wb.nee_weight = q;
         if ((st = ensure_buffer(c, "__wave_rng", count * 48, &q)) != HDR_OK) return st;
         wb.rng_state = (uint4 *)q;
         if ((st = ensure_buffer(c, "__wave_done", count, &q)) != HDR_OK) return st;
@@ -1429,8 +1444,6 @@ hdr_status hdr_scene_share(hdr_ctx *dst, hdr_ctx *src) {
     dst->scene.sh4_closest = closest_mode(dst->flags, dst->scene.sh4, dst->scene_store->ref_links);
     dst->scene.dev = dst->scene_store->desc_dev + desc_index(dst->scene);
     dst->scene_opaque = src->scene_opaque;
-    dst->scene_light_geometry = src->scene_light_geometry;
-    dst->scene_emissive = src->scene_emissive;
     dst->has_scene = true;
     dst->have_wave = false;
     return HDR_OK;
@@ -1572,6 +1585,7 @@ struct RisJob {
     int trace_level;
     size_t count;
     int n_closest, n_shadow;
+    size_t weight_bytes;
     uint4 *rng_state;
     unsigned char *done;
 };
@@ -1609,6 +1623,7 @@ hdr_status prepare_ris_job(hdr_ctx *c, const hdr_camera *cam, int32_t frame_inde
     d.render_ibl_background = p->path.render_ibl_background;
     d.roulette = p->path.roulette_aggressiveness;
     d.m_cap = p->m_cap;
+    d.trace_all = (p->flags & HDR_RIS_TRACE_ALL_RAYS) ? 1 : 0;
     d.spatial_neighbors = p->spatial_neighbors;
     d.spatial_radius = p->spatial_radius;
     j.cd = make_camera(cam);
@@ -1616,6 +1631,7 @@ hdr_status prepare_ris_job(hdr_ctx *c, const hdr_camera *cam, int32_t frame_inde
     j.trace_level = ris_trace_level(c, p);
     j.n_closest = closest_slots(j.trace_level, std::max(0, p->candidate_count - n_nee));
     j.n_shadow = n_nee;
+    j.weight_bytes = (j.count * j.n_shadow * nee_weight_size(p) + 15) & ~(size_t)15;
     if ((st = ensure_buffer(c, "__wave_rng", j.count * 48, &q)) != HDR_OK) return st;
     j.rng_state = (uint4 *)q;
     if ((st = ensure_buffer(c, "__wave_done", j.count, &q)) != HDR_OK) return st;
@@ -1665,6 +1681,7 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
     std::vector<RisJob> jobs((size_t)n);
     std::vector<long long> base_c((size_t)n), base_s((size_t)n);
     long long total_c = 0, total_s = 0;
+    size_t total_w = 0;
     hdr_status st;
     for (int32_t i = 0; i < n; ++i) {
         if ((st = prepare_ris_job(ctxs[i], &cams[i], frame_indices[i], &params[i], jobs[(size_t)i])) != HDR_OK)
@@ -1673,6 +1690,7 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
         base_s[(size_t)i] = total_s;
         total_c += (long long)jobs[(size_t)i].count * jobs[(size_t)i].n_closest;
         total_s += (long long)jobs[(size_t)i].count * jobs[(size_t)i].n_shadow;
+        total_w += jobs[(size_t)i].weight_bytes;
     }
     if (total_c >= (1ll << 31) || total_s >= (1ll << 31))
         return fail(HDR_EINVAL, "batch of %lld closest / %lld shadow ray slots exceeds 2^31", total_c, total_s);
@@ -1696,6 +1714,8 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
     all.hit_v = (float *)q;
     if ((st = ensure_batch_scratch(store, "occ", (size_t)total_s, &q, done, lead->stream)) != HDR_OK) return st;
     all.occ = (unsigned char *)q;
+    if ((st = ensure_batch_scratch(store, "nee_weight", total_w, &q, done, lead->stream)) != HDR_OK) return st;
+    char *weights = (char *)q;
     if (!store->batch_done) HDR_CUDA(cudaEventCreateWithFlags(&store->batch_done, cudaEventDisableTiming));
     // the previous batch on this scene (another lead's stream) has finished with the queues
     HDR_CUDA(cudaStreamWaitEvent(lead->stream, store->batch_done, 0));
@@ -1715,6 +1735,8 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
         wb.hits = all.hits + base_c[(size_t)i];
         wb.hit_v = all.hit_v + base_c[(size_t)i];
         wb.occ = all.occ + base_s[(size_t)i];
+        wb.nee_weight = weights;
+        weights += j.weight_bytes;
         wb.rng_state = j.rng_state;
         wb.done = j.done;
         wb.pixels = j.count;

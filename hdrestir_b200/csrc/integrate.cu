@@ -24,7 +24,7 @@ __device__ __forceinline__ void integrate_pixel(const DeviceScene &s, const Came
     const SpectralCtx sc = make_spectral_ctx(rng.next_float());
     Hit h;
     const bool has = load_gbuffer_hit(s, gb, i, h);
-    const TraceNow now{&s};
+    const TraceNow now{&s, ris.trace_all};
     const Spec L = path_li<kRis>(s, now, ray.o, ray.d, has, h, sc, rng, pr, ris, rv, i, nullptr, e);
     V3 rgb = spectrum_to_rgb(L, sc.cie);
     if (cam.p.has_params && cam.p.enable_exposure) rgb = rgb * cam.p.exposure_mult;
@@ -84,6 +84,7 @@ void launch_ris_path_trace(const DeviceScene &s, const CameraD &cam, int frame_i
     ris.use_reservoir = p.use_reservoir != 0;
     ris.skip_vis = p.skip_visibility != 0;
     ris.m_cap = p.m_cap;
+    ris.trace_all = p.trace_all != 0;
     ris.reproj = p.reproj;
     integrate_kernel<true><<<tile_blocks(cam.width, cam.height), 256, 0, st>>>(s, cam, frame_index, pr, ris, gb, res,
                                                                              color, err);

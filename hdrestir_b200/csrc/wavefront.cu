@@ -8,15 +8,17 @@
 //              230-262), and appends the rays those draws define to two
 //              compacted queues: closest-hit (the bounce ray, BSDF candidates)
 //              and shadow (one per NEE candidate that passes the early-outs of
-//              _evaluateLightSample, :628-658). It saves the stream state at the
+//              _evaluateLightSample, :628-658). A light candidate's resampling
+//              weight, should its ray be unoccluded, is computed and stored here,
+//              while its sample is at hand. It saves the stream state at the
 //              end of generation: the reservoir-update numbers start there.
-//   trace    : one thread per queued ray; closest hit or "occluded before the
-//              light" for the ray's slot.
-//   shade    : per pixel, repeats the same draws, reads the slot results instead
-//              of tracing, and runs the reference's resampling, temporal merge and
-//              colour write-back with the saved stream state supplying the
-//              update numbers.
-// The shade kernel checks that its own stream ends where generate's did
+//   trace    : closest hit or "occluded before the light" for the ray's slot (trace.cu).
+//   resample : per pixel, the reference's choice among the stored weights, the
+//              temporal merge and the colour write-back, the saved stream state
+//              supplying the update numbers; the chosen light candidate alone is
+//              evaluated again. Where BSDF rays matter, the general form (shade)
+//              also replays the draws of the BSDF candidates.
+// The general form checks that its own stream ends where generate's did
 // whenever it replays every candidate.
 //
 // Rays whose result cannot reach the image are not queued unless the caller
@@ -25,7 +27,7 @@
 // every such candidate an empty one whatever the ray hits; without emissive
 // materials either, the path's bounce ray cannot change the connection
 // candidate's weight. Generate then only advances the stream past those
-// candidates, and shade counts them as misses and continues from the stream
+// candidates, and resampling counts them as misses and continues from the stream
 // state generate saved.
 // Compiled twice: here (namespace hdr) with closures that leave the texture code
 // out, for scenes without textures, and in wavefront_tex.cu (namespace
@@ -58,11 +60,21 @@ __device__ __forceinline__ int queue_append(int *counter, bool want) {
     return base + __popc(mask & ((1u << lane) - 1u));
 }
 
+// WaveBuffers::done of a pixel
+constexpr int kPixelMiss = 1;     // no GBuffer hit: its colour is written
+constexpr int kPixelConn = 2;     // the path's bounce is a candidate (its pdf is above 0)
+constexpr int kPixelConnNan = 4;  // and its pdf squared overflows: its weight is a NaN
+
 // Kernel parameters of struct type are __grid_constant__: code that takes their
 // address (a reference kept in a struct, a call) reads the parameter space
 // instead of a per-thread copy in local memory (a few hundred bytes written per
 // thread).
-__global__ void __launch_bounds__(256)
+//
+// Shape: 16 light candidates per 1080p terrain pixel, weights included, take 1.64 ms in four
+// blocks of 128 (128 registers, 28 bytes spilled), 1.69 in two of 256, 1.57 in three of 256 (80
+// registers) and 1.66 in four; 512 x 512 boxes with 8 candidates 0.117, 0.120, 0.129, 0.118.
+constexpr int kGenerateThreads = 128;
+__global__ void __launch_bounds__(kGenerateThreads, 4)
     ris_generate_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ CameraD cam, int frame_arg,
                         const __grid_constant__ PathRun pr, const __grid_constant__ RisRun ris,
                         const __grid_constant__ GBufferView gb, const __grid_constant__ WaveBuffers wb, float4 *color,
@@ -70,7 +82,7 @@ __global__ void __launch_bounds__(256)
     uint64_t spill[312];
     MtStream rng;
     PixelStart ps;
-    if (!pixel_start(s, cam, live_frame(cam, frame_arg), gb, rng, spill, ps)) return;
+    if (!pixel_start<kGenerateThreads>(s, cam, live_frame(cam, frame_arg), gb, rng, spill, ps)) return;
     const size_t i = ps.i;
     if (!ps.has_hit) {  // PathIntegrator::Li without a hit: background only, no reservoir access
         V3 rgb = v3s(0.0f);
@@ -78,17 +90,16 @@ __global__ void __launch_bounds__(256)
             rgb = spectrum_to_rgb(rgb_to_spectrum(env_radiance(s, ps.ray.d), ps.sc.up), ps.sc.cie);
         if (cam.p.has_params && cam.p.enable_exposure) rgb = rgb * cam.p.exposure_mult;
         color[i] = make_float4(rgb.x, rgb.y, rgb.z, 1.0f);
-        wb.done[i] = 1;
+        wb.done[i] = kPixelMiss;
         if (wb.nee_light)
             for (int j = 0; j < wb.n_shadow; ++j) wb.nee_light[i * (size_t)wb.n_shadow + j] = -1;
         return;
     }
-    wb.done[i] = 0;
     Closure c = get_closure(s, ps.hit);
     if (!pr.enable_subsurface) c.subsurface = 0.0f;
     const bool inside = dot(c.normal, ps.ray.d) > 0.0f;
     const Surface sf = make_surface(s, ps.ray.o, ps.ray.d, ps.hit, c, inside);
-    const size_t cbase = i * (size_t)wb.n_closest, sbase = i * (size_t)wb.n_shadow;
+    const size_t cbase = i * (size_t)wb.n_closest;
     // the path's bounce ray (_li, path_integrator.cpp:104-111)
     BounceState st{0, 0};
     const Bounce fb = sample_bounce(c, sf.sn, inside, ps.hit.position, ps.ray.d, pr.max_refl, pr.max_refr, st, ps.sc,
@@ -104,30 +115,40 @@ __global__ void __launch_bounds__(256)
     // technique split and NEE candidates (:239-246, :553-589)
     const int N = ris.candidate_count;
     const int n_nee = smaxi(1, N / 2), n_bsdf = smaxi(0, N - n_nee);
+    const bool conn = fb.ok && fb.pdf > 0.0f;
+    wb.done[i] = (unsigned char)((conn ? kPixelConn : 0) | (conn && isinf(fb.pdf * fb.pdf) ? kPixelConnNan : 0));
+    const uint32_t k0 = rng.k;
+    const RisStrategy strat{n_nee, 0, n_bsdf, ris.skip_vis};
     for (int j = 0; j < n_nee; ++j) {
         int li;
         LightSampleD ls;
-        V3 o, d;
-        float lim = 0.0f;
+        RisNeeRay ray;
+        ray.cast = ray.stays = false;
+        ray.weight = 0.0;
         const bool proposed = propose_candidate(s, ps.hit.position, rng, li, ls);
-        if (wb.nee_light) wb.nee_light[sbase + j] = proposed ? li : -1;
-        const bool want = proposed && ris_nee_shadow_ray(s, sf, li, ls, ris.skip_vis, o, d, lim);
-        const int q = queue_append(&wb.counts[1], want);
+        if (wb.nee_light) wb.nee_light[i * (size_t)wb.n_shadow + j] = proposed ? li : -1;
+        if (proposed) ray = ris_nee_ray(s, sf, li, ls, strat, ps.sc);
+        const size_t slot = (size_t)j * wb.pixels + i;
+        if (ris.use_reservoir)
+            ((float *)wb.nee_weight)[slot] = nee_weight_bits<float>(ray.weight, ray.stays);
+        else
+            ((double *)wb.nee_weight)[slot] = nee_weight_bits<double>(ray.weight, ray.stays);
+        const int q = queue_append(&wb.counts[1], ray.cast);
         if (q >= 0) {
             wb.q_shadow[2 * (size_t)q] =
-                make_float4(o.x, o.y, o.z, __int_as_float(wb.slot_base_shadow + (int)(sbase + j)));
-            wb.q_shadow[2 * (size_t)q + 1] = make_float4(d.x, d.y, d.z, lim);
+                make_float4(ray.o.x, ray.o.y, ray.o.z, __int_as_float(wb.slot_base_shadow + (int)slot));
+            wb.q_shadow[2 * (size_t)q + 1] = make_float4(ray.d.x, ray.d.y, ray.d.z, ray.limit);
         }
     }
     // generated BSDF candidates (:442-450)
-    const int n_fresh = n_bsdf - ((fb.ok && fb.pdf > 0.0f) ? 1 : 0);
+    const int n_fresh = n_bsdf - (conn ? 1 : 0);
     if (trace_level < kTraceAllBsdfRays) {  // their rays are not cast: only the stream has to advance
         const BounceDraws bd = bounce_draws_of(c, sf.sn, inside, ps.ray.d, ps.sc);
         for (int k = 0; k < n_fresh; ++k) {
             BounceState st2{0, 0};
             bounce_draws(bd, 1, 1, st2, rng);
         }
-        store_stream(wb.rng_state, i, wb.pixels, rng);
+        store_stream_from(wb.rng_state, i, wb.pixels, rng, ps.s156, k0);
         return;
     }
     for (int k = 0; k < n_fresh; ++k) {
@@ -140,31 +161,205 @@ __global__ void __launch_bounds__(256)
             wb.q_closest[2 * (size_t)q + 1] = make_float4(b.dir.x, b.dir.y, b.dir.z, 0.0f);
         }
     }
-    store_stream(wb.rng_state, i, wb.pixels, rng);
+    store_stream_from(wb.rng_state, i, wb.pixels, rng, ps.s156, k0);
 }
 
-template <int kThreads, int kMinBlocks>
-__global__ void __launch_bounds__(kThreads, kMinBlocks)
-    ris_shade_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ CameraD cam, int frame_arg,
-                     const __grid_constant__ PathRun pr, const __grid_constant__ RisRun ris,
-                     const __grid_constant__ GBufferView gb, const __grid_constant__ ReservoirView rv,
-                     const __grid_constant__ WaveBuffers wb, float4 *color, int trace_level, unsigned *err) {
+__device__ __forceinline__ TracedResults traced_results(const DeviceScene &s, const RisRun &ris, const WaveBuffers &wb,
+                                                        int trace_level, size_t i) {
+    return TracedResults{&s, wb.hits + i * (size_t)wb.n_closest, wb.hit_v + i * (size_t)wb.n_closest, wb.occ + i,
+                         (const char *)wb.nee_weight + i * (ris.use_reservoir ? sizeof(float) : sizeof(double)),
+                         wb.pixels, ris.skip_vis, trace_level, wb.q_winner, wb.counts + 4, (int)i};
+}
+
+// The general form of a pixel's resampling: every candidate that is not a light's is replayed.
+__device__ __forceinline__ void shade_general(const DeviceScene &s, const CameraD &cam, int frame_index,
+                                              const PathRun &pr, const RisRun &ris, const GBufferView &gb,
+                                              const ReservoirView &rv, const WaveBuffers &wb, float4 *color,
+                                              int trace_level, int x, int y, unsigned &e) {
+    const size_t i = (size_t)y * (size_t)cam.width + (size_t)x;
     uint64_t spill[312];
     MtStream rng;
     PixelStart ps;
-    if (!pixel_start<kThreads>(s, cam, live_frame(cam, frame_arg), gb, rng, spill, ps)) return;
-    const size_t i = ps.i;
-    if (wb.done[i]) return;
-    unsigned e = 0;
-    const TracedResults tr{&s, wb.hits + i * (size_t)wb.n_closest, wb.hit_v + i * (size_t)wb.n_closest,
-                           wb.occ + i * (size_t)wb.n_shadow, trace_level, wb.q_winner, wb.counts + 4, (int)i};
-    const MtStream gen_end = load_stream(wb.rng_state, i, wb.pixels);
+    uint32_t k0;
+    const MtStream gen_end =
+        load_stream_from(wb.rng_state, i, wb.pixels, pixel_seed(i, frame_index), ps.s156, k0);
+    ps.i = i;
+    pixel_start_at<true>(s, cam, frame_index, gb, x, y, rng, spill, ps);
+    const TracedResults tr = traced_results(s, ris, wb, trace_level, i);
     // past 311 draws the state lives in local memory only: replay instead
     const MtStream *gen_end_ptr = gen_end.k < 312 ? &gen_end : nullptr;
     // the wavefront form runs only for maxDepth 1 and opaque scenes
     const Spec L =
         path_li<true, TracedResults, true>(s, tr, ps.ray.o, ps.ray.d, true, ps.hit, ps.sc, rng, pr, ris, rv, i, gen_end_ptr, e);
     V3 rgb = spectrum_to_rgb(L, ps.sc.cie);
+    if (cam.p.has_params && cam.p.enable_exposure) rgb = rgb * cam.p.exposure_mult;
+    color[i] = make_float4(rgb.x, rgb.y, rgb.z, 1.0f);
+}
+
+__global__ void __launch_bounds__(256, 2)
+    ris_shade_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ CameraD cam, int frame_arg,
+                     const __grid_constant__ PathRun pr, const __grid_constant__ RisRun ris,
+                     const __grid_constant__ GBufferView gb, const __grid_constant__ ReservoirView rv,
+                     const __grid_constant__ WaveBuffers wb, float4 *color, int trace_level, unsigned *err) {
+    int x, y;
+    if (!tile_pixel(cam.width, cam.height, x, y)) return;
+    if (wb.done[(size_t)y * (size_t)cam.width + (size_t)x] & kPixelMiss) return;
+    unsigned e = 0;
+    shade_general(s, cam, live_frame(cam, frame_arg), pr, ris, gb, rv, wb, color, trace_level, x, y, e);
+    if (e) atomicOr(err, e);
+}
+
+// A light candidate (or a history's sample) as the reservoir holds it: target function and
+// throughput of a sample that is not dropped and not occluded (ris_nee_candidate,
+// _reEvaluateForTemporalReuse :675-691).
+__device__ __forceinline__ Spec light_throughput(const DeviceScene &s, const Surface &sf, int li,
+                                                 const LightSampleD &ls, const SpectralCtx &sc) {
+    const V3 bval = ggx_eval_f(sf.g, sf.sn, -sf.ray_d, ls.dir);
+    return light_emission(s, li, ls.color, sc) * rgb_to_spectrum(bval * dot(sf.sn, ls.dir), sc.up);
+}
+
+// Resampling of a pixel none of whose BSDF rays matter (trace level kTraceNoBsdfRays: no light
+// geometry, no environment, no emission). Its BSDF candidates, the path's bounce among them,
+// weigh 0 and only count, so no bounce is sampled: the light candidates' weights choose, and
+// only the winner is evaluated, from its own draws (found by index: no draw before it is
+// replayed). Evaluating the candidates here, as the general form's kernel did, took 2.15 ms of a
+// 1080p terrain frame, most of it local memory and draws repeated; weights from the generate
+// kernel, where the candidate is in registers anyway, and this kernel take 0.42 ms next to 0.59
+// ms more in generate. More resident warps pay against spills: 0.60 ms at 128 registers, 0.53
+// at 96, 0.43 at 64 in blocks of 256, 0.42 in blocks of 128.
+// ris_direct_li with the loops that cannot matter left out, for frames whose streams
+// stay below draw 312 during generation (launch_ris_shade).
+template <int kThreads, int kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks)
+    ris_resample_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ CameraD cam, int frame_arg,
+                        const __grid_constant__ PathRun pr, const __grid_constant__ RisRun ris,
+                        const __grid_constant__ GBufferView gb, const __grid_constant__ ReservoirView rv,
+                        const __grid_constant__ WaveBuffers wb, float4 *color, unsigned *err) {
+    int x, y;
+    if (!tile_pixel<kThreads>(cam.width, cam.height, x, y)) return;
+    const size_t i = (size_t)y * (size_t)cam.width + (size_t)x;
+    const int done = wb.done[i];
+    if (done & kPixelMiss) return;
+    const int frame_index = live_frame(cam, frame_arg);
+    unsigned e = 0;
+    uint64_t spill[312];
+    PixelStart ps;
+    uint32_t k0;
+    MtStream upd = load_stream_from(wb.rng_state, i, wb.pixels, pixel_seed(i, frame_index), ps.s156, k0);
+    upd.spill = spill;
+    const TracedResults tr = traced_results(s, ris, wb, kTraceNoBsdfRays, i);
+    const int N = ris.candidate_count;
+    const int n_nee = smaxi(1, N / 2), n_bsdf = smaxi(0, N - n_nee), conn = (done & kPixelConn) ? 1 : 0;
+    const int n_total = n_nee + conn + smaxi(0, n_bsdf - conn);
+
+    // the light candidates' choice
+    int winner = -1;
+    float wsum = 0.0f;
+    double wsum_d = 0.0;
+    if (ris.use_reservoir) {
+        for (int j = 0; j < n_nee; ++j) {
+            const float w = tr.nee_weight<float>(j);
+            if (w <= 0.0f) continue;
+            wsum += w;
+            if (upd.next_float() <= w / wsum) winner = j;
+        }
+        if (done & kPixelConnNan) {  // not <= 0: it enters the sum and draws, and is never chosen
+            wsum += __int_as_float(0x7fffffff);
+            (void)upd.next_raw();
+        }
+    } else if (n_total > kMaxPlainRisCandidates) {
+        e |= kErrRisCapacity;
+    } else {
+        for (int j = 0; j < n_nee; ++j) {
+            const double w = tr.nee_weight<double>(j);
+            if (w > 0.0) wsum_d += w;
+        }
+        if (wsum_d > 0.0) {
+            double remaining = (double)upd.next_float() * wsum_d;
+            for (int j = 0; j < n_nee && winner < 0; ++j) {
+                const double w = tr.nee_weight<double>(j);
+                if (w <= 0.0) continue;
+                remaining -= w;
+                if (remaining <= 0.0) winner = j;
+            }
+        }
+    }
+
+    MtStream rng;
+    ps.i = i;
+    pixel_start_at<true>(s, cam, frame_index, gb, x, y, rng, spill, ps);
+    Closure c = get_closure(s, ps.hit);
+    if (!pr.enable_subsurface) c.subsurface = 0.0f;
+    const bool inside = dot(c.normal, ps.ray.d) > 0.0f;
+    Spec beer = spec(1.0f);
+    beer_absorption(beer, c, ps.hit.depth, inside, ps.sc);
+    const Surface sf = make_surface(s, ps.ray.o, ps.ray.d, ps.hit, c, inside);
+    const Spec emitted = rgb_to_spectrum(sf.c.emission, ps.sc.up);
+
+    Reservoir r;
+    r.chosen = cand_none();
+    r.wsum = wsum;
+    r.m = n_total;
+    r.w = 0.0f;
+    if (ris.use_reservoir) {  // temporal reuse (:284-305)
+        Reservoir prev;
+        bool have_prev = true;
+        if (ris.reproj.mode == 0)
+            reservoir_load(rv, i, prev);
+        else
+            have_prev = reprojected_history(ris.reproj, sf.hit.position, prev);
+        if (have_prev && prev.chosen.valid && prev.chosen.has_lc && prev.chosen.target > 0.0f) {
+            const float phat_gen = prev.chosen.target;
+            const Spec reeval = ris_reevaluate(s, sf, prev.chosen.light, prev.chosen.ls, ps.sc);
+            const float phat_curr = spectrum_luminance(reeval, ps.sc.cie);
+            if (ris.m_cap > 0) {  // extension: bound the history (M-cap)
+                const int cap = ris.m_cap * n_total;
+                if (prev.m > cap) {
+                    prev.wsum *= (float)cap / (float)prev.m;
+                    prev.m = cap;
+                }
+            }
+            const float mw = prev.wsum * (phat_curr / phat_gen);
+            r.m += prev.m;  // Merge (:157-166)
+            if (mw > 0.0f) {
+                r.wsum += mw;
+                if (upd.next_float() <= mw / r.wsum) {
+                    r.chosen = prev.chosen;
+                    r.chosen.target = phat_curr;
+                    r.chosen.tp = reeval;
+                    winner = -1;
+                }
+            }
+        }
+    }
+    if (winner >= 0) {
+        rng.skip(k0 - rng.k);
+        skip_candidates(s, winner, rng);
+        Cand &k = r.chosen;
+        k.valid = k.has_lc = propose_candidate(s, ps.hit.position, rng, k.light, k.ls);
+        k.tp = light_throughput(s, sf, k.light, k.ls, ps.sc);
+        k.target = spectrum_luminance(k.tp, ps.sc.cie);
+        k.vis_tested = !ris.skip_vis;
+    }
+    float W = 0.0f;
+    if (ris.use_reservoir)
+        reservoir_finalize(r, n_total);
+    else if (r.chosen.valid)
+        W = (float)(wsum_d / (double)r.chosen.target);
+    if (r.chosen.valid && !r.chosen.vis_tested && r.chosen.has_lc) {  // winner visibility (:309-321)
+        const RisContrib nee =
+            ris_evaluate_light_sample(s, tr, -1, sf, r.chosen.light, r.chosen.ls, false, ps.sc, e);
+        r.chosen.tp = nee.emission * nee.tmul;
+        r.chosen.vis_tested = true;
+    }
+    Spec direct = spec(0.0f);
+    if (ris.use_reservoir) {
+        reservoir_store(rv, i, r);
+        if (r.chosen.valid && !(r.w <= 0.0f)) direct = r.chosen.tp * r.w;
+    } else if (r.chosen.valid) {
+        direct = r.chosen.tp * W;
+    }
+    V3 rgb = spectrum_to_rgb(beer * (emitted + direct), ps.sc.cie);
     if (cam.p.has_params && cam.p.enable_exposure) rgb = rgb * cam.p.exposure_mult;
     color[i] = make_float4(rgb.x, rgb.y, rgb.z, 1.0f);
     if (e) atomicOr(err, e);
@@ -187,6 +382,7 @@ RisRun ris_run(const RisParamsD &p) {
     ris.use_reservoir = p.use_reservoir != 0;
     ris.skip_vis = p.skip_visibility != 0;
     ris.m_cap = p.m_cap;
+    ris.trace_all = p.trace_all != 0;
     ris.reproj = p.reproj;
     return ris;
 }
@@ -195,9 +391,8 @@ RisRun ris_run(const RisParamsD &p) {
 int launch_ris_generate(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
                         GBufferView gb, WaveBuffers wb, float4 *color, int trace_level, unsigned *err,
                         cudaStream_t st) {
-    ris_generate_kernel<<<tile_blocks(cam.width, cam.height), 256, 0, st>>>(s, cam, frame_index, path_run(p),
-                                                                             ris_run(p), gb, wb, color, trace_level,
-                                                                             err);
+    ris_generate_kernel<<<tile_blocks<kGenerateThreads>(cam.width, cam.height), kGenerateThreads, 0, st>>>(
+        s, cam, frame_index, path_run(p), ris_run(p), gb, wb, color, trace_level, err);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
@@ -206,23 +401,22 @@ int launch_ris_shade(const DeviceScene &s, const CameraD &cam, int frame_index, 
                      cudaStream_t st, const TraceTuning &tune) {
     const PathRun pr = path_run(p);
     const RisRun ris = ris_run(p);
-    const int blocks = tile_blocks(cam.width, cam.height);
-    switch (tune.shade_shape) {
-        case 1:
-            ris_shade_kernel<256, 2><<<blocks, 256, 0, st>>>(s, cam, frame_index, pr, ris, gb, rv, wb, color,
-                                                             trace_level, err);
-            break;
-        case 2:
-            ris_shade_kernel<128, 3><<<tile_blocks<128>(cam.width, cam.height), 128, 0, st>>>(
-                s, cam, frame_index, pr, ris, gb, rv, wb, color, trace_level, err);
-            break;
-        case 3:
-            ris_shade_kernel<128, 4><<<tile_blocks<128>(cam.width, cam.height), 128, 0, st>>>(
-                s, cam, frame_index, pr, ris, gb, rv, wb, color, trace_level, err);
-            break;
-        default:
-            ris_shade_kernel<256, 1><<<blocks, 256, 0, st>>>(s, cam, frame_index, pr, ris, gb, rv, wb, color,
-                                                             trace_level, err);
+    // Draws up to the end of generation: pixel and lens 4, wavelengths 1, 3 per light candidate,
+    // at most 5 per bounce. The resampling kernel continues a stream it has not replayed, whose
+    // state travels only below draw 312.
+    const int n_nee = smaxi(1, p.candidate_count / 2), n_bsdf = smaxi(0, p.candidate_count - n_nee);
+    const bool lean = trace_level == kTraceNoBsdfRays && 5 + 3 * n_nee + 5 * (n_bsdf + 1) < 312;
+    if (lean) {
+        const bool wide = tune.shade_shape < 2;  // 256 threads per block, else 128
+        const int blocks = wide ? tile_blocks<256>(cam.width, cam.height) : tile_blocks<128>(cam.width, cam.height);
+        auto k = tune.shade_shape == 0   ? ris_resample_kernel<256, 2>
+                 : tune.shade_shape == 1 ? ris_resample_kernel<256, 4>
+                 : tune.shade_shape == 2 ? ris_resample_kernel<128, 5>
+                                         : ris_resample_kernel<128, 8>;
+        k<<<blocks, wide ? 256 : 128, 0, st>>>(s, cam, frame_index, pr, ris, gb, rv, wb, color, err);
+    } else {
+        ris_shade_kernel<<<tile_blocks(cam.width, cam.height), 256, 0, st>>>(s, cam, frame_index, pr, ris, gb, rv, wb,
+                                                                             color, trace_level, err);
     }
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }

@@ -591,9 +591,9 @@ hdr_status hdr_trace_rays(hdr_ctx *ctx, const float *rays, const float *tmax, in
  * on results). node_quorum: node steps continue while this many lanes of a
  * warp step nodes (1..32); blocks_per_sm: persistent blocks per SM (1..64).
  * trace_ms: device time of the two trace kernels (autotune output).
- * shade_shape: launch shape of the resampling kernel: 0 = 256 threads with the
- * register file of one block per SM, 1 (default) = 256 threads for two blocks,
- * 2 / 3 = 128 threads for three / four blocks (no effect on results).
+ * shade_shape: launch shape of the resampling kernel: 0 / 1 = 256 threads for two / four
+ * resident blocks per SM, 2 / 3 (default) = 128 threads for five / eight (no effect on
+ * results; frames whose BSDF rays matter have one shape).
  * shadow_shape: register budget of the SAH-tree walk kernels: 0 (default) = 64 registers
  * (8 resident blocks of 128 threads), 1 = 80 (6 blocks), 2 = 90 (5 blocks). */
 typedef struct hdr_trace_tuning {
