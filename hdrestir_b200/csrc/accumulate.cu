@@ -10,24 +10,41 @@
 // about its threshold 4 max_n(q) + 0.5 >= 4 lum(p) + 0.5 for every later
 // neighbour p. Such a p would need lum(p) > 4 lum(q') + 0.5 for its clamped
 // neighbour q' as well, which no positive luminance satisfies, so a clamped
-// pixel never changes a neighbour's decision or threshold. An infinite
-// luminance breaks this (its clamp scale is 0 and inf * 0 is NaN, which the
-// neighbour maximum then skips).
+// pixel never changes a neighbour's decision or threshold. Two things break
+// this: an infinite luminance (its clamp scale is 0 and inf * 0 is NaN, which the
+// neighbour maximum then skips), and channels of both signs that all but cancel in
+// the luminance, whose clamped luminance is then rounding error.
 //
-// Parity mode therefore runs the parallel clamp, lets a second pass check on
-// the device whether any pixel's result changes under the in-place order, and
-// hands the frame to `firefly_sequential_kernel` only when one does. That
-// kernel reads the check's flag itself and returns at once when it is clear,
-// so no mode reads anything back to the host or waits for the stream.
+// Parity mode therefore runs the parallel clamp, checks on the device whether any
+// pixel's result changes under the in-place order (only in tiles that hold such a
+// pixel, breaks_order), and hands the frame to
+// `firefly_sequential_kernel` only when one does. That kernel reads the check's flag
+// itself and returns at once when it is clear, so no mode reads anything back to the
+// host or waits for the stream.
+//
+// The clamp, its check and the sum are one pass over the frame (firefly_sum_kernel), the
+// mean a second one: neighbours still read the unclamped colour while the first runs.
+// 96 bytes per pixel in parity mode (the sums go to a scratch plane, so that the exact clamp
+// can still start from the unchanged ones), 80 in shader mode, instead of 128 and 96 in four
+// and two passes: 3840 x 2160 takes 80 + 64 us where the clamp, its check and the sum took
+// 2 x 77 + 79.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 
 #include "device/gf.cuh"
 
 namespace hdr {
 
 __device__ __forceinline__ float lum4(float4 c) { return 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z; }
+
+// Could clamping this pixel change what a later neighbour does? Not with a finite luminance
+// that keeps 12 of its 24 bits when it is taken again from the scaled channels.
+__device__ __forceinline__ bool breaks_order(float4 c, float lum) {
+    const float terms = 0.2126f * fabsf(c.x) + 0.7152f * fabsf(c.y) + 0.0722f * fabsf(c.z);
+    return !(terms <= FLT_MAX) || (lum > 0.5f && terms > 1024.0f * lum);  // below 0.5 nothing is clamped
+}
 
 __device__ __forceinline__ bool same_bits(float4 a, float4 b) {
     return __float_as_int(a.x) == __float_as_int(b.x) && __float_as_int(a.y) == __float_as_int(b.y) &&
@@ -63,18 +80,129 @@ __device__ __forceinline__ float4 firefly_pixel(const float4 *__restrict__ orig,
     return c;
 }
 
-// One firefly pass over the frame: the shader's clamp (prev == nullptr), or
-// the in-place-order check of a clamped plane `prev`, which sets *changed when
-// some pixel's result differs from prev's.
-__global__ void __launch_bounds__(256) firefly_kernel(const float4 *__restrict__ orig, const float4 *prev,
-                                                      float4 *dst, int width, int height, int *changed) {
-    const int x = blockIdx.x * 16 + (threadIdx.x & 15);
-    const int y = blockIdx.y * 16 + (threadIdx.x >> 4);
-    if (x >= width || y >= height) return;
-    const size_t p = (size_t)y * width + x;
-    const float4 c = firefly_pixel(orig, prev, x, y, width, height);
-    if (dst) dst[p] = c;
-    if (changed && prev && !same_bits(c, prev[p])) atomicOr(changed, 1);
+// A tile of kTileW x kTileH pixels per block: a thread has kRows rows of one column, a warp
+// kRows rows. The luminances of the tile and of the two pixels around it are in shared memory: a
+// pixel's neighbours, and theirs for the in-place check, are clamped coordinates of the frame,
+// which stay inside that margin.
+constexpr int kTileW = 32, kTileH = 32, kRows = 4, kMargin = 2;
+constexpr int kTileThreads = kTileW * kTileH / kRows;
+constexpr int kLumW = kTileW + 2 * kMargin, kLumH = kTileH + 2 * kMargin;
+constexpr int kMarginRows = 2 * kMargin * kLumW, kMarginPixels = kMarginRows + 2 * kMargin * kTileH;
+
+// Tile coordinates (from lum[0]) of pixel m of the margin: the rows above and below, then the sides.
+__device__ __forceinline__ void margin_pixel(int m, int &lx, int &ly) {
+    if (m < kMarginRows) {
+        ly = m / kLumW;
+        lx = m - ly * kLumW;
+        if (ly >= kMargin) ly += kTileH;
+    } else {
+        const int k = m - kMarginRows;
+        ly = kMargin + k / (2 * kMargin);
+        lx = k % (2 * kMargin);
+        if (lx >= kMargin) lx += kTileW;
+    }
+}
+
+struct LumTile {
+    const float *lum;
+    int x0, y0, width, height;  // frame coordinates of lum[0]; the frame
+    __device__ __forceinline__ float at(int x, int y) const {
+        return lum[(sclampi(y, 0, height - 1) - y0) * kLumW + (sclampi(x, 0, width - 1) - x0)];
+    }
+    __device__ __forceinline__ float threshold(int x, int y) const {
+        float max_n = 0.0f;
+        for (int dy = -1; dy <= 1; ++dy)
+            for (int dx = -1; dx <= 1; ++dx)
+                if (dx != 0 || dy != 0) max_n = smaxf(max_n, at(x + dx, y + dy));
+        return max_n * 4.0f + 0.5f;
+    }
+};
+
+__device__ __forceinline__ float4 firefly_clamp(float4 c, float lum, float thr) {
+    if (lum > thr && lum > 0.0f) {
+        const float scale = thr / lum;
+        c.x *= scale;
+        c.y *= scale;
+        c.z *= scale;
+    }
+    return c;
+}
+
+// sums = accum + clamped colour for the frame (sums may be accum itself when nothing needs the
+// old sums: kParity false). kParity: *changed is set when some pixel's clamp would come out
+// differently with its earlier neighbours already clamped. Bound by memory: all of a thread's
+// loads are issued before the first luminance, and a column's maxima of three are shared by the
+// rows above and below (a maximum from 0 up that skips NaN has no order). 3840 x 2160: 80 us for
+// 398 MB; with the colours read a second time after the luminances, eight loads for each
+// threshold and a thread's rows eight apart it took 112.
+template <bool kParity>
+__global__ void __launch_bounds__(kTileThreads)
+    firefly_sum_kernel(const float4 *__restrict__ color, const float4 *accum, float4 *sums, int width, int height,
+                       int *changed) {
+    __shared__ float lum[kLumH * kLumW];
+    const int tiles_x = (width + kTileW - 1) / kTileW;
+    const int tx = (int)(blockIdx.x % (unsigned)tiles_x) * kTileW, ty = (int)(blockIdx.x / (unsigned)tiles_x) * kTileH;
+    const int t = threadIdx.x, x = tx + t % kTileW, y0 = ty + t / kTileW * kRows;
+    float4 c[kRows], a[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        c[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (x < width && y0 + r < height) {
+            c[r] = color[(size_t)(y0 + r) * width + x];
+            a[r] = accum[(size_t)(y0 + r) * width + x];
+        }
+    }
+    bool odd = false;
+    for (int m = t; m < kMarginPixels; m += kTileThreads) {
+        int lx, ly;
+        margin_pixel(m, lx, ly);
+        const int mx = tx - kMargin + lx, my = ty - kMargin + ly;
+        float l = 0.0f;
+        if (mx >= 0 && my >= 0 && mx < width && my < height) {
+            const float4 v = color[(size_t)my * width + mx];
+            l = lum4(v);
+            if (kParity) odd |= breaks_order(v, l);
+        }
+        lum[ly * kLumW + lx] = l;
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        const float l = lum4(c[r]);
+        lum[(y0 - ty + r + kMargin) * kLumW + kMargin + t % kTileW] = l;
+        if (kParity) odd |= breaks_order(c[r], l);
+    }
+    const bool check = kParity ? __syncthreads_or(odd) : (__syncthreads(), false);
+    if (x >= width || y0 >= height) return;
+    const LumTile tile{lum, tx - kMargin, ty - kMargin, width, height};
+    float side[kRows + 2], mid[kRows + 2];  // rows y0 - 1 .. y0 + kRows: the columns beside x; x
+#pragma unroll
+    for (int r = 0; r < kRows + 2; ++r) {
+        const int yr = smini(y0 + r - 1, height);  // rows past the frame's edge repeat it (at())
+        side[r] = smaxf(smaxf(0.0f, tile.at(x - 1, yr)), tile.at(x + 1, yr));
+        mid[r] = tile.at(x, yr);
+    }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        if (y0 + r >= height) break;
+        const float sides = smaxf(smaxf(side[r], side[r + 1]), side[r + 2]);
+        const float thr = smaxf(smaxf(sides, mid[r]), mid[r + 2]) * 4.0f + 0.5f;
+        const float4 k = firefly_clamp(c[r], lum4(c[r]), thr);
+        const size_t p = (size_t)(y0 + r) * width + x;
+        if (check) {  // ApplyFireflySuppression's body with the earlier neighbours clamped
+            float max_n = 0.0f;
+            for (int dy = -1; dy <= 1; ++dy)
+                for (int dx = -1; dx <= 1; ++dx) {
+                    if (dx == 0 && dy == 0) continue;
+                    const int nx = sclampi(x + dx, 0, width - 1), ny = sclampi(y0 + r + dy, 0, height - 1);
+                    const size_t q = (size_t)ny * width + nx;
+                    float4 v = color[q];
+                    if (q < p) v = firefly_clamp(v, lum4(v), tile.threshold(nx, ny));
+                    max_n = smaxf(max_n, lum4(v));
+                }
+            if (!same_bits(firefly_clamp(c[r], lum4(c[r]), max_n * 4.0f + 0.5f), k)) atomicOr(changed, 1);
+        }
+        sums[p] = make_float4(a[r].x + k.x, a[r].y + k.y, a[r].z + k.z, a[r].w + k.w);
+    }
 }
 
 // The row-major in-place clamp, exactly, in one block, run only when the check
@@ -85,7 +213,9 @@ __global__ void __launch_bounds__(256) firefly_kernel(const float4 *__restrict__
 // parallel from the final values of earlier ones (in `plane`) and the
 // unclamped values of later ones (in `orig`), and meets at a barrier before the
 // next diagonal. Bounded: w + 2h - 2 steps, each at most min(h, w/2 + 1) pixels.
-__global__ void __launch_bounds__(1024) firefly_sequential_kernel(const float4 *__restrict__ orig, float4 *plane,
+// The sums are then taken again from the unchanged accum.
+__global__ void __launch_bounds__(1024) firefly_sequential_kernel(const float4 *__restrict__ orig,
+                                                                  const float4 *__restrict__ accum, float4 *plane,
                                                                   int width, int height, int *changed) {
     __shared__ int run;
     if (threadIdx.x == 0) run = *(volatile int *)changed;
@@ -102,10 +232,28 @@ __global__ void __launch_bounds__(1024) firefly_sequential_kernel(const float4 *
         }
         __syncthreads();
     }
+    for (size_t p = threadIdx.x; p < (size_t)width * height; p += blockDim.x) {
+        const float4 c = plane[p], a = accum[p];
+        plane[p] = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, a.w + c.w);
+    }
 }
 
-__global__ void __launch_bounds__(256) accumulate_kernel(const float4 *__restrict__ in, float4 *__restrict__ accum,
-                                                         float4 *__restrict__ out, size_t count, float inv_n,
+// The mean, and the sums in their place (sums may be accum itself: kCopy false). From the last
+// pixel down: the sums written last are still in L2.
+template <bool kCopy>
+__global__ void __launch_bounds__(256) mean_kernel(const float4 *__restrict__ sums, float4 *accum,
+                                                   float4 *__restrict__ out, size_t count, float inv_n,
+                                                   const int *frame_slot) {
+    if (frame_slot) inv_n = 1.0f / (float)(*frame_slot + 1);
+    for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) {
+        const size_t i = count - 1 - k;
+        const float4 a = sums[i];
+        if (kCopy) accum[i] = a;
+        out[i] = make_float4(a.x * inv_n, a.y * inv_n, a.z * inv_n, a.w * inv_n);
+    }
+}
+
+__global__ void __launch_bounds__(256) accumulate_kernel(const float4 *in, float4 *__restrict__ accum, float4 *out, size_t count, float inv_n,
                                                          const int *frame_slot) {
     // a recorded pass reads its frame index from the slot (the same float division the host does)
     if (frame_slot) inv_n = 1.0f / (float)(*frame_slot + 1);
@@ -131,27 +279,30 @@ int launch_accumulate(float4 *color, float4 *accum, float4 *scratch, int *flag_d
     const size_t count = (size_t)width * height;
     const float inv_n = 1.0f / (float)(frame_index + 1);
     int launches = 0;
-    const float4 *src = color;
     cudaError_t e = cudaSuccess;
+    const int blocks = (int)std::max<size_t>(1, std::min<size_t>((count + 255) / 256, (size_t)148 * 8));
     if (firefly) {
-        const dim3 grid((width + 15) / 16, (height + 15) / 16);
-        firefly_kernel<<<grid, 256, 0, st>>>(color, nullptr, scratch, width, height, nullptr);
-        ++launches;
-        src = scratch;
+        const unsigned grid =
+            (unsigned)((size_t)((width + kTileW - 1) / kTileW) * (size_t)((height + kTileH - 1) / kTileH));
         if (mode == 0) {
-            // in-place-order check, then the exact in-place clamp when it failed
+            // the in-place-order check, then the exact in-place clamp when it failed
             if ((e = cudaMemsetAsync(flag_dev, 0, sizeof(int), st)) != cudaSuccess) {
                 if (err) *err = e;
                 return -1;
             }
-            firefly_kernel<<<grid, 256, 0, st>>>(color, scratch, nullptr, width, height, flag_dev);
-            firefly_sequential_kernel<<<1, 1024, 0, st>>>(color, scratch, width, height, flag_dev);
+            firefly_sum_kernel<true><<<grid, kTileThreads, 0, st>>>(color, accum, scratch, width, height, flag_dev);
+            firefly_sequential_kernel<<<1, 1024, 0, st>>>(color, accum, scratch, width, height, flag_dev);
+            mean_kernel<true><<<blocks, 256, 0, st>>>(scratch, accum, color, count, inv_n, frame_slot);
+            launches += 3;
+        } else {
+            firefly_sum_kernel<false><<<grid, kTileThreads, 0, st>>>(color, accum, accum, width, height, nullptr);
+            mean_kernel<false><<<blocks, 256, 0, st>>>(accum, accum, color, count, inv_n, frame_slot);
             launches += 2;
         }
+    } else {
+        accumulate_kernel<<<blocks, 256, 0, st>>>(color, accum, color, count, inv_n, frame_slot);
+        ++launches;
     }
-    const int blocks = (int)std::min<size_t>((count + 255) / 256, (size_t)148 * 8);
-    accumulate_kernel<<<blocks > 0 ? blocks : 1, 256, 0, st>>>(src, accum, color, count, inv_n, frame_slot);
-    ++launches;
     if ((e = cudaGetLastError()) != cudaSuccess) {
         if (err) *err = e;
         return -1;
