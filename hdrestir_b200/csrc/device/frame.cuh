@@ -95,8 +95,7 @@ struct WaveBuffers {
     float4 *q_closest;    // 2 per entry: origin.xyz + slot bits | direction.xyz
     float4 *q_shadow;     // 2 per entry: origin.xyz + slot bits | direction.xyz + distance limit
     int *counts;          // [0] closest-hit queue length, [1] shadow queue length (8 ints)
-    int *fix;             // one per closest-hit queue entry: entries whose checked SAH hit the reference walk
-                          // redoes (nullptr exactly when the queue has no entries)
+    size_t closest_slots, shadow_slots;  // entries the queues can hold (0 closest-hit slots: no such queue)
     float4 *hits;         // pixels * n_closest: t, instance bits, triangle bits, u
     float *hit_v;         // pixels * n_closest
     unsigned char *occ;   // n_shadow planes of pixels
@@ -136,7 +135,7 @@ constexpr int kShadowShapes = 3;
 struct TraceTuning {
     int mode = 0;
     int node_quorum = 12;  // best for the SAH-tree walks (16 for the reference-tree ones)
-    int blocks_per_sm = 16;
+    int blocks_per_sm = 8;  // what is resident; more only wait for a drained queue
     int sm_count = 148;
     int shade_shape = 3;  // ris_resample launch shape, 0 .. kShadeShapes - 1 (128 x 8: fastest at 1080p)
     // shadow-BVH walk register budget, 0 .. kShadowShapes - 1: 64 / 80 / 90 registers. With one ray
@@ -148,14 +147,13 @@ struct TraceTuning {
 // = (256, 2), (256, 4), (128, 5), (128, 8)
 constexpr int kShadeShapes = 4;
 // The trace kernels over the queues of the last ris_generate: closest hits, then
-// shadow queries; with checked SAH closest hits (s.sh4_closest == 2) also the
-// check and the reference walk of the entries it rejected (counts[6..7], wb.fix).
+// shadow queries; with checked SAH closest hits (s.sh4_closest == 2) also the check.
 // They read the queue counts and reset nothing but their own fetch counters' use,
 // so the caller zeroes counts[2..3] before a rerun; returns the launches, -1 on error.
 // The shadow-ray queue q over the shadow BVH when the scene has it (s.sh4), else the
-// phased walk of the reference trees; *count rays, *fetch the hand-out counter.
-int launch_shadow_queue(const DeviceScene &s, const float4 *q, const int *count, int *fetch, unsigned char *occ,
-                        const TraceTuning &tune, unsigned *err, cudaStream_t st);
+// phased walk of the reference trees; *count rays of at most `slots`, *fetch the hand-out counter.
+int launch_shadow_queue(const DeviceScene &s, const float4 *q, size_t slots, const int *count, int *fetch,
+                        unsigned char *occ, const TraceTuning &tune, unsigned *err, cudaStream_t st);
 int launch_wave_trace(const DeviceScene &s, WaveBuffers wb, const TraceTuning &tune, unsigned *err, cudaStream_t st,
                       cudaEvent_t *ev_begin = nullptr, cudaEvent_t *ev_end = nullptr);
 // Spatial reuse (extension, spatial.cu): merges up to p.spatial_neighbors
@@ -241,13 +239,13 @@ struct PtBuffers {
     uint4 *rng;             // 3 planes: stream state between kernels
     float4 *tp, *total;     // throughput and running radiance of _li (4 wavelengths)
     float4 *outer;          // PathIntegrator::Li's throughput (primary Beer), applied at the end
-    float4 *ray_o, *ray_d;  // the current vertex's incoming ray; ray_o.w: the wavelength draw
-    float4 *b_origin_pdf, *b_dir, *b_tmul;  // the vertex's BSDF sample
+    float4 *b_origin_pdf, *b_dir, *b_tmul;  // the vertex's BSDF sample; b_dir.w: the wavelength draw
     float4 *nee_add;        // the vertex's NEE term, added if its shadow ray is unoccluded
-    int4 *state;            // BounceState refl, refr; flags; spare
+    int4 *state;            // BounceState refl, refr; flags; the path's image
     int *active[2];         // live-path lists (ping-pong)
-    int *counts;            // [0..3] queue lengths and fetch counters, [4..5] active-list lengths
-    int *fix;               // WaveBuffers::fix of the closest-hit queue
+    int *active_count[2];   // their lengths
+    int *counts;            // [0..3] queue lengths and fetch counters
+    int *all_counts;        // active_count[1], counts[0..3], active_count[0]: a round clears five in a row
     float4 *q_closest, *q_shadow, *hits;
     float *hit_v;
     unsigned char *occ;

@@ -1298,8 +1298,8 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         wb.q_shadow = (float4 *)q;
         if ((st = ensure_buffer(c, "__wave_counts", 32, &q)) != HDR_OK) return st;
         wb.counts = (int *)q;
-        if ((st = ensure_buffer(c, "__wave_fix", count * wb.n_closest * 4, &q)) != HDR_OK) return st;
-        wb.fix = (int *)q;
+        wb.closest_slots = count * (size_t)wb.n_closest;
+        wb.shadow_slots = count * (size_t)wb.n_shadow;
         if ((st = ensure_buffer(c, "__wave_hits", count * wb.n_closest * 16, &q)) != HDR_OK) return st;
         wb.hits = (float4 *)q;
         if ((st = ensure_buffer(c, "__wave_hit_v", count * wb.n_closest * 4, &q)) != HDR_OK) return st;
@@ -1381,16 +1381,14 @@ hdr_status pt_buffers_from(Alloc alloc, size_t count, hdr::PtBuffers &B) {
         size_t bytes;
         void **dst;
     };
-    void *rng, *tp, *total, *outer, *ro, *rd, *bo, *bd, *bt, *nee, *state, *a0, *a1, *cnt, *qc, *qs, *hits, *hv, *occ,
-        *fix;
+    void *rng, *tp, *total, *outer, *bo, *bd, *bt, *nee, *state, *a0, *a1, *cnt, *qc, *qs, *hits, *hv, *occ;
     const Plane planes[] = {
         {"__pt_rng", count * 48, &rng},     {"__pt_tp", count * 16, &tp},       {"__pt_total", count * 16, &total},
-        {"__pt_outer", count * 16, &outer}, {"__pt_ray_o", count * 16, &ro},    {"__pt_ray_d", count * 16, &rd},
-        {"__pt_b_origin", count * 16, &bo}, {"__pt_b_dir", count * 16, &bd},    {"__pt_b_tmul", count * 16, &bt},
+        {"__pt_outer", count * 16, &outer}, {"__pt_b_origin", count * 16, &bo}, {"__pt_b_dir", count * 16, &bd},    {"__pt_b_tmul", count * 16, &bt},
         {"__pt_nee", count * 16, &nee},     {"__pt_state", count * 16, &state}, {"__pt_active0", count * 4, &a0},
         {"__pt_active1", count * 4, &a1},   {"__pt_counts", 32, &cnt},          {"__pt_q_closest", count * 32, &qc},
         {"__pt_q_shadow", count * 32, &qs}, {"__pt_hits", count * 16, &hits},   {"__pt_hit_v", count * 4, &hv},
-        {"__pt_occ", count, &occ},          {"__pt_fix", count * 4, &fix}};
+        {"__pt_occ", count, &occ}};
     hdr_status st;
     for (const Plane &pl : planes)
         if ((st = alloc(pl.name, pl.bytes, pl.dst)) != HDR_OK) return st;
@@ -1398,8 +1396,6 @@ hdr_status pt_buffers_from(Alloc alloc, size_t count, hdr::PtBuffers &B) {
     B.tp = (float4 *)tp;
     B.total = (float4 *)total;
     B.outer = (float4 *)outer;
-    B.ray_o = (float4 *)ro;
-    B.ray_d = (float4 *)rd;
     B.b_origin_pdf = (float4 *)bo;
     B.b_dir = (float4 *)bd;
     B.b_tmul = (float4 *)bt;
@@ -1407,8 +1403,10 @@ hdr_status pt_buffers_from(Alloc alloc, size_t count, hdr::PtBuffers &B) {
     B.state = (int4 *)state;
     B.active[0] = (int *)a0;
     B.active[1] = (int *)a1;
-    B.counts = (int *)cnt;
-    B.fix = (int *)fix;
+    B.all_counts = (int *)cnt;
+    B.active_count[1] = B.all_counts;
+    B.counts = B.all_counts + 1;
+    B.active_count[0] = B.all_counts + 5;
     B.q_closest = (float4 *)qc;
     B.q_shadow = (float4 *)qs;
     B.hits = (float4 *)hits;
@@ -1706,8 +1704,8 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
     all.q_shadow = (float4 *)q;
     if ((st = ensure_batch_scratch(store, "counts", 32, &q, done, lead->stream)) != HDR_OK) return st;
     all.counts = (int *)q;
-    if ((st = ensure_batch_scratch(store, "fix", (size_t)total_c * 4, &q, done, lead->stream)) != HDR_OK) return st;
-    all.fix = (int *)q;
+    all.closest_slots = (size_t)total_c;
+    all.shadow_slots = (size_t)total_s;
     if ((st = ensure_batch_scratch(store, "hits", (size_t)total_c * 16, &q, done, lead->stream)) != HDR_OK) return st;
     all.hits = (float4 *)q;
     if ((st = ensure_batch_scratch(store, "hit_v", (size_t)total_c * 4, &q, done, lead->stream)) != HDR_OK) return st;

@@ -3,15 +3,19 @@
 // 48-209) with MisDirectLightIntegrator (mis_direct_light_integrator.cpp:
 // 122-269), one vertex of every live path per round:
 //   start   (vertex 0)  the pixel prologue of IntegrationPass (seed, jitter,
-//                       wavelengths, GBuffer hit), then `sample`
-//   sample  (vertex v)  BSDF sample of the vertex (its draws), queued as the
-//                       extension ray; the light sample of _integrateNEE (its
-//                       draws, after the BSDF's), queued as a shadow ray with
-//                       what it adds if unoccluded
-//   trace               the phased closest-hit and shadow kernels over the queues
+//                       wavelengths, GBuffer hit) and the vertex's samples
+//   trace               the closest-hit and shadow queues
 //   connect (vertex v)  NEE term if unoccluded, _integrateBSDFConnection with
 //                       the extension hit, throughput, roulette (its draw);
-//                       surviving paths are appended to the next active list
+//                       a path that goes on is appended to the next active list
+//                       and takes the samples of vertex v + 1 at its hit
+// A vertex's samples (sample_vertex): its BSDF sample (its draws), queued as the
+// extension ray; the light sample of _integrateNEE (its draws, after the BSDF's),
+// queued as a shadow ray with what it adds if unoccluded.
+//
+// Connecting and sampling the next vertex in one kernel keeps the hit, the closure's
+// surface, the wavelength tables and the stream in registers: as two kernels they took
+// 1.04 + 0.94 ms of the 8.8 ms of nine dome views at depth 16, and two launches per vertex.
 // The draws of a pixel keep the order of the one-thread form (BSDF sample,
 // light sample, roulette per vertex) and every value is computed by the same
 // functions, so the image is that form's. The stream state, throughput and
@@ -24,11 +28,14 @@
 #define HDR_BOUNCE_INLINE __forceinline__
 #include "device/integrator.cuh"
 
+#include <algorithm>
+
 namespace hdr {
 
 namespace {
 
-constexpr unsigned kFlagNee = 1, kFlagOk = 2, kFlagImpossibleNee = 4, kFlagSkipRoulette = 8;
+constexpr unsigned kFlagNee = 1, kFlagOk = 2, kFlagImpossibleNee = 4, kFlagSkipRoulette = 8, kFlagCast = 16;
+constexpr int kPtThreads = 128;
 constexpr uint32_t kStreamHandOffLimit = 250;
 
 __device__ __forceinline__ int active_append(int *count, int *list, bool want, int path) {
@@ -58,13 +65,21 @@ __device__ __forceinline__ float4 f4(const Spec &s) { return make_float4(s.v[0],
 __device__ __forceinline__ Spec spec4(float4 a) { return Spec{{a.x, a.y, a.z, a.w}}; }
 __device__ __forceinline__ V3 v3(float4 a) { return V3{a.x, a.y, a.z}; }
 
-// BSDF sample and light sample of vertex `v` of path i (surface sf), queued.
+// BSDF sample and light sample of vertex `vertex` of path i (surface sf), queued; u: the
+// wavelength draw, job: the path's image.
+//
+// The last vertex's extension ray can only meet emission: where nothing emits, no light has
+// geometry and there is no environment, its term is the sample's throughput times zero
+// whatever it hits, which adds nothing unless the throughput is not finite.
 __device__ __forceinline__ void sample_vertex(const DeviceScene &s, const PtBuffers &B, size_t i, const Surface &sf,
                                               BounceState &st, const SpectralCtx &sc, MtStream &rng,
-                                              const PathRun &pr) {
+                                              const PathRun &pr, int vertex, float u, int job) {
     const Bounce b = sample_bounce(sf.c, sf.sn, sf.inside, sf.hit.position, sf.ray_d, pr.max_refl, pr.max_refr, st,
                                    sc, rng);
-    const int qc = queue_slot(&B.counts[0], b.ok);
+    const bool dark = vertex + 1 >= pr.max_depth && !s.bsdf_lights && !s.emissive && isfinite(b.tmul.v[0]) &&
+                      isfinite(b.tmul.v[1]) && isfinite(b.tmul.v[2]) && isfinite(b.tmul.v[3]);
+    const bool cast = b.ok && !dark;
+    const int qc = queue_slot(&B.counts[0], cast);
     if (qc >= 0) {
         B.q_closest[2 * (size_t)qc] = f4(b.origin, __int_as_float((int)i));
         B.q_closest[2 * (size_t)qc + 1] = f4(b.dir, 0.0f);
@@ -76,12 +91,13 @@ __device__ __forceinline__ void sample_vertex(const DeviceScene &s, const PtBuff
         B.q_shadow[2 * (size_t)qs + 1] = f4(nee.d, nee.limit);
     }
     const unsigned flags = (nee.cast ? kFlagNee : 0) | (b.ok ? kFlagOk : 0) |
-                           (b.impossible_nee ? kFlagImpossibleNee : 0) | (b.skip_roulette ? kFlagSkipRoulette : 0);
+                           (b.impossible_nee ? kFlagImpossibleNee : 0) | (b.skip_roulette ? kFlagSkipRoulette : 0) |
+                           (cast ? kFlagCast : 0);
     B.b_origin_pdf[i] = f4(b.origin, b.pdf);
-    B.b_dir[i] = f4(b.dir, 0.0f);
+    B.b_dir[i] = f4(b.dir, u);
     B.b_tmul[i] = f4(b.tmul);
     B.nee_add[i] = f4(nee.add);
-    B.state[i] = make_int4(st.refl, st.refr, (int)flags, B.state[i].w);
+    B.state[i] = make_int4(st.refl, st.refr, (int)flags, job);
     store_stream(B.rng, i, B.pixels, rng);
 }
 
@@ -164,44 +180,15 @@ __global__ void __launch_bounds__(256) pt_start_kernel(const __grid_constant__ D
     B.outer[i] = f4(outer);
     B.total[i] = f4(rgb_to_spectrum(sf.c.emission, sc.up));
     B.tp[i] = f4(spec(1.0f));
-    B.ray_o[i] = f4(ray.o, u);
-    B.ray_d[i] = f4(ray.d, 0.0f);
-    B.state[i] = make_int4(0, 0, 0, jk);  // .w: the path's image
     BounceState st{0, 0};
-    sample_vertex(s, B, i, sf, st, sc, rng, pr);
-    active_append(&B.counts[4], B.active[0], true, (int)i);
-}
-
-// vertex v >= 1 of the paths in `list` (their extension hit is in the hit slots)
-__global__ void __launch_bounds__(256) pt_sample_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ PathRun pr, const __grid_constant__ PtBuffers B, const int *list,
-                                                        const int *count, unsigned *err) {
-    const int n = *count;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const size_t i = (size_t)list[k];
-        MtStream rng = load_stream(B.rng, i, B.pixels);
-        const float4 ro4 = B.ray_o[i], rd4 = B.ray_d[i];
-        const SpectralCtx sc = make_spectral_ctx(ro4.w);
-        const float4 hr = B.hits[i];
-        const HitId id{hr.x, __float_as_int(hr.y), hit_tri(__float_as_int(hr.z)), hr.w, B.hit_v[i]};
-        const V3 ro = v3(ro4), rd = v3(rd4);
-        const Hit bh = make_hit(s, ro, rd, id);
-        Closure c = get_closure(s, bh);
-        if (!pr.enable_subsurface) c.subsurface = 0.0f;
-        const bool inside = dot(c.normal, rd) > 0.0f;
-        Spec tp = spec4(B.tp[i]);
-        beer_absorption(tp, c, bh.depth, inside, sc);
-        B.tp[i] = f4(tp);
-        const Surface sf = make_surface(s, ro, rd, bh, c, inside);
-        const int4 stt = B.state[i];
-        BounceState st{stt.x, stt.y};
-        sample_vertex(s, B, i, sf, st, sc, rng, pr);
-    }
+    sample_vertex(s, B, i, sf, st, sc, rng, pr, 0, u, jk);
+    active_append(B.active_count[0], B.active[0], true, (int)i);
 }
 
 // vertex v of the paths in `list`: the vertex's direct light, then the path goes
-// on (appended to `next`) or ends (its colour written)
+// on (appended to `next`, the samples of vertex v + 1 queued) or ends (its colour written)
 template <bool kBatch>
-__global__ void __launch_bounds__(256) pt_connect_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ PtJobD one, const PtJobD *table,
+__global__ void __launch_bounds__(kPtThreads, 4) pt_connect_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ PtJobD one, const PtJobD *table,
                                                          const __grid_constant__ PathRun pr, const __grid_constant__ PtBuffers B, const int *list, const int *count, int *next,
                                                          int *next_count, int vertex, unsigned *err) {
     const int n = *count;
@@ -217,14 +204,13 @@ __global__ void __launch_bounds__(256) pt_connect_kernel(const __grid_constant__
             i = (size_t)list[k];
             const int4 stt = B.state[i];
             const unsigned flags = (unsigned)stt.z;
-            const float4 ro4 = B.ray_o[i];
-            const SpectralCtx sc = make_spectral_ctx(ro4.w);
+            const float4 bo = B.b_origin_pdf[i], bd = B.b_dir[i];
+            const SpectralCtx sc = make_spectral_ctx(bd.w);
             MtStream rng = load_stream(B.rng, i, B.pixels);
             // _integrateNEE's term if its shadow ray was unoccluded
             Spec direct = spec(0.0f);
             if ((flags & kFlagNee) && B.occ[i] == 0) direct = direct + spec4(B.nee_add[i]);
             // _integrateBSDFConnection with the extension ray's hit
-            const float4 bo = B.b_origin_pdf[i], bd = B.b_dir[i];
             Connection cn;
             cn.b.ok = (flags & kFlagOk) != 0;
             cn.b.origin = v3(bo);
@@ -235,7 +221,7 @@ __global__ void __launch_bounds__(256) pt_connect_kernel(const __grid_constant__
             cn.b.impossible_nee = (flags & kFlagImpossibleNee) != 0;
             cn.b.skip_roulette = (flags & kFlagSkipRoulette) != 0;
             cn.has_hit = false;
-            if (cn.b.ok) {
+            if (flags & kFlagCast) {
                 const float4 hr = B.hits[i];
                 const HitId id{hr.x, __float_as_int(hr.y), hit_tri(__float_as_int(hr.z)), hr.w, B.hit_v[i]};
                 if (id.inst >= 0) {
@@ -266,11 +252,15 @@ __global__ void __launch_bounds__(256) pt_connect_kernel(const __grid_constant__
                 alive = false;
             }
             if (alive) {
-                B.tp[i] = f4(tp);
                 B.total[i] = f4(total);
-                B.ray_o[i] = f4(cn.b.origin, ro4.w);
-                B.ray_d[i] = f4(cn.b.dir, 0.0f);
-                store_stream(B.rng, i, B.pixels, rng);
+                Closure c = get_closure(s, cn.hit);
+                if (!pr.enable_subsurface) c.subsurface = 0.0f;
+                const bool inside = dot(c.normal, cn.b.dir) > 0.0f;
+                beer_absorption(tp, c, cn.hit.depth, inside, sc);
+                B.tp[i] = f4(tp);
+                const Surface sf = make_surface(s, cn.b.origin, cn.b.dir, cn.hit, c, inside);
+                BounceState st{stt.x, stt.y};
+                sample_vertex(s, B, i, sf, st, sc, rng, pr, vertex + 1, bd.w, stt.w);
                 go_on = true;
             } else {
                 finish_path(kBatch ? table[stt.w] : one, B, i, total, sc);
@@ -287,33 +277,27 @@ int launch_path_trace_wavefront(const DeviceScene &s, const PtJobD *jobs, int n_
     const bool batch = n_jobs > 1;
     const PathRun pr = jobs[0].pr;
     int launches = 0;
-    // [0] / [1] closest / shadow queue, [2] / [3] their fetch counters, [4] / [5] active-list lengths
-    if (cudaMemsetAsync(B.counts, 0, 8 * sizeof(int), st) != cudaSuccess) return -1;
+    if (cudaMemsetAsync(B.all_counts, 0, 6 * sizeof(int), st) != cudaSuccess) return -1;
     (batch ? pt_start_kernel<true> : pt_start_kernel<false>)<<<total_tiles, 256, 0, st>>>(s, jobs[0], table, n_jobs, B);
     ++launches;
     WaveBuffers wb{};
     wb.q_closest = B.q_closest;
     wb.q_shadow = B.q_shadow;
     wb.counts = B.counts;
-    wb.fix = B.fix;
+    wb.closest_slots = wb.shadow_slots = B.pixels;
     wb.hits = B.hits;
     wb.hit_v = B.hit_v;
     wb.occ = B.occ;
-    const int grid = tune.sm_count * 8;
+    const int grid = (int)std::min<size_t>((size_t)tune.sm_count * 16, (B.pixels + kPtThreads - 1) / kPtThreads);
     for (int v = 0; v < pr.max_depth; ++v) {
         const int cur = v & 1, nxt = cur ^ 1;
-        if (v > 0) {
-            // the queues of this vertex start empty; `cur` was filled by the last connect
-            if (cudaMemsetAsync(B.counts, 0, 4 * sizeof(int), st) != cudaSuccess) return -1;
-            pt_sample_kernel<<<grid, 256, 0, st>>>(s, pr, B, B.active[cur], &B.counts[4 + cur], err);
-            ++launches;
-        }
         const int t = launch_wave_trace(s, wb, tune, err, st);
         if (t < 0) return -1;
         launches += t;
-        if (cudaMemsetAsync(&B.counts[4 + nxt], 0, sizeof(int), st) != cudaSuccess) return -1;
-        (batch ? pt_connect_kernel<true> : pt_connect_kernel<false>)<<<grid, 256, 0, st>>>(
-            s, jobs[0], table, pr, B, B.active[cur], &B.counts[4 + cur], B.active[nxt], &B.counts[4 + nxt], v, err);
+        // the queues of the next vertex and its active list start empty
+        if (cudaMemsetAsync(nxt ? B.all_counts : B.counts, 0, 5 * sizeof(int), st) != cudaSuccess) return -1;
+        (batch ? pt_connect_kernel<true> : pt_connect_kernel<false>)<<<grid, kPtThreads, 0, st>>>(
+            s, jobs[0], table, pr, B, B.active[cur], B.active_count[cur], B.active[nxt], B.active_count[nxt], v, err);
         ++launches;
     }
     return cudaPeekAtLastError() == cudaSuccess ? launches : -1;

@@ -1,5 +1,6 @@
 // Ray-queue kernels of the wavefront passes: the closest-hit and shadow queries over
 // the queues the generate / sample kernels fill, one answer per ray in its slot.
+#include <algorithm>
 #include <type_traits>
 
 #include "device/frame.cuh"
@@ -69,8 +70,7 @@ __device__ __forceinline__ void bind_deep(SplitStack<Entry, kDepth, kThreads> &s
 
 template <bool kWide, bool kShallow, bool kAnyHit, class Put>
 __device__ __forceinline__ void phased_trace(const DeviceScene &s, const float4 *__restrict__ q,
-                                             const int *__restrict__ order, int n, int *fetch_at, int quorum,
-                                             Put put, unsigned &e) {
+                                             int n, int *fetch_at, int quorum, Put put, unsigned &e) {
     using PW = PhasedTraceWalk<kWide, kAnyHit, kShallow>;
     __shared__ typename PW::Entry col[PW::kShared * kTraceThreads];
     typename PW::Entry deep[kShallow ? 1 : kTraceStack - PW::kShared];
@@ -90,8 +90,7 @@ __device__ __forceinline__ void phased_trace(const DeviceScene &s, const float4 
         const int k = fetch_ray(fetch_at, n, done, drained);
         if (done) {
             if (k >= 0) {
-                const size_t r = order ? (size_t)order[k] : (size_t)k;
-                const float4 a = q[2 * r], b = q[2 * r + 1];
+                const float4 a = q[2 * (size_t)k], b = q[2 * (size_t)k + 1];
                 w.start(s, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, kAnyHit ? b.w : 0.0f);
                 slot = __float_as_int(a.w);
             } else {
@@ -119,16 +118,14 @@ constexpr int phased_min_blocks() {
     return kWide ? 6 : 8;
 }
 
-// Closest hits on the reference's trees for the queue entries order[0..*count)
-// (order nullptr: entries 0..*count), fetch counting the entries handed out.
+// Closest hits on the reference's trees, fetch counting the entries handed out.
 template <bool kWide, bool kShallow>
 __global__ void __launch_bounds__(kTraceThreads, phased_min_blocks<kWide>()) trace_closest_phased_kernel(DeviceScene s, const float4 *__restrict__ q,
-                                                                             const int *order, const int *count,
-                                                                             int *fetch, float4 *hits, float *hit_v,
+                                                                             const int *count, int *fetch, float4 *hits, float *hit_v,
                                                                              int quorum, unsigned *err) {
     unsigned e = 0;
     phased_trace<kWide, kShallow, false>(
-        s, q, order, *count, fetch, quorum,
+        s, q, *count, fetch, quorum,
         [&](int slot, const auto &w) {
             hits[slot] = make_float4(w.hit.t, __int_as_float(w.hit.inst), __int_as_float(w.hit.tri), w.hit.u);
             hit_v[slot] = w.hit.v;
@@ -144,7 +141,7 @@ __global__ void __launch_bounds__(kTraceThreads, phased_min_blocks<kWide>()) tra
                                                                             unsigned *err) {
     unsigned e = 0;
     phased_trace<kWide, kShallow, true>(
-        s, q, nullptr, *count, fetch, quorum,
+        s, q, *count, fetch, quorum,
         [&](int slot, const auto &w) { occ[slot] = w.shadow_answer() ? 1 : 0; }, e);
     if (e) atomicOr(err, e);
 }
@@ -193,8 +190,7 @@ struct RayChunk {
 // W: the walk; start(w, entry a, entry b) gives it a ray; put(slot, w) stores its answer.
 template <class W, class Start, class Put>
 __device__ __forceinline__ void walk4_queue(const DeviceScene &s, W &w, const float4 *__restrict__ q, int n, int *fetch,
-                                            int quorum, Start start, Put put, unsigned &e) {
-    __shared__ int col[kSh4Shared * kTraceThreads];
+                                            int quorum, int *col, Start start, Put put, unsigned &e) {
     int deep[kSh4Stack - kSh4Shared];
     w.stack.bind(col + threadIdx.x, deep);
     w.cur = kSh4Done;
@@ -229,34 +225,22 @@ __device__ __forceinline__ void walk4_queue(const DeviceScene &s, W &w, const fl
 
 using Sh4QueueStack = Sh4SplitStack<kSh4Shared, kTraceThreads>;
 
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kTraceThreads, kMinBlocks) trace_shadow4_kernel(const __grid_constant__ DeviceScene s,
-                                                                       const float4 *__restrict__ q, const int *count,
-                                                                       int *fetch, unsigned char *occ, int quorum,
-                                                                       unsigned *err) {
-    unsigned e = 0;
+__device__ __forceinline__ void shadow4_queue(const DeviceScene &s, const float4 *__restrict__ q, int n, int *fetch,
+                                              unsigned char *occ, int quorum, int *col, unsigned &e) {
     Shadow4Walk<Sh4QueueStack, Sh4RayRecord> w;
     walk4_queue(
-        s, w, q, *count, fetch, quorum,
+        s, w, q, n, fetch, quorum, col,
         [&](auto &x, float4 a, float4 b) { x.start(s, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, b.w); },
         [&](int slot, const auto &x) { occ[slot] = x.blocked() ? 1 : 0; }, e);
-    if (e) atomicOr(err, e);
 }
 
-// Closest-hit queue over the 4-wide SAH trees (DeviceScene::sh4_closest),
-// scheduled like trace_shadow4_kernel. With sh4_closest == 2 the hits are then
-// checked by check_closest_kernel, for which the triangle's upper bits carry the
-// walk's bound (hit_pack).
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kTraceThreads, kMinBlocks) trace_closest4_kernel(const __grid_constant__ DeviceScene s,
-                                                                                 const float4 *__restrict__ q,
-                                                                                 int *counts, float4 *hits,
-                                                                                 float *hit_v, int quorum,
-                                                                                 unsigned *err) {
-    unsigned e = 0;
+// Closest hits (DeviceScene::sh4_closest). With sh4_closest == 2 the hits are then checked by
+// check_closest_kernel, for which the triangle's upper bits carry the walk's bound (hit_pack).
+__device__ __forceinline__ void closest4_queue(const DeviceScene &s, const float4 *__restrict__ q, int n, int *fetch,
+                                               float4 *hits, float *hit_v, int quorum, int *col, unsigned &e) {
     Closest4Walk<Sh4QueueStack, Sh4RayRecord> w;
     walk4_queue(
-        s, w, q, counts[0], &counts[3], quorum,
+        s, w, q, n, fetch, quorum, col,
         [&](auto &x, float4 a, float4 b) { x.start(s, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}); },
         [&](int slot, const auto &x) {
             hits[slot] = make_float4(x.best_t, __int_as_float(x.hit_inst(s)),
@@ -264,33 +248,88 @@ __global__ void __launch_bounds__(kTraceThreads, kMinBlocks) trace_closest4_kern
             hit_v[slot] = x.best_v;
         },
         e);
+}
+
+template <int kMinBlocks>
+__global__ void __launch_bounds__(kTraceThreads, kMinBlocks) trace_shadow4_kernel(const __grid_constant__ DeviceScene s,
+                                                                       const float4 *__restrict__ q, const int *count,
+                                                                       int *fetch, unsigned char *occ, int quorum,
+                                                                       unsigned *err) {
+    __shared__ int col[kSh4Shared * kTraceThreads];
+    unsigned e = 0;
+    shadow4_queue(s, q, *count, fetch, occ, quorum, col, e);
     if (e) atomicOr(err, e);
 }
 
-// The check of the SAH walk's closest hits (sh4_closest == 2), one thread per
-// queue entry: an entry whose hit ref_reaches cannot vouch for is listed in
-// fix[0..*n_fix) for the reference walk. A miss needs no check: the SAH trees'
-// boxes hold every triangle, so the reference walk finds no hit either.
+template <int kMinBlocks>
+__global__ void __launch_bounds__(kTraceThreads, kMinBlocks) trace_closest4_kernel(const __grid_constant__ DeviceScene s,
+                                                                                 const float4 *__restrict__ q,
+                                                                                 int *counts, float4 *hits,
+                                                                                 float *hit_v, int quorum,
+                                                                                 unsigned *err) {
+    __shared__ int col[kSh4Shared * kTraceThreads];
+    unsigned e = 0;
+    closest4_queue(s, q, counts[0], &counts[3], hits, hit_v, quorum, col, e);
+    if (e) atomicOr(err, e);
+}
+
+// Both queues in one launch: even blocks take the closest hits first, odd ones the shadow rays,
+// each then helps with what is left of the other. A path tracer's late rounds have few rays, and
+// the last of them are waited for once instead of twice.
+template <int kMinBlocks>
+__global__ void __launch_bounds__(kTraceThreads, kMinBlocks) trace_both4_kernel(const __grid_constant__ DeviceScene s,
+                                                                              const float4 *__restrict__ q_closest,
+                                                                              const float4 *__restrict__ q_shadow,
+                                                                              int *counts, float4 *hits, float *hit_v,
+                                                                              unsigned char *occ, int quorum,
+                                                                              unsigned *err) {
+    __shared__ int col[kSh4Shared * kTraceThreads];
+    unsigned e = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        if ((pass ^ blockIdx.x) & 1)
+            shadow4_queue(s, q_shadow, counts[1], &counts[2], occ, quorum, col, e);
+        else
+            closest4_queue(s, q_closest, counts[0], &counts[3], hits, hit_v, quorum, col, e);
+    }
+    if (e) atomicOr(err, e);
+}
+
+// The check of the SAH walk's closest hits (sh4_closest == 2), one thread per queue entry: an
+// entry whose hit ref_reaches cannot vouch for walks the reference's trees here. Few do (of
+// 500,000 random rays the unchecked walk answers 19 differently among coplanar boxes, none over
+// the terrain), so they get no list and no kernel of their own: the two kernels took 208 us of
+// the four rounds of a 256 x 256 path-traced box, this one takes 23. A miss needs no check: the SAH trees' boxes hold every triangle, so
+// the reference walk finds no hit either.
 __global__ void __launch_bounds__(256) check_closest_kernel(const __grid_constant__ DeviceScene s,
                                                             const float4 *__restrict__ q, const int *count,
-                                                            const float4 *__restrict__ hits, int *fix, int *n_fix) {
+                                                            float4 *hits, float *hit_v, unsigned *err) {
     const int n = *count;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const float4 a = q[2 * (size_t)k];
-        const float4 h = hits[__float_as_int(a.w)];
+        const int slot = __float_as_int(a.w);
+        const float4 h = hits[slot];
         const int inst = __float_as_int(h.y), tri = __float_as_int(h.z);
         if (inst < 0) continue;
         const float4 b = q[2 * (size_t)k + 1];
+        const V3 o{a.x, a.y, a.z}, d{b.x, b.y, b.z};
         const float bound = __int_as_float(__float_as_int(h.x) + hit_bound_ulps(tri));
-        if (!ref_reaches(s.dev, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, inst, hit_tri(tri), bound))
-            fix[atomicAdd(n_fix, 1)] = k;
+        if (ref_reaches(s.dev, o, d, inst, hit_tri(tri), bound)) continue;
+        const RefClosest r = reference_closest(s.dev, o, d);
+        hits[slot] = make_float4(r.hit.t, __int_as_float(r.hit.inst), __int_as_float(r.hit.tri), r.hit.u);
+        hit_v[slot] = r.hit.v;
+        if (r.err) atomicOr(err, r.err);
     }
 }
 
+// Blocks of a persistent launch over a queue of at most `slots` entries.
+int grid_for(int most, size_t slots, int threads) {
+    return (int)std::max<size_t>(1, std::min<size_t>((size_t)most, (slots + (size_t)threads - 1) / (size_t)threads));
+}
+
 // The shadow-ray queue q (count / fetch counters on the device, answers into occ).
-int launch_shadow_queue(const DeviceScene &s, const float4 *q, const int *count, int *fetch, unsigned char *occ,
-                        const TraceTuning &tune, unsigned *err, cudaStream_t st) {
-    const int tgrid = tune.sm_count * tune.blocks_per_sm;
+int launch_shadow_queue(const DeviceScene &s, const float4 *q, size_t slots, const int *count, int *fetch,
+                        unsigned char *occ, const TraceTuning &tune, unsigned *err, cudaStream_t st) {
+    const int tgrid = grid_for(tune.sm_count * tune.blocks_per_sm, slots, kTraceThreads);
     if (s.sh4) {
         // register budget: 64 (8 resident blocks), 80 (6) or 90 (5) per thread
         auto k = tune.shadow_shape == 0 ? trace_shadow4_kernel<8>
@@ -393,44 +432,59 @@ __global__ void __launch_bounds__(kTraceThreads) trace_shadow_kernel(DeviceScene
 int launch_wave_trace(const DeviceScene &s, WaveBuffers wb, const TraceTuning &tune, unsigned *err, cudaStream_t st,
                       cudaEvent_t *ev_begin, cudaEvent_t *ev_end) {
     auto mark = [&](cudaEvent_t *ev, int k) { return !ev || cudaEventRecord(ev[k], st) == cudaSuccess; };
-    const int tgrid = tune.sm_count * tune.blocks_per_sm;
+    const int most = tune.sm_count * tune.blocks_per_sm;
+    const int cgrid = grid_for(most, wb.closest_slots, kTraceThreads);
+    const int sgrid = grid_for(most, wb.shadow_slots, kTraceThreads);
     const bool refill = (tune.mode & kTraceLanePerRay) == 0;
     const bool phased = refill && (tune.mode & kTraceUnphased) == 0;
     const bool shallow = s.shallow && (tune.mode & kTraceSplitStack) == 0;
+    const bool both = s.sh4 && s.sh4_closest && wb.closest_slots > 0 && !ev_begin;  // not timed one by one
     if (!mark(ev_begin, 0)) return -1;
-    int launches = 2;
-    auto reference_phased = s.wide    ? trace_closest_phased_kernel<true, false>
-                            : shallow ? trace_closest_phased_kernel<false, true>
-                                      : trace_closest_phased_kernel<false, false>;
-    if (s.sh4_closest) {
+    int launches = 0;
+    if (both) {
+        const int grid = grid_for(most, wb.closest_slots + wb.shadow_slots, kTraceThreads);
+        auto k = tune.shadow_shape == 0 ? trace_both4_kernel<8>
+                                        : (tune.shadow_shape == 1 ? trace_both4_kernel<6> : trace_both4_kernel<5>);
+        k<<<grid, kTraceThreads, 0, st>>>(s, wb.q_closest, wb.q_shadow, wb.counts, wb.hits, wb.hit_v, wb.occ,
+                                          tune.node_quorum, err);
+        ++launches;
+    } else if (wb.closest_slots == 0) {
+        // no closest-hit queue (kTraceNoBsdfRays)
+    } else if (s.sh4_closest) {
         auto closest = tune.shadow_shape == 0 ? trace_closest4_kernel<8>
                                               : (tune.shadow_shape == 1 ? trace_closest4_kernel<6>
                                                                         : trace_closest4_kernel<5>);
-        closest<<<tgrid, kTraceThreads, 0, st>>>(s, wb.q_closest, wb.counts, wb.hits, wb.hit_v, tune.node_quorum, err);
-        if (s.sh4_closest == 2 && wb.fix) {  // (no fix list: the queue has no entries)
-            // counts[6] entries the check rejected, counts[7] of them handed out
-            if (cudaMemsetAsync(wb.counts + 6, 0, 2 * sizeof(int), st) != cudaSuccess) return -1;
-            check_closest_kernel<<<tune.sm_count * 8, 256, 0, st>>>(s, wb.q_closest, wb.counts, wb.hits, wb.fix,
-                                                                      wb.counts + 6);
-            reference_phased<<<tgrid, kTraceThreads, 0, st>>>(s, wb.q_closest, wb.fix, wb.counts + 6, wb.counts + 7,
-                                                              wb.hits, wb.hit_v, tune.node_quorum, err);
-            launches += 2;
-        }
+        closest<<<cgrid, kTraceThreads, 0, st>>>(s, wb.q_closest, wb.counts, wb.hits, wb.hit_v, tune.node_quorum, err);
+        ++launches;
     } else if (phased) {
-        reference_phased<<<tgrid, kTraceThreads, 0, st>>>(s, wb.q_closest, nullptr, wb.counts, wb.counts + 3, wb.hits,
-                                                          wb.hit_v, tune.node_quorum, err);
+        auto closest = s.wide    ? trace_closest_phased_kernel<true, false>
+                       : shallow ? trace_closest_phased_kernel<false, true>
+                                 : trace_closest_phased_kernel<false, false>;
+        closest<<<cgrid, kTraceThreads, 0, st>>>(s, wb.q_closest, wb.counts, wb.counts + 3, wb.hits, wb.hit_v,
+                                                 tune.node_quorum, err);
+        ++launches;
     } else {
         auto closest = s.wide ? (refill ? trace_closest_kernel<true, true> : trace_closest_kernel<true, false>)
                               : (refill ? trace_closest_kernel<false, true> : trace_closest_kernel<false, false>);
-        closest<<<tgrid, kTraceThreads, 0, st>>>(s, wb.q_closest, wb.counts, wb.hits, wb.hit_v, err);
+        closest<<<cgrid, kTraceThreads, 0, st>>>(s, wb.q_closest, wb.counts, wb.hits, wb.hit_v, err);
+        ++launches;
+    }
+    if (wb.closest_slots > 0 && s.sh4_closest == 2) {
+        check_closest_kernel<<<grid_for(tune.sm_count * 8, wb.closest_slots, 256), 256, 0, st>>>(
+            s, wb.q_closest, wb.counts, wb.hits, wb.hit_v, err);
+        ++launches;
     }
     if (!mark(ev_end, 0) || !mark(ev_begin, 1)) return -1;
-    if (phased || s.sh4) {
-        if (launch_shadow_queue(s, wb.q_shadow, wb.counts + 1, wb.counts + 2, wb.occ, tune, err, st) < 0) return -1;
+    if (both) {
+    } else if (phased || s.sh4) {
+        if (launch_shadow_queue(s, wb.q_shadow, wb.shadow_slots, wb.counts + 1, wb.counts + 2, wb.occ, tune, err, st) < 0)
+            return -1;
+        ++launches;
     } else {
         auto shadow = s.wide ? (refill ? trace_shadow_kernel<true, true> : trace_shadow_kernel<true, false>)
                              : (refill ? trace_shadow_kernel<false, true> : trace_shadow_kernel<false, false>);
-        shadow<<<tgrid, kTraceThreads, 0, st>>>(s, wb.q_shadow, wb.counts, wb.occ, err);
+        shadow<<<sgrid, kTraceThreads, 0, st>>>(s, wb.q_shadow, wb.counts, wb.occ, err);
+        ++launches;
     }
     if (!mark(ev_end, 1)) return -1;
     return cudaPeekAtLastError() == cudaSuccess ? launches : -1;

@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(256) ris_winner_fixup_kernel(DeviceScene s, Ca
 int launch_winner_visibility(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
                              GBufferView gb, ReservoirView rv, WaveBuffers wb, float4 *color, unsigned *err,
                              cudaStream_t st, const TraceTuning &tune) {
-    if (hdr::launch_shadow_queue(s, wb.q_winner, wb.counts + 4, wb.counts + 5, wb.occ_winner, tune, err, st) < 0)
+    if (hdr::launch_shadow_queue(s, wb.q_winner, wb.pixels, wb.counts + 4, wb.counts + 5, wb.occ_winner, tune, err, st) < 0)
         return -1;
     ris_winner_fixup_kernel<<<tune.sm_count * 4, 256, 0, st>>>(s, cam, frame_index, path_run(p), gb, rv, wb.q_winner,
                                                                wb.counts + 4, wb.occ_winner, color);
