@@ -194,23 +194,33 @@ class Camera:
     params: dict | None = None  # CameraParams (scene/camera_params.h:8-20) or None = pinhole
 
     def c_desc(self) -> abi.CameraDesc:
-        d = abi.CameraDesc()
-        d.view[:] = [float(v) for v in np.asarray(self.view, np.float64).reshape(-1)]
-        d.proj[:] = [float(v) for v in np.asarray(self.proj, np.float64).reshape(-1)]
-        d.width, d.height = int(self.width), int(self.height)
+        # every pass makes one: it was 8 of the 28 us of a 321 x 181 raycast with its AOV copies
         p = self.params
-        d.has_params = 1 if p is not None else 0
-        p = p or {}
-        d.enable_dof = int(p.get("enable_dof", 0))
-        d.enable_exposure = int(p.get("enable_exposure", 0))
-        d.focal_length = float(p.get("focal_length", 50.0))
-        d.f_stop = float(p.get("f_stop", 5.6))
-        d.focus_distance = float(p.get("focus_distance", 10.0))
-        d.bokeh_blades = int(p.get("bokeh_blades", 0))
-        d.lens_distortion = float(p.get("lens_distortion", 0.0))
-        d.iso = float(p.get("iso", 100.0))
-        d.shutter_speed = float(p.get("shutter_speed", 0.02))
+        d = abi.CameraDesc.from_buffer_copy(_PINHOLE) if p is None else abi.CameraDesc()
+        d.view[:] = np.asarray(self.view, np.float64).ravel().tolist()
+        d.proj[:] = np.asarray(self.proj, np.float64).ravel().tolist()
+        d.width, d.height = int(self.width), int(self.height)
+        if p is None:
+            return d
+        d.has_params = 1
+        _set_camera_params(d, p)
         return d
+
+
+def _set_camera_params(d: abi.CameraDesc, p: dict) -> None:
+    d.enable_dof = int(p.get("enable_dof", 0))
+    d.enable_exposure = int(p.get("enable_exposure", 0))
+    d.focal_length = float(p.get("focal_length", 50.0))
+    d.f_stop = float(p.get("f_stop", 5.6))
+    d.focus_distance = float(p.get("focus_distance", 10.0))
+    d.bokeh_blades = int(p.get("bokeh_blades", 0))
+    d.lens_distortion = float(p.get("lens_distortion", 0.0))
+    d.iso = float(p.get("iso", 100.0))
+    d.shutter_speed = float(p.get("shutter_speed", 0.02))
+
+
+_PINHOLE = abi.CameraDesc()  # a camera without params: their defaults
+_set_camera_params(_PINHOLE, {})
 
 
 def look_at(eye, target, up=(0.0, 1.0, 0.0)) -> np.ndarray:
