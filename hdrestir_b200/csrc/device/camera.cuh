@@ -39,7 +39,8 @@ struct RayF {
     V3 o, d;
 };
 
-__device__ __forceinline__ RayF camera_ray(const CameraD &c, float px, float py, MtStream &rng) {
+template <class Rng>
+__device__ __forceinline__ RayF camera_ray(const CameraD &c, float px, float py, Rng &rng) {
     float ndc_x = (2.0f * px / (float)c.width) - 1.0f;
     float ndc_y = (2.0f * py / (float)c.height) - 1.0f;
     if (c.p.has_params && c.p.lens_distortion != 0.0f) {

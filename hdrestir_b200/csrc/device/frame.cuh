@@ -161,8 +161,8 @@ int launch_wave_trace(const DeviceScene &s, WaveBuffers wb, const TraceTuning &t
 // winner queue (q_winner, counts[4]) the shadow rays of moved samples are
 // queued for launch_winner_visibility instead of cast in the kernel.
 int launch_ris_spatial(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
-                       GBufferView gb, ReservoirView in, ReservoirView out, float4 *color, float4 *q_winner,
-                       int *winner_count, unsigned *err, cudaStream_t st);
+                       GBufferView gb, const uint4 *rng_state, ReservoirView in, ReservoirView out, float4 *color,
+                       float4 *q_winner, int *winner_count, unsigned *err, cudaStream_t st);
 // The queued winner shadow rays (wb.q_winner, counts[4] / [5]) traced, then the
 // pixels found occluded fixed up in rv and color.
 int launch_winner_visibility(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,

@@ -237,8 +237,9 @@ struct MisNeePart {
     Spec add;
 };
 
+template <class Rng>
 __device__ inline MisNeePart mis_nee_part(const DeviceScene &s, const Surface &sf, bool has_conn,
-                                          const SpectralCtx &sc, MtStream &rng) {
+                                          const SpectralCtx &sc, Rng &rng) {
     MisNeePart r;
     r.cast = false;
     r.add = spec(0.0f);

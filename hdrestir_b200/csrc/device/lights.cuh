@@ -151,7 +151,8 @@ __device__ __forceinline__ float env_pdf(const DeviceScene &s, V3 dir) {
 }
 
 // ILight::SampleLight
-__device__ inline bool sample_light(const DeviceScene &s, int li, V3 hit_pos, MtStream &rng, LightSampleD &ls) {
+template <class Rng>
+__device__ inline bool sample_light(const DeviceScene &s, int li, V3 hit_pos, Rng &rng, LightSampleD &ls) {
     const float4 *p = s.lights + 12 * li;
     const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
     const int type = fbits(a.x);
@@ -260,13 +261,14 @@ __device__ __forceinline__ void light_eval_pdf(const DeviceScene &s, int li, V3 
 }
 
 // UniformLightSampler::ProposeCandidate: light index, then SampleLight, pdf x 1/L.
-__device__ __forceinline__ bool propose_candidate(const DeviceScene &s, V3 hit_pos, MtStream &rng, int &li,
+template <class Rng>
+__device__ __forceinline__ bool propose_candidate(const DeviceScene &s, V3 hit_pos, Rng &rng, int &li,
                                                   LightSampleD &ls) {
     const int L = s.num_lights;
     if (L <= 0) return false;
     const float u = rng.next_float();
-    unsigned long long idx = (unsigned long long)(u * (float)L);
-    if (idx > (unsigned long long)(L - 1)) idx = (unsigned long long)(L - 1);
+    unsigned idx = (unsigned)(u * (float)L);  // u < 1, L < 2^31
+    if (idx > (unsigned)(L - 1)) idx = (unsigned)(L - 1);
     li = (int)idx;
     if (!sample_light(s, li, hit_pos, rng, ls)) return false;
     ls.pdf *= 1.0f / (float)L;
@@ -277,8 +279,8 @@ __device__ __forceinline__ void skip_propose_candidate(const DeviceScene &s, MtS
     const int L = s.num_lights;
     if (L <= 0) return;
     const float u = rng.next_float();
-    unsigned long long idx = (unsigned long long)(u * (float)L);
-    if (idx > (unsigned long long)(L - 1)) idx = (unsigned long long)(L - 1);
+    unsigned idx = (unsigned)(u * (float)L);  // u < 1, L < 2^31
+    if (idx > (unsigned)(L - 1)) idx = (unsigned)(L - 1);
     const int n = light_sample_draws(s, (int)idx);
     for (int k = 0; k < n; ++k) (void)rng.next_raw();
 }

@@ -359,8 +359,9 @@ struct BounceState {
 };
 
 // DefaultMaterial::SampleBounce (default_material.cpp:66-86): ONB of Duff et al. 2017, z-up cosine sample.
+template <class Rng>
 __device__ __forceinline__ Bounce sample_bounce_default(const Closure &c, V3 sn, V3 hit_pos, const SpectralCtx &sc,
-                                                        MtStream &rng) {
+                                                        Rng &rng) {
     const float sign = (sn.z >= 0.0f) ? 1.0f : -1.0f;
     const float a = -1.0f / (sign + sn.z);
     const float bb = sn.x * sn.y * a;
@@ -444,8 +445,9 @@ __device__ __forceinline__ Bounce specular_bounce(V3 origin, V3 dir, Spec tmul, 
 #define HDR_BOUNCE_INLINE inline
 #endif
 // IMaterial::SampleBounce dispatch
+template <class Rng>
 __device__ HDR_BOUNCE_INLINE Bounce sample_bounce(const Closure &c, V3 sn, bool inside, V3 hit_pos, V3 ray_dir, int max_refl,
-                                int max_refr, BounceState &st, const SpectralCtx &sc, MtStream &rng) {
+                                int max_refr, BounceState &st, const SpectralCtx &sc, Rng &rng) {
     if (c.is_default) return sample_bounce_default(c, sn, hit_pos, sc, rng);
     // --- coat (preview_surface.cpp:136-196)
     if (c.coat > 0.0f && !inside) {
@@ -628,8 +630,9 @@ __device__ __forceinline__ BounceDraws bounce_draws_of(const Closure &c, V3 sn, 
     d.refract_ok = 1.0f - eta * eta * (1.0f - cos_i * cos_i) >= 0;
     return d;
 }
+template <class Rng>
 __device__ __forceinline__ void bounce_draws(const BounceDraws &d, int max_refl, int max_refr, BounceState &st,
-                                             MtStream &rng) {
+                                             Rng &rng) {
     if (d.is_default) {
         (void)rng.next_raw();
         (void)rng.next_raw();

@@ -148,6 +148,42 @@ struct MtStream {
     }
 };
 
+// A stream of at most 155 draws, whose draws take no branch: its three words are the first
+// cursors of MtStream.
+struct MtShort {
+    uint64_t a, b, c;  // s[k], s[k+1], s[k+156]
+    uint32_t k, seed;
+
+    HDR_HD void init(uint32_t s, uint64_t * = nullptr) {
+        MtStream x;
+        x.init(s, nullptr);
+        a = x.a;
+        b = x.b;
+        c = x.c;
+        k = 0;
+        seed = s;
+    }
+    HDR_HD void init_from(uint32_t s, uint64_t s156, uint64_t * = nullptr) {
+        a = (uint64_t)s;
+        b = mt_seed_step(a, 1);
+        c = s156;
+        k = 0;
+        seed = s;
+    }
+    HDR_HD uint64_t next_raw() {
+        const uint64_t r = c ^ mt_twist(a, b);
+        a = b;
+        b = mt_seed_step(b, k + 2);
+        c = mt_seed_step(c, k + 157);
+        ++k;
+        return mt_temper(r);
+    }
+    HDR_HD float next_float() { return mt_to_float(next_raw()); }
+    HDR_HD MtStream stream() const { return MtStream{a, b, c, 0, 0, k, seed, nullptr}; }
+};
+HDR_HD const MtStream &whole_stream(const MtStream &r) { return r; }
+HDR_HD MtStream whole_stream(const MtShort &r) { return r.stream(); }
+
 // A stream in three uint4 planes of n entries (entry i): the state of a
 // stream below draw 312, handed from one kernel to the next.
 __device__ __forceinline__ void store_stream(uint4 *st, size_t i, size_t n, const MtStream &r) {
@@ -155,9 +191,8 @@ __device__ __forceinline__ void store_stream(uint4 *st, size_t i, size_t n, cons
     st[n + i] = make_uint4((unsigned)r.c, (unsigned)(r.c >> 32), (unsigned)r.d, (unsigned)(r.d >> 32));
     st[2 * n + i] = make_uint4((unsigned)r.new0, (unsigned)(r.new0 >> 32), r.k, r.seed);
 }
-__device__ __forceinline__ MtStream load_stream(const uint4 *st, size_t i, size_t n) {
+__device__ __forceinline__ void load_stream(const uint4 *st, size_t i, size_t n, MtStream &r) {
     const uint4 p = st[i], q = st[n + i], w = st[2 * n + i];
-    MtStream r;
     r.a = (uint64_t)p.x | ((uint64_t)p.y << 32);
     r.b = (uint64_t)p.z | ((uint64_t)p.w << 32);
     r.c = (uint64_t)q.x | ((uint64_t)q.y << 32);
@@ -166,9 +201,12 @@ __device__ __forceinline__ MtStream load_stream(const uint4 *st, size_t i, size_
     r.k = w.z;
     r.seed = w.w;
     r.spill = nullptr;
-    return r;
 }
-
+__device__ __forceinline__ void load_stream(const uint4 *st, size_t i, size_t n, MtShort &r) {
+    MtStream x;
+    load_stream(st, i, n, x);
+    r = MtShort{x.a, x.b, x.c, x.k, x.seed};
+}
 
 // The same with the stream's own start and one draw index of the pixel's: s156 stands in the
 // place of b, which is the step after a, and k0 in the place of the seed, which the pixel and
@@ -180,9 +218,14 @@ __device__ __forceinline__ void store_stream_from(uint4 *st, size_t i, size_t n,
     x.seed = k0;
     store_stream(st, i, n, x);
 }
+__device__ __forceinline__ uint64_t stored_s156(const uint4 *st, size_t i) {
+    const uint4 p = st[i];
+    return (uint64_t)p.z | ((uint64_t)p.w << 32);
+}
 __device__ __forceinline__ MtStream load_stream_from(const uint4 *st, size_t i, size_t n, uint32_t seed,
                                                      uint64_t &s156, uint32_t &k0) {
-    MtStream r = load_stream(st, i, n);
+    MtStream r;
+    load_stream(st, i, n, r);
     s156 = r.b;
     k0 = r.seed;
     r.b = mt_seed_step(r.a, r.k + 1);

@@ -1344,8 +1344,8 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         c->launches += (uint64_t)n;
         if (spatial) {  // merged reservoirs, copied back, then the moved samples' shadow rays
             HDR_CUDA(cudaMemsetAsync(wb.counts + 4, 0, 2 * sizeof(int), c->stream));
-            if (hdr::launch_ris_spatial(c->scene, cd, frame_index, d, gb, rv, rv_spatial, (float4 *)color,
-                                        wb.q_winner, wb.counts + 4, c->d_err, c->stream) < 0)
+            if (hdr::launch_ris_spatial(c->scene, cd, frame_index, d, gb, wb.rng_state, rv, rv_spatial,
+                                        (float4 *)color, wb.q_winner, wb.counts + 4, c->d_err, c->stream) < 0)
                 return fail(HDR_ECUDA, "spatial reuse launch failed: %s", cudaGetErrorString(cudaGetLastError()));
             HDR_CUDA(cudaMemcpyAsync(rv.dir_dist, rv_spatial.dir_dist, count * kResPlanes * sizeof(float4),
                                      cudaMemcpyDeviceToDevice, c->stream));

@@ -56,14 +56,19 @@ __device__ __forceinline__ void copy_record(const ReservoirView &in, const Reser
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads) ris_spatial_kernel(DeviceScene s, CameraD cam, int frame_arg,
                                                                PathRun pr, int cpf, int m_cap, int neighbours,
-                                                               float radius, GBufferView gb, ReservoirView in,
+                                                               float radius, GBufferView gb, const uint4 *rng_state,
+                                                               ReservoirView in,
                                                                ReservoirView out, float4 *color, float4 *q_winner,
                                                                int *winner_count, unsigned *err) {
     const int frame_index = live_frame(cam, frame_arg);
-    MtStream rng;
+    int x, y;
+    if (!tile_pixel<kThreads>(cam.width, cam.height, x, y)) return;
+    MtShort rng;
     PixelStart ps;
-    if (!pixel_start<kThreads>(s, cam, frame_index, gb, rng, nullptr, ps)) return;
-    const size_t i = ps.i;
+    const size_t i = ps.i = (size_t)y * (size_t)cam.width + (size_t)x;
+    ps.s156 = stored_s156(rng_state, i);  // a hit pixel's; else unused
+    // (seeding again took 80 of the 519 us of a 1080p frame with five neighbours)
+    pixel_start_at<true>(s, cam, frame_index, gb, x, y, rng, nullptr, ps);
     if (!ps.has_hit) {  // background pixel: the resampling pass left no reservoir to merge
         copy_record(in, out, i);
         return;
@@ -77,7 +82,6 @@ __global__ void __launch_bounds__(kThreads) ris_spatial_kernel(DeviceScene s, Ca
 
     Reservoir r;
     reservoir_load(in, i, r);
-    const int x = (int)(i % (size_t)cam.width), y = (int)(i / (size_t)cam.width);
     HashStream h{pcg_hash((uint32_t)i ^ pcg_hash((uint32_t)frame_index + 0x9e3779b9u))};
     bool shifted = false;
     unsigned e = 0;
@@ -146,8 +150,8 @@ __global__ void __launch_bounds__(kThreads) ris_spatial_kernel(DeviceScene s, Ca
 }  // namespace
 
 int launch_ris_spatial(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
-                       GBufferView gb, ReservoirView in, ReservoirView out, float4 *color, float4 *q_winner,
-                       int *winner_count, unsigned *err, cudaStream_t st) {
+                       GBufferView gb, const uint4 *rng_state, ReservoirView in, ReservoirView out, float4 *color,
+                       float4 *q_winner, int *winner_count, unsigned *err, cudaStream_t st) {
     PathRun pr{};
     pr.max_depth = p.max_depth;
     pr.enable_subsurface = p.enable_subsurface != 0;
@@ -156,8 +160,8 @@ int launch_ris_spatial(const DeviceScene &s, const CameraD &cam, int frame_index
     const int cpf = n_nee + (p.candidate_count - n_nee > 0 ? p.candidate_count - n_nee : 0);
     const float radius = p.spatial_radius > 0.0f ? p.spatial_radius : 30.0f;
     ris_spatial_kernel<256><<<tile_blocks(cam.width, cam.height), 256, 0, st>>>(
-        s, cam, frame_index, pr, cpf, p.m_cap, p.spatial_neighbors, radius, gb, in, out, color, q_winner,
-        winner_count, err);
+        s, cam, frame_index, pr, cpf, p.m_cap, p.spatial_neighbors, radius, gb, rng_state, in, out, color,
+        q_winner, winner_count, err);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 

@@ -70,17 +70,22 @@ constexpr int kPixelConnNan = 4;  // and its pdf squared overflows: its weight i
 // instead of a per-thread copy in local memory (a few hundred bytes written per
 // thread).
 //
-// Shape: 16 light candidates per 1080p terrain pixel, weights included, take 1.64 ms in four
-// blocks of 128 (128 registers, 28 bytes spilled), 1.69 in two of 256, 1.57 in three of 256 (80
-// registers) and 1.66 in four; 512 x 512 boxes with 8 candidates 0.117, 0.120, 0.129, 0.118.
+// Bound by instruction issue (16 light candidates per 1080p terrain pixel, weights included: about
+// 900 instructions per candidate, a quarter of them the stream). A stream of at most 155 draws
+// takes no branch per draw and needs no spill block: 1.64 -> 1.42 ms, 512 x 512 boxes with 8
+// candidates 0.119 -> 0.105, textured 960 x 540 0.417 -> 0.368.
+//
+// Shape: four blocks of 128 (128 registers, nothing spilled). Five (96 registers): 1.45, 0.115,
+// 0.416 ms; six (80): 1.41, 0.117, 0.415.
 constexpr int kGenerateThreads = 128;
+template <class Rng>  // MtShort where draws_to_generation_end is at most 155
 __global__ void __launch_bounds__(kGenerateThreads, 4)
     ris_generate_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ CameraD cam, int frame_arg,
                         const __grid_constant__ PathRun pr, const __grid_constant__ RisRun ris,
                         const __grid_constant__ GBufferView gb, const __grid_constant__ WaveBuffers wb, float4 *color,
                         int trace_level, unsigned *err) {
     uint64_t spill[312];
-    MtStream rng;
+    Rng rng;
     PixelStart ps;
     if (!pixel_start<kGenerateThreads>(s, cam, live_frame(cam, frame_arg), gb, rng, spill, ps)) return;
     const size_t i = ps.i;
@@ -148,7 +153,7 @@ __global__ void __launch_bounds__(kGenerateThreads, 4)
             BounceState st2{0, 0};
             bounce_draws(bd, 1, 1, st2, rng);
         }
-        store_stream_from(wb.rng_state, i, wb.pixels, rng, ps.s156, k0);
+        store_stream_from(wb.rng_state, i, wb.pixels, whole_stream(rng), ps.s156, k0);
         return;
     }
     for (int k = 0; k < n_fresh; ++k) {
@@ -161,7 +166,7 @@ __global__ void __launch_bounds__(kGenerateThreads, 4)
             wb.q_closest[2 * (size_t)q + 1] = make_float4(b.dir.x, b.dir.y, b.dir.z, 0.0f);
         }
     }
-    store_stream_from(wb.rng_state, i, wb.pixels, rng, ps.s156, k0);
+    store_stream_from(wb.rng_state, i, wb.pixels, whole_stream(rng), ps.s156, k0);
 }
 
 __device__ __forceinline__ TracedResults traced_results(const DeviceScene &s, const RisRun &ris, const WaveBuffers &wb,
@@ -386,12 +391,19 @@ RisRun ris_run(const RisParamsD &p) {
     ris.reproj = p.reproj;
     return ris;
 }
+// Most draws of a pixel up to the end of generation: pixel and lens 4, wavelengths 1, 3 per
+// light candidate, 5 per bounce.
+int draws_to_generation_end(const RisParamsD &p) {
+    const int n_nee = smaxi(1, p.candidate_count / 2), n_bsdf = smaxi(0, p.candidate_count - n_nee);
+    return 5 + 3 * n_nee + 5 * (n_bsdf + 1);
+}
 }  // namespace
 
 int launch_ris_generate(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
                         GBufferView gb, WaveBuffers wb, float4 *color, int trace_level, unsigned *err,
                         cudaStream_t st) {
-    ris_generate_kernel<<<tile_blocks<kGenerateThreads>(cam.width, cam.height), kGenerateThreads, 0, st>>>(
+    auto k = draws_to_generation_end(p) <= 155 ? ris_generate_kernel<MtShort> : ris_generate_kernel<MtStream>;
+    k<<<tile_blocks<kGenerateThreads>(cam.width, cam.height), kGenerateThreads, 0, st>>>(
         s, cam, frame_index, path_run(p), ris_run(p), gb, wb, color, trace_level, err);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
@@ -401,11 +413,9 @@ int launch_ris_shade(const DeviceScene &s, const CameraD &cam, int frame_index, 
                      cudaStream_t st, const TraceTuning &tune) {
     const PathRun pr = path_run(p);
     const RisRun ris = ris_run(p);
-    // Draws up to the end of generation: pixel and lens 4, wavelengths 1, 3 per light candidate,
-    // at most 5 per bounce. The resampling kernel continues a stream it has not replayed, whose
-    // state travels only below draw 312.
-    const int n_nee = smaxi(1, p.candidate_count / 2), n_bsdf = smaxi(0, p.candidate_count - n_nee);
-    const bool lean = trace_level == kTraceNoBsdfRays && 5 + 3 * n_nee + 5 * (n_bsdf + 1) < 312;
+    // The resampling kernel continues a stream it has not replayed, whose state travels only
+    // below draw 312.
+    const bool lean = trace_level == kTraceNoBsdfRays && draws_to_generation_end(p) < 312;
     if (lean) {
         const bool wide = tune.shade_shape < 2;  // 256 threads per block, else 128
         const int blocks = wide ? tile_blocks<256>(cam.width, cam.height) : tile_blocks<128>(cam.width, cam.height);
@@ -425,7 +435,8 @@ int launch_ris_shade(const DeviceScene &s, const CameraD &cam, int frame_index, 
 // gets what the test on the spot would have given it, throughput 0 (so the
 // direct term is 0) and Color = Beer * emission of its surface.
 __global__ void __launch_bounds__(256) ris_winner_fixup_kernel(DeviceScene s, CameraD cam, int frame_arg, PathRun pr,
-                                                              GBufferView gb, ReservoirView rv, const float4 *q,
+                                                              GBufferView gb, ReservoirView rv,
+                                                              const uint4 *rng_state, const float4 *q,
                                                               const int *count, const unsigned char *occ,
                                                               float4 *color) {
     const int frame_index = live_frame(cam, frame_arg);
@@ -434,8 +445,8 @@ __global__ void __launch_bounds__(256) ris_winner_fixup_kernel(DeviceScene s, Ca
         const int px = __float_as_int(q[2 * (size_t)k].w);
         if (!occ[px]) continue;
         const int x = px % cam.width, y = px / cam.width;
-        MtStream rng;
-        rng.init((uint32_t)px ^ (uint32_t)((unsigned long long)frame_index * 12345ULL), nullptr);
+        MtShort rng;
+        rng.init_from(pixel_seed((size_t)px, frame_index), stored_s156(rng_state, (size_t)px));
         const float fx = (float)x + rng.next_float();
         const float fy = (float)y + rng.next_float();
         const RayF ray = camera_ray(cam, fx, fy, rng);
@@ -460,8 +471,8 @@ int launch_winner_visibility(const DeviceScene &s, const CameraD &cam, int frame
                              cudaStream_t st, const TraceTuning &tune) {
     if (hdr::launch_shadow_queue(s, wb.q_winner, wb.pixels, wb.counts + 4, wb.counts + 5, wb.occ_winner, tune, err, st) < 0)
         return -1;
-    ris_winner_fixup_kernel<<<tune.sm_count * 4, 256, 0, st>>>(s, cam, frame_index, path_run(p), gb, rv, wb.q_winner,
-                                                               wb.counts + 4, wb.occ_winner, color);
+    ris_winner_fixup_kernel<<<tune.sm_count * 4, 256, 0, st>>>(s, cam, frame_index, path_run(p), gb, rv, wb.rng_state,
+                                                               wb.q_winner, wb.counts + 4, wb.occ_winner, color);
     return cudaPeekAtLastError() == cudaSuccess ? 2 : -1;
 }
 
