@@ -17,10 +17,9 @@
 //
 // Parity mode therefore runs the parallel clamp, checks on the device whether any
 // pixel's result changes under the in-place order (only in tiles that hold such a
-// pixel, breaks_order), and hands the frame to
-// `firefly_sequential_kernel` only when one does. That kernel reads the check's flag
-// itself and returns at once when it is clear, so no mode reads anything back to the
-// host or waits for the stream.
+// pixel, breaks_order), and clamps the frame exactly (firefly_sequential) only when one
+// does. The kernel of the mean reads the check's flag itself, so no mode reads anything back
+// to the host or waits for the stream.
 //
 // The clamp, its check and the sum are one pass over the frame (firefly_sum_kernel), the
 // mean a second one: neighbours still read the unclamped colour while the first runs.
@@ -205,22 +204,14 @@ __global__ void __launch_bounds__(kTileThreads)
     }
 }
 
-// The row-major in-place clamp, exactly, in one block, run only when the check
-// set *changed (else it returns at once). Pixel (x, y) depends on its earlier
+// The row-major in-place clamp, exactly, by one block. Pixel (x, y) depends on its earlier
 // neighbours (x-1, y), (x-1, y-1), (x, y-1), (x+1, y-1) (or on itself, at the
 // border), and all of them lie on earlier anti-diagonals t = x + 2y. So the
 // block walks t = 0 .. (w-1) + 2(h-1), computes every pixel of one diagonal in
 // parallel from the final values of earlier ones (in `plane`) and the
 // unclamped values of later ones (in `orig`), and meets at a barrier before the
 // next diagonal. Bounded: w + 2h - 2 steps, each at most min(h, w/2 + 1) pixels.
-// The sums are then taken again from the unchanged accum.
-__global__ void __launch_bounds__(1024) firefly_sequential_kernel(const float4 *__restrict__ orig,
-                                                                  const float4 *__restrict__ accum, float4 *plane,
-                                                                  int width, int height, int *changed) {
-    __shared__ int run;
-    if (threadIdx.x == 0) run = *(volatile int *)changed;
-    __syncthreads();
-    if (!run) return;
+__device__ __noinline__ void firefly_sequential(const float4 *orig, float4 *plane, int width, int height) {
     const int t_end = (width - 1) + 2 * (height - 1);
     for (int t = 0; t <= t_end; ++t) {
         // y with 0 <= t - 2y <= width - 1 and 0 <= y <= height - 1
@@ -232,24 +223,38 @@ __global__ void __launch_bounds__(1024) firefly_sequential_kernel(const float4 *
         }
         __syncthreads();
     }
-    for (size_t p = threadIdx.x; p < (size_t)width * height; p += blockDim.x) {
-        const float4 c = plane[p], a = accum[p];
-        plane[p] = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, a.w + c.w);
-    }
 }
 
-// The mean, and the sums in their place (sums may be accum itself: kCopy false). From the last
-// pixel down: the sums written last are still in L2.
-template <bool kCopy>
-__global__ void __launch_bounds__(256) mean_kernel(const float4 *__restrict__ sums, float4 *accum,
-                                                   float4 *__restrict__ out, size_t count, float inv_n,
-                                                   const int *frame_slot) {
+__device__ __forceinline__ float4 mean_of(float4 a, float inv_n) {
+    return make_float4(a.x * inv_n, a.y * inv_n, a.z * inv_n, a.w * inv_n);
+}
+
+// The mean, and the sums in their place (kParity; else sums is accum itself). From the last
+// pixel down: the sums written last are still in L2. kParity: where the check set *changed the
+// first block does the frame's exact clamp, sums and mean from the unchanged accum and colours
+// (`out` still holds them), and the others have nothing to do; a kernel of its own for that,
+// which almost always only read the flag, took 2.6 us of every frame.
+template <bool kParity>
+__global__ void __launch_bounds__(1024, 2) mean_kernel(float4 *sums, float4 *accum, float4 *out, int width, int height,
+                                                       float inv_n, const int *frame_slot, const int *changed) {
     if (frame_slot) inv_n = 1.0f / (float)(*frame_slot + 1);
+    const size_t count = (size_t)width * height;
+    if (kParity && *changed) {  // the same for every thread
+        if (blockIdx.x != 0) return;
+        firefly_sequential(out, sums, width, height);
+        for (size_t p = threadIdx.x; p < count; p += blockDim.x) {
+            const float4 c = sums[p], b = accum[p];
+            const float4 a = make_float4(b.x + c.x, b.y + c.y, b.z + c.z, b.w + c.w);
+            accum[p] = a;
+            out[p] = mean_of(a, inv_n);
+        }
+        return;
+    }
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) {
         const size_t i = count - 1 - k;
         const float4 a = sums[i];
-        if (kCopy) accum[i] = a;
-        out[i] = make_float4(a.x * inv_n, a.y * inv_n, a.z * inv_n, a.w * inv_n);
+        if (kParity) accum[i] = a;
+        out[i] = mean_of(a, inv_n);
     }
 }
 
@@ -282,23 +287,23 @@ int launch_accumulate(float4 *color, float4 *accum, float4 *scratch, int *flag_d
     cudaError_t e = cudaSuccess;
     const int blocks = (int)std::max<size_t>(1, std::min<size_t>((count + 255) / 256, (size_t)148 * 8));
     if (firefly) {
+        const int mean_blocks = (int)std::max<size_t>(1, std::min<size_t>((count + 1023) / 1024, (size_t)148 * 2));
         const unsigned grid =
             (unsigned)((size_t)((width + kTileW - 1) / kTileW) * (size_t)((height + kTileH - 1) / kTileH));
         if (mode == 0) {
-            // the in-place-order check, then the exact in-place clamp when it failed
             if ((e = cudaMemsetAsync(flag_dev, 0, sizeof(int), st)) != cudaSuccess) {
                 if (err) *err = e;
                 return -1;
             }
             firefly_sum_kernel<true><<<grid, kTileThreads, 0, st>>>(color, accum, scratch, width, height, flag_dev);
-            firefly_sequential_kernel<<<1, 1024, 0, st>>>(color, accum, scratch, width, height, flag_dev);
-            mean_kernel<true><<<blocks, 256, 0, st>>>(scratch, accum, color, count, inv_n, frame_slot);
-            launches += 3;
+            mean_kernel<true><<<mean_blocks, 1024, 0, st>>>(scratch, accum, color, width, height, inv_n, frame_slot,
+                                                            flag_dev);
         } else {
             firefly_sum_kernel<false><<<grid, kTileThreads, 0, st>>>(color, accum, accum, width, height, nullptr);
-            mean_kernel<false><<<blocks, 256, 0, st>>>(accum, accum, color, count, inv_n, frame_slot);
-            launches += 2;
+            mean_kernel<false><<<mean_blocks, 1024, 0, st>>>(accum, accum, color, width, height, inv_n, frame_slot,
+                                                             nullptr);
         }
+        launches += 2;
     } else {
         accumulate_kernel<<<blocks, 256, 0, st>>>(color, accum, color, count, inv_n, frame_slot);
         ++launches;

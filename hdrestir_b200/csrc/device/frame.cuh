@@ -233,6 +233,8 @@ void launch_trace_stats(const DeviceScene &s, const float *rays, const float *tm
 void launch_rng_floats(const uint32_t *seeds, int n, int count, float *out, cudaStream_t st);
 void launch_ris_path_trace(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
                            GBufferView gb, ReservoirView res, float4 *color, unsigned *err, cudaStream_t st);
+constexpr int kPtRounds = 64, kPtCounts = 8;  // blocks of counters, counters of a round
+constexpr int kPtActive = 4;                  // the one that counts the round's live paths
 // Per-path state of the wavefront PathTracePass (pathtrace.cu), one entry
 // per pixel, plus its ray queues and hit slots (slot = pixel index).
 struct PtBuffers {
@@ -243,9 +245,8 @@ struct PtBuffers {
     float4 *nee_add;        // the vertex's NEE term, added if its shadow ray is unoccluded
     int4 *state;            // BounceState refl, refr; flags; the path's image
     int *active[2];         // live-path lists (ping-pong)
-    int *active_count[2];   // their lengths
-    int *counts;            // [0..3] queue lengths and fetch counters
-    int *all_counts;        // active_count[1], counts[0..3], active_count[0]: a round clears five in a row
+    int *counts;            // [0..3] queue lengths and fetch counters, [kPtActive]: of the round a kernel fills
+    int *round_counts;      // kPtRounds x kPtCounts: the counts of round v are block v % kPtRounds
     float4 *q_closest, *q_shadow, *hits;
     float *hit_v;
     unsigned char *occ;

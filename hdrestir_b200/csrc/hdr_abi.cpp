@@ -1386,7 +1386,8 @@ hdr_status pt_buffers_from(Alloc alloc, size_t count, hdr::PtBuffers &B) {
         {"__pt_rng", count * 48, &rng},     {"__pt_tp", count * 16, &tp},       {"__pt_total", count * 16, &total},
         {"__pt_outer", count * 16, &outer}, {"__pt_b_origin", count * 16, &bo}, {"__pt_b_dir", count * 16, &bd},    {"__pt_b_tmul", count * 16, &bt},
         {"__pt_nee", count * 16, &nee},     {"__pt_state", count * 16, &state}, {"__pt_active0", count * 4, &a0},
-        {"__pt_active1", count * 4, &a1},   {"__pt_counts", 32, &cnt},          {"__pt_q_closest", count * 32, &qc},
+        {"__pt_active1", count * 4, &a1},   {"__pt_counts", sizeof(int) * hdr::kPtRounds * hdr::kPtCounts, &cnt},
+        {"__pt_q_closest", count * 32, &qc},
         {"__pt_q_shadow", count * 32, &qs}, {"__pt_hits", count * 16, &hits},   {"__pt_hit_v", count * 4, &hv},
         {"__pt_occ", count, &occ}};
     hdr_status st;
@@ -1403,10 +1404,7 @@ hdr_status pt_buffers_from(Alloc alloc, size_t count, hdr::PtBuffers &B) {
     B.state = (int4 *)state;
     B.active[0] = (int *)a0;
     B.active[1] = (int *)a1;
-    B.all_counts = (int *)cnt;
-    B.active_count[1] = B.all_counts;
-    B.counts = B.all_counts + 1;
-    B.active_count[0] = B.all_counts + 5;
+    B.round_counts = (int *)cnt;
     B.q_closest = (float4 *)qc;
     B.q_shadow = (float4 *)qs;
     B.hits = (float4 *)hits;

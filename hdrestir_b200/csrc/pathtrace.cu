@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) pt_start_kernel(const __grid_constant__ D
     B.tp[i] = f4(spec(1.0f));
     BounceState st{0, 0};
     sample_vertex(s, B, i, sf, st, sc, rng, pr, 0, u, jk);
-    active_append(B.active_count[0], B.active[0], true, (int)i);
+    active_append(B.counts + kPtActive, B.active[0], true, (int)i);
 }
 
 // vertex v of the paths in `list`: the vertex's direct light, then the path goes
@@ -284,13 +284,15 @@ int launch_path_trace_wavefront(const DeviceScene &s, const PtJobD *jobs, int n_
     const bool batch = n_jobs > 1;
     const PathRun pr = jobs[0].pr;
     int launches = 0;
-    if (cudaMemsetAsync(B.all_counts, 0, 6 * sizeof(int), st) != cudaSuccess) return -1;
+    // A round has counters of its own: one memset for kPtRounds rounds, not one for each
+    if (cudaMemsetAsync(B.round_counts, 0, kPtRounds * kPtCounts * sizeof(int), st) != cudaSuccess) return -1;
+    const auto counts_of = [&](int v) { return B.round_counts + (size_t)(v % kPtRounds) * kPtCounts; };
+    B.counts = counts_of(0);
     (batch ? pt_start_kernel<true> : pt_start_kernel<false>)<<<total_tiles, 256, 0, st>>>(s, jobs[0], table, n_jobs, B);
     ++launches;
     WaveBuffers wb{};
     wb.q_closest = B.q_closest;
     wb.q_shadow = B.q_shadow;
-    wb.counts = B.counts;
     wb.closest_slots = wb.shadow_slots = B.pixels;
     wb.hits = B.hits;
     wb.hit_v = B.hit_v;
@@ -298,17 +300,24 @@ int launch_path_trace_wavefront(const DeviceScene &s, const PtJobD *jobs, int n_
     const int grid = (int)std::min<size_t>((size_t)tune.sm_count * 16, (B.pixels + kPtThreads - 1) / kPtThreads);
     for (int v = 0; v < pr.max_depth; ++v) {
         const int cur = v & 1, nxt = cur ^ 1;
+        wb.counts = counts_of(v);
         const int t = launch_wave_trace(s, wb, tune, err, st);
         if (t < 0) return -1;
         launches += t;
-        // the queues of the next vertex and its active list start empty
-        if (cudaMemsetAsync(nxt ? B.all_counts : B.counts, 0, 5 * sizeof(int), st) != cudaSuccess) return -1;
+        // past the last block all others start again at zero, and that one a round later
+        if ((v + 1) % kPtRounds == 0 &&
+            cudaMemsetAsync(B.round_counts, 0, (kPtRounds - 1) * kPtCounts * sizeof(int), st) != cudaSuccess)
+            return -1;
+        if (v > 0 && v % kPtRounds == 0 &&
+            cudaMemsetAsync(counts_of(v - 1), 0, kPtCounts * sizeof(int), st) != cudaSuccess)
+            return -1;
+        B.counts = counts_of(v + 1);
         // Draws when the round ends: 5 for the pixel, 5 and 3 for a vertex's samples, roulette
         const bool few = 5 + 8 * std::min(v + 2, pr.max_depth) + (v + 1) <= 155;
         auto connect = few ? (batch ? pt_connect_kernel<true, MtShort> : pt_connect_kernel<false, MtShort>)
                            : (batch ? pt_connect_kernel<true, MtStream> : pt_connect_kernel<false, MtStream>);
         connect<<<grid, kPtThreads, 0, st>>>(
-            s, jobs[0], table, pr, B, B.active[cur], B.active_count[cur], B.active[nxt], B.active_count[nxt], v, err);
+            s, jobs[0], table, pr, B, B.active[cur], wb.counts + kPtActive, B.active[nxt], B.counts + kPtActive, v, err);
         ++launches;
     }
     return cudaPeekAtLastError() == cudaSuccess ? launches : -1;

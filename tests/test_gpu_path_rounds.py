@@ -46,3 +46,25 @@ def test_rounds_equal_one_thread_form(kind, w, h, depth):
         path_trace_batch([a, c], [cam, cam], [0, 7], max_depth=depth)
         for ctx, img in zip((a, c), want):
             assert np.array_equal(ctx.download("Color").view(np.uint32), img.view(np.uint32))
+
+
+@pytest.mark.parametrize("depth", [63, 64, 65, 66, 130])
+def test_many_rounds(depth):
+    """A lightless box of mirrors with one glowing material: two draws a vertex, so paths live
+    for 122 rounds, past the rounds' last block of counters."""
+    from hdrestir_b200.context import Context
+    sc, cam = configs.config0(24, 17)
+    sc.lights = []
+    for k, m in enumerate(sc.materials):
+        m.metallic, m.roughness, m.diffuse_color = 1.0, 0.0, (1.0, 1.0, 1.0)
+        m.emission = 0.5 if k == 0 else 0.0
+    images = []
+    for one in (False, True):
+        with Context(device=0, pt_one_kernel=one) as ctx:
+            ctx.upload_scene(sc)
+            ctx.raycast(cam, 3)
+            for _ in range(2):  # the counters a frame leaves are the next frame's start
+                ctx.path_trace(cam, 3, max_depth=depth, max_reflection_bounces=1000, roulette_aggressiveness=1e6)
+            images.append(ctx.download("Color").copy())
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
+    assert np.abs(images[0][:, :3]).sum() > 0
