@@ -31,9 +31,9 @@
 //    resolves it again.
 //  * neither mode reads anything back to the host or waits for the stream: the
 //    in-place-order check and its fallback run on the device.
-//  * nothing in the scratch has to start at zero: the clamp pass writes the
-//    plane in full before anything reads it, and the flag is zeroed on the
-//    stream before every use. The caller's accum plane must be zero before
+//  * nothing in the scratch has to start at zero: the pass writes the plane
+//    (the frame's sums) in full before anything reads it, and the flag is zeroed
+//    on the stream before every use. The caller's accum plane must be zero before
 //    frame 0, as "__accum_color" is after hdr_clear_persistent.
 //  * one scratch per device, shared by all callers: calls that overlap on the
 //    same device (different streams or host threads) race on it. Serialise
@@ -56,7 +56,7 @@ namespace {
 
 constexpr size_t kNoAllocMaxPixels = size_t(1) << 21;
 
-// one plane of kNoAllocMaxPixels RGBA f32 (the clamped frame)
+// one plane of kNoAllocMaxPixels RGBA f32 (the frame's sums)
 static __device__ __align__(256) float4 g_accum_scratch[kNoAllocMaxPixels];
 static __device__ __align__(256) int g_accum_flag[64];
 

@@ -64,7 +64,7 @@ struct DeviceScene {
     int has_textures;          // 1: some material has a texture (closures read uv and tangents)
     // shadow-ray BVH (host/shadow_bvh.h): 4-wide SAH trees over the same triangles,
     // walked for "hit nearer than the limit" queries when sh4 is 1
-    const float4 *sh4_nodes;   // 8 per node
+    const float4 *sh4_nodes;   // 4 per node (sh4_layout.h)
     const float4 *sh4_tris;    // 3 per triangle (tri_geo records in leaf order)
     const int *sh4_inst_root;  // per instance: its mesh's root node, -1 = no triangles
     const int *sh4_inst_rank;  // per instance: its position in the reference TLAS's leaf order

@@ -1202,8 +1202,8 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
     // wavefront form: direct light only (no later bounces), no stochastic opacity, no physical
     // sky (its sun technique is served by the one-kernel form only) and no blackbody lights
     // (an extension the wavefront kernels are built without, to keep their registers)
-    const bool wave = p->path.max_depth == 1 && c->scene_opaque && !c->scene.sky && !c->scene.blackbody &&
-                      !(p->flags & HDR_RIS_ONE_KERNEL);
+    bool wave = p->path.max_depth == 1 && c->scene_opaque && !c->scene.sky && !c->scene.blackbody &&
+                !(p->flags & HDR_RIS_ONE_KERNEL);
     const bool spatial = p->spatial_neighbors > 0 && p->use_reservoir;
     if (spatial && !wave)
         return fail(HDR_EINVAL, "spatial reuse runs in the wavefront form only (max_depth 1, opaque scene)");
@@ -1283,11 +1283,11 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         float4 *r = (float4 *)q;
         rv_spatial = hdr::ReservoirView{r, r + count, r + 2 * count, r + 3 * count, r + 4 * count};
     }
+    hdr::WaveBuffers wb{};
+    const int trace_level = ris_trace_level(c, p);
     if (wave) {
         const int n_nee = std::max(1, p->candidate_count / 2);
         const int n_bsdf = std::max(0, p->candidate_count - n_nee);
-        const int trace_level = ris_trace_level(c, p);
-        hdr::WaveBuffers wb{};
         wb.pixels = count;
         wb.n_closest = closest_slots(trace_level, n_bsdf);
         wb.n_shadow = n_nee;
@@ -1306,9 +1306,6 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         wb.hit_v = (float *)q;
         if ((st = ensure_buffer(c, "__wave_occ", count * wb.n_shadow, &q)) != HDR_OK) return st;
         wb.occ = (unsigned char *)q;
-        if ((st = ensure_scratch(c, "__wave_nee_weight", count * wb.n_shadow * nee_weight_size(p), &q)) != HDR_OK)
-            return st;
-        wb.nee_weight = q;
         if ((st = ensure_buffer(c, "__wave_rng", count * 48, &q)) != HDR_OK) return st;
         wb.rng_state = (uint4 *)q;
         if ((st = ensure_buffer(c, "__wave_done", count, &q)) != HDR_OK) return st;
@@ -1323,6 +1320,15 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
             if ((st = ensure_buffer(c, "__wave_occ_winner", count, &q)) != HDR_OK) return st;
             wb.occ_winner = (unsigned char *)q;
         }
+        // Last, since a frame for which only the weights have no room (a budget, a recording that
+        // cannot allocate) renders in the one-kernel form, which gives the same image.
+        st = ensure_scratch(c, "__wave_nee_weight", count * wb.n_shadow * nee_weight_size(p), &q);
+        wb.nee_weight = q;
+        wave = st == HDR_OK;
+        if (!wave && ((st != HDR_ENOMEM && !c->recording) || spatial || tune || (c->flags & HDR_CTX_RECORD_LIGHTS)))
+            return st;
+    }
+    if (wave) {
         if ((st = begin_pass(c, 1)) != HDR_OK) return st;
         const bool timed = timing_on(c);
         if (timed)

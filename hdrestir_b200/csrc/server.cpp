@@ -51,7 +51,8 @@ size_t pixels_of(const hdr_job_desc &d) { return (size_t)d.camera.width * (size_
 // Device bytes a job's context allocates, per pixel: GBuffer 96, Color 16,
 // accumulator 16, firefly scratch 16; RIS adds the reservoir (80), the
 // stream state and done flag (49) and its share of the batch's ray queues and
-// result slots (52 per closest-hit slot, 33 per shadow slot).
+// result slots (52 per closest-hit slot, 33 per shadow slot). The light candidates' weights
+// (4 or 8 each) stay within the closest-hit slots a default frame is charged for and does not allocate.
 size_t job_bytes(const hdr_job_desc &d) {
     const size_t px = pixels_of(d);
     size_t per = 96 + 16 + 16 + (d.firefly ? 16 : 0);

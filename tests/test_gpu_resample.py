@@ -56,3 +56,56 @@ def test_resampling_equals_one_kernel_form(scene, width, height, candidates, res
             got = _frames(ctx, cam, 3, **ris)
             assert all(np.array_equal(a.view(np.uint32), b.view(np.uint32)) for a, b in zip(got, want))
         assert any(np.abs(a[:, :3]).sum() > 0 for a in want if a.ndim == 2)
+
+
+def test_budget_without_room_for_the_weights():
+    """A frame for which everything but the light candidates' weights fits the context's budget
+    renders all the same, with the same image; with nothing to spare it is refused."""
+    from hdrestir_b200.context import Context
+    sc, cam = SCENES["terrain"](64, 48)
+    ris = dict(candidate_count=32, use_reservoir=True, skip_visibility=False)
+
+    def frames(budget):
+        with Context(device=0, hbm_budget=budget) as ctx:
+            try:
+                ctx.upload_scene(sc)
+                out = _frames(ctx, cam, 2, **ris)
+            except RuntimeError:
+                return None, None
+            try:
+                return out, ctx.buffer_size("__wave_nee_weight")
+            except RuntimeError:
+                return out, 0
+
+    want, weights = frames(0)
+    assert weights == 64 * 48 * 16 * 4
+    lo, hi = 1, 1 << 28  # refused, enough
+    assert frames(lo)[0] is None
+    while hi - lo > 1024:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if frames(mid)[0] is not None else (mid, hi)
+    for budget, held in ((hi, 0), (hi + weights // 2, 0), (hi + weights, weights)):
+        got, have = frames(budget)
+        assert have == held
+        assert all(np.array_equal(a.view(np.uint32), b.view(np.uint32)) for a, b in zip(got, want))
+
+
+def test_recording_whose_weights_cannot_grow():
+    """Recorded after frames with a reservoir, a frame without one needs larger weights, which a
+    recording cannot allocate: it is recorded in the one-kernel form."""
+    from hdrestir_b200.context import Context
+    sc, cam = SCENES["boxes"](40, 24)
+    ris = dict(candidate_count=16, max_depth=1, skip_visibility=False)
+    with Context(device=0) as ctx, Context(device=0) as plain:
+        for c in (ctx, plain):
+            c.upload_scene(sc)
+            c.raycast(cam, 0)
+        ctx.ris_path_trace(cam, 0, use_reservoir=True, **ris)
+        ctx.graph_begin()
+        ctx.raycast(cam, 1)
+        ctx.ris_path_trace(cam, 1, use_reservoir=False, **ris)
+        ctx.graph_end()
+        ctx.graph_launch(1)
+        plain.raycast(cam, 1)
+        plain.ris_path_trace(cam, 1, use_reservoir=False, **ris)
+        assert np.array_equal(ctx.download("Color").view(np.uint32), plain.download("Color").view(np.uint32))
