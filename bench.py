@@ -44,9 +44,9 @@ METRIC = "ReSTIR 1080p frames/s"
 # reservoir write 80 B + GBuffer read 64 B + colour write 16 B (five float4 reservoir planes,
 # four float4 GBuffer planes)
 INTEGRATE_BYTES_PER_PX = 80 + 80 + 64 + 16
-# accumulation: colour in 16 + accum in 16 + accum out 16 + colour out 16, plus the firefly
-# clamp and its check (colour in 16 + clamped out 16; clamped in 16 + colour in 16)
-ACCUM_BYTES_PER_PX = 64 + 32 + 32
+# accumulation: colour in 16 + accum in 16 + accum out 16 + colour out 16, plus the sums, which
+# pass through a plane of their own (16 out, 16 in) until the firefly clamp's check has run
+ACCUM_BYTES_PER_PX = 64 + 32
 # trace_shadow4_kernel, the dominant kernel: per shadow ray it must read its queue record
 # (origin, slot, direction, limit: 32 B) and write one occlusion byte; the BVH and the
 # triangles it reads are the scene's, shared by all rays of the launch
