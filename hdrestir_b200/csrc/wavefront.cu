@@ -63,7 +63,8 @@ __device__ __forceinline__ int queue_append(int *counter, bool want) {
 // WaveBuffers::done of a pixel
 constexpr int kPixelMiss = 1;     // no GBuffer hit: its colour is written
 constexpr int kPixelConn = 2;     // the path's bounce is a candidate (its pdf is above 0)
-constexpr int kPixelConnNan = 4;  // and its pdf squared overflows: its weight is a NaN
+constexpr int kPixelConnNan = 4;  // and its pdf squared overflows: its weight is a NaN (power_heuristic3
+                                  // with a count of 0 in front of it is 0)
 
 // Kernel parameters of struct type are __grid_constant__: code that takes their
 // address (a reference kept in a struct, a call) reads the parameter space
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(kGenerateThreads, 4)
     const int N = ris.candidate_count;
     const int n_nee = smaxi(1, N / 2), n_bsdf = smaxi(0, N - n_nee);
     const bool conn = fb.ok && fb.pdf > 0.0f;
-    wb.done[i] = (unsigned char)((conn ? kPixelConn : 0) | (conn && isinf(fb.pdf * fb.pdf) ? kPixelConnNan : 0));
+    wb.done[i] = (unsigned char)((conn ? kPixelConn : 0) | (conn && n_bsdf > 0 && isinf(fb.pdf * fb.pdf) ? kPixelConnNan : 0));
     const uint32_t k0 = rng.k;
     const RisStrategy strat{n_nee, 0, n_bsdf, ris.skip_vis};
     for (int j = 0; j < n_nee; ++j) {
