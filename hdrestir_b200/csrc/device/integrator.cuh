@@ -99,8 +99,8 @@ struct TraceNow {
 };
 
 // A candidate's weight is mis * target / pdf; an occluded one has target 0 and so weight 0,
-// except that 0 times an infinite or undefined mis is a NaN, which the reference lets into the
-// reservoir's sum. Such a weight is stored with all its lower bits set and stays when the
+// except that 0 times an undefined mis, or over an undefined pdf, is a NaN, which the reference
+// lets into the reservoir's sum. Such a weight is stored with all its lower bits set and stays when the
 // candidate is occluded; any other NaN is stored with one bit set.
 __device__ __forceinline__ bool nee_weight_stays(float w) { return __float_as_uint(w) == 0x7fffffffu; }
 __device__ __forceinline__ bool nee_weight_stays(double w) {
@@ -436,7 +436,8 @@ struct RisNeeRay {  // a light candidate as the generate kernel leaves it
 // A light candidate's shadow ray and its weight (_generateNEECandidates, :553-589, with
 // _evaluateLightSample, :628-673): the values ris_nee_candidate computes after the trace.
 // A candidate that the early-outs drop weighs 0 whatever its densities are, unless the
-// light's density squared overflows (mis is then undefined): only then are they evaluated.
+// light's density is a NaN (an environment with an infinite texel) or its square overflows (mis
+// is then undefined): only then are they evaluated.
 __device__ __forceinline__ RisNeeRay ris_nee_ray(const DeviceScene &s, const Surface &sf, int li,
                                                  const LightSampleD &ls, const RisStrategy &strat,
                                                  const SpectralCtx &sc) {
@@ -453,7 +454,7 @@ __device__ __forceinline__ RisNeeRay ris_nee_ray(const DeviceScene &s, const Sur
     r.limit = ls.dist - 1e-3f;
     r.weight = 0.0;
     r.stays = false;
-    if (dropped && (delta || !isinf(p_nee * p_nee))) return r;
+    if (dropped && isfinite(p_nee * p_nee)) return r;
     const V3 wo = -sf.ray_d;
     const float mis = delta ? 1.0f
                             : power_heuristic3(p_nee, strat.n_nee, 0.0f, strat.n_sky,
@@ -464,7 +465,7 @@ __device__ __forceinline__ RisNeeRay ris_nee_ray(const DeviceScene &s, const Sur
         target = spectrum_luminance(light_emission(s, li, ls.color, sc) * rgb_to_spectrum(bval * n_l, sc.up), sc.cie);
     }
     r.weight = (double)(mis * target) / ((double)p_nee + 1e-9);
-    r.stays = !isfinite(mis);
+    r.stays = !isfinite(mis) || isnan(p_nee);
     return r;
 }
 

@@ -2,11 +2,13 @@
 light candidate's weight before its shadow ray is cast and does not evaluate the path's bounce,
 equals the one-kernel form, which evaluates every candidate after its ray. Near-mirror lobes
 (a density that is infinite when the half vector rounds to the normal), throughputs and
-emissions past the largest float, lights whose density overflows."""
+emissions past the largest float, environments with an infinite or undefined texel, lights whose
+density overflows."""
 import numpy as np
 import pytest
 
-from hdrestir_b200 import configs
+from hdrestir_b200 import abi, configs
+from hdrestir_b200.scene import Light
 
 pytestmark = pytest.mark.gpu
 
@@ -27,12 +29,23 @@ def _lights(**values):
     return sc, cam
 
 
+def _dome(texel):
+    sc, cam = configs.config1(61, 43, n_lights=4)
+    tex = np.random.default_rng(3).uniform(0.1, 1.0, (8, 16, 3)).astype(np.float32)
+    tex[2, 5] = texel
+    sc.lights.append(Light(abi.LIGHT_DOME, color=(1.0, 1.0, 1.0), intensity=1.0, texture=tex))
+    return sc, cam
+
+
 SCENES = {
     "mirror_0.005": lambda: _materials(metallic=1.0, roughness=0.005),
     "mirror_0.012": lambda: _materials(metallic=1.0, roughness=0.012),
     "coat_0.005": lambda: _materials(coat=1.0, coat_roughness=0.005, coat_ior=3.0),
     "sheen_0.004": lambda: _materials(sheen=1.0, sheen_roughness=0.004),
     "colour_3e38": lambda: _materials(diffuse_color=(3e38, 1.0, 1.0)),
+    "dome_inf": lambda: _dome(np.inf),
+    "dome_nan": lambda: _dome(np.nan),
+    "dome_3e38": lambda: _dome(3e38),
     "light_inf": lambda: _lights(intensity=np.inf),
     "light_3e38": lambda: _lights(intensity=3e38),
     "light_tiny": lambda: _lights(width=1e-20, height=1e-20),
