@@ -27,8 +27,11 @@ struct PrimBox {
     float lo[3], hi[3], c[3];
 };
 
-// Coordinates the node encoding holds; beyond them the reference's trees are walked.
-constexpr float kSh4MaxBound = 1e30f;
+// Coordinates the node encoding serves; beyond them the reference's trees are walked. The walk
+// multiplies a node's scale, 128.5 times its extent, by up to 1e20 (sh4_axis's reciprocal of a
+// direction along which the ray does not move): 2.7e18 * 1e20 stays below the largest float, so
+// that scale and origin do not overflow one without the other.
+constexpr float kSh4MaxBound = 1e16f;
 inline bool encodable(const float *lo, const float *hi) {
     for (int k = 0; k < 3; ++k)
         if (!(std::fabs(lo[k]) < kSh4MaxBound) || !(std::fabs(hi[k]) < kSh4MaxBound)) return false;
