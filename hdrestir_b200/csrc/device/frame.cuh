@@ -100,7 +100,8 @@ struct WaveBuffers {
     float *hit_v;         // pixels * n_closest
     unsigned char *occ;   // n_shadow planes of pixels
     // n_shadow planes of pixels: each light candidate's resampling weight if its shadow ray is
-    // unoccluded (float with a reservoir, double without; nee_weight_bits)
+    // unoccluded (float with a reservoir, double without; nee_weight_bits); nullptr: no room for
+    // them, the shade kernel evaluates the candidates again
     void *nee_weight;
     uint4 *rng_state;     // 3 planes of pixels: stream state at the end of candidate generation
                           // (store_stream_from)

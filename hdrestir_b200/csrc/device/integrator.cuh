@@ -118,8 +118,10 @@ __device__ __forceinline__ double nee_weight_bits<double>(double w, bool stays) 
                                       : (isnan(w) ? 0x7ff8000000000000ll : __double_as_longlong(w)));
 }
 
+// kWeights: the generate kernel stored the light candidates' weights (else they are evaluated again).
+template <bool kWeights>
 struct TracedResults {
-    static constexpr bool kNeeWeights = true;  // the generate kernel evaluated the light candidates
+    static constexpr bool kNeeWeights = kWeights;
     __device__ __forceinline__ int last_bounce_slot() const { return 0; }
     const DeviceScene *s;
     const float4 *hits;        // this pixel's closest-hit slots: t, instance bits, triangle bits, u

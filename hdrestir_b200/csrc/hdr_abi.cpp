@@ -206,8 +206,10 @@ struct hdr_ctx {
 
 namespace {
 
+bool budget_room(hdr_ctx *c, size_t bytes);
+
 hdr_status dev_alloc(hdr_ctx *c, DevBuf &b, size_t bytes) {
-    if (c->budget && c->allocated + bytes > c->budget)
+    if (!budget_room(c, bytes))
         return fail(HDR_ENOMEM, "allocation of %zu bytes exceeds the HBM budget (%zu of %zu in use)", bytes,
                     c->allocated, c->budget);
     void *p = nullptr;
@@ -254,29 +256,48 @@ cudaMemPool_t frame_pool(int device) {
     return p;
 }
 
+void frame_free(hdr_ctx *c, DevBuf &b) {
+    if (b.ptr) cudaFreeAsync(b.ptr, c->stream);
+    c->allocated -= b.bytes;
+    b = DevBuf{};
+}
+
+// The light candidates' weights only make a frame faster (ris_path_trace_pass renders without
+// them too), so they give way to a buffer that something cannot do without. True when any were held.
+constexpr const char *kWeightBuffer = "__wave_nee_weight";
+bool give_back(hdr_ctx *c) {
+    auto it = c->buffers.find(kWeightBuffer);
+    if (it == c->buffers.end()) return false;
+    frame_free(c, it->second);
+    c->buffers.erase(it);
+    return true;
+}
+bool budget_room(hdr_ctx *c, size_t bytes) {
+    auto fits = [&] { return !c->budget || c->allocated + bytes <= c->budget; };
+    return fits() || (give_back(c) && fits());
+}
+
 // A frame buffer of ctx c, allocated and freed in order on the ctx stream (another
 // stream that uses it is ordered after the ctx stream's work and before its later work).
 hdr_status frame_alloc(hdr_ctx *c, DevBuf &b, size_t bytes) {
-    if (c->budget && c->allocated + bytes > c->budget)
+    if (!budget_room(c, bytes))
         return fail(HDR_ENOMEM, "allocation of %zu bytes exceeds the HBM budget (%zu of %zu in use)", bytes,
                     c->allocated, c->budget);
     void *p = nullptr;
     if (bytes) {
         cudaMemPool_t pool = frame_pool(c->device);
         if (!pool) return fail(HDR_ECUDA, "cannot create the frame-buffer memory pool on device %d", c->device);
-        const cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, c->stream);
-        if (e != cudaSuccess) return fail(HDR_ENOMEM, "frame buffer of %zu bytes: %s", bytes, cudaGetErrorString(e));
+        cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, c->stream);
+        if (e != cudaSuccess && give_back(c)) e = cudaMallocFromPoolAsync(&p, bytes, pool, c->stream);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();  // reported here: a frame that goes on without the buffer has not failed
+            return fail(HDR_ENOMEM, "frame buffer of %zu bytes: %s", bytes, cudaGetErrorString(e));
+        }
     }
     b.ptr = p;
     b.bytes = bytes;
     c->allocated += bytes;
     return HDR_OK;
-}
-
-void frame_free(hdr_ctx *c, DevBuf &b) {
-    if (b.ptr) cudaFreeAsync(b.ptr, c->stream);
-    c->allocated -= b.bytes;
-    b = DevBuf{};
 }
 
 // FrameBuffersMap::Add / AddOrGetPersistent: create (zeroed) or resize keeping
@@ -354,7 +375,10 @@ hdr_status ensure_batch_scratch(SceneStore *store, const char *name, size_t byte
     cudaMemPool_t pool = frame_pool(store->device);
     if (!pool) return fail(HDR_ECUDA, "cannot create the frame-buffer memory pool on device %d", store->device);
     const cudaError_t e = cudaMallocFromPoolAsync(&p, want, pool, stream);
-    if (e != cudaSuccess) return fail(HDR_ENOMEM, "batch buffer of %zu bytes: %s", want, cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();  // as in frame_alloc
+        return fail(HDR_ENOMEM, "batch buffer of %zu bytes: %s", want, cudaGetErrorString(e));
+    }
     store->batch_bufs[name] = {p, want};
     store->bytes += want;
     *out = p;
@@ -1202,8 +1226,8 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
     // wavefront form: direct light only (no later bounces), no stochastic opacity, no physical
     // sky (its sun technique is served by the one-kernel form only) and no blackbody lights
     // (an extension the wavefront kernels are built without, to keep their registers)
-    bool wave = p->path.max_depth == 1 && c->scene_opaque && !c->scene.sky && !c->scene.blackbody &&
-                !(p->flags & HDR_RIS_ONE_KERNEL);
+    const bool wave = p->path.max_depth == 1 && c->scene_opaque && !c->scene.sky && !c->scene.blackbody &&
+                      !(p->flags & HDR_RIS_ONE_KERNEL);
     const bool spatial = p->spatial_neighbors > 0 && p->use_reservoir;
     if (spatial && !wave)
         return fail(HDR_EINVAL, "spatial reuse runs in the wavefront form only (max_depth 1, opaque scene)");
@@ -1283,9 +1307,9 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         float4 *r = (float4 *)q;
         rv_spatial = hdr::ReservoirView{r, r + count, r + 2 * count, r + 3 * count, r + 4 * count};
     }
-    hdr::WaveBuffers wb{};
-    const int trace_level = ris_trace_level(c, p);
     if (wave) {
+        hdr::WaveBuffers wb{};
+        const int trace_level = ris_trace_level(c, p);
         const int n_nee = std::max(1, p->candidate_count / 2);
         const int n_bsdf = std::max(0, p->candidate_count - n_nee);
         wb.pixels = count;
@@ -1320,15 +1344,14 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
             if ((st = ensure_buffer(c, "__wave_occ_winner", count, &q)) != HDR_OK) return st;
             wb.occ_winner = (unsigned char *)q;
         }
-        // Last, since a frame for which only the weights have no room (a budget, a recording that
-        // cannot allocate) renders in the one-kernel form, which gives the same image.
-        st = ensure_scratch(c, "__wave_nee_weight", count * wb.n_shadow * nee_weight_size(p), &q);
-        wb.nee_weight = q;
-        wave = st == HDR_OK;
-        if (!wave && ((st != HDR_ENOMEM && !c->recording) || spatial || tune || (c->flags & HDR_CTX_RECORD_LIGHTS)))
+        if (tune && p->use_reservoir && (st = ensure_scratch(c, "__tune_reservoir", count * kResPlanes * sizeof(float4), &q)) != HDR_OK)
             return st;
-    }
-    if (wave) {
+        // Last, since a frame for which only the weights have no room (a budget, a recording that
+        // cannot allocate) renders without them: the same image, its light candidates evaluated
+        // a second time after the trace.
+        st = ensure_scratch(c, kWeightBuffer, count * wb.n_shadow * nee_weight_size(p), &q);
+        if (st != HDR_OK && st != HDR_ENOMEM && !c->recording) return st;
+        wb.nee_weight = st == HDR_OK ? q : nullptr;
         if ((st = begin_pass(c, 1)) != HDR_OK) return st;
         const bool timed = timing_on(c);
         if (timed)
@@ -1716,8 +1739,10 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
     all.hit_v = (float *)q;
     if ((st = ensure_batch_scratch(store, "occ", (size_t)total_s, &q, done, lead->stream)) != HDR_OK) return st;
     all.occ = (unsigned char *)q;
-    if ((st = ensure_batch_scratch(store, "nee_weight", total_w, &q, done, lead->stream)) != HDR_OK) return st;
-    char *weights = (char *)q;
+    // without room for the weights the batch renders without them, as a single frame does
+    st = ensure_batch_scratch(store, "nee_weight", total_w, &q, done, lead->stream);
+    if (st != HDR_OK && st != HDR_ENOMEM) return st;
+    char *weights = st == HDR_OK ? (char *)q : nullptr;
     if (!store->batch_done) HDR_CUDA(cudaEventCreateWithFlags(&store->batch_done, cudaEventDisableTiming));
     // the previous batch on this scene (another lead's stream) has finished with the queues
     HDR_CUDA(cudaStreamWaitEvent(lead->stream, store->batch_done, 0));
@@ -1738,7 +1763,7 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
         wb.hit_v = all.hit_v + base_c[(size_t)i];
         wb.occ = all.occ + base_s[(size_t)i];
         wb.nee_weight = weights;
-        weights += j.weight_bytes;
+        if (weights) weights += j.weight_bytes;
         wb.rng_state = j.rng_state;
         wb.done = j.done;
         wb.pixels = j.count;

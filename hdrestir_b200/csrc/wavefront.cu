@@ -135,10 +135,12 @@ __global__ void __launch_bounds__(kGenerateThreads, 4)
         if (wb.nee_light) wb.nee_light[i * (size_t)wb.n_shadow + j] = proposed ? li : -1;
         if (proposed) ray = ris_nee_ray(s, sf, li, ls, strat, ps.sc);
         const size_t slot = (size_t)j * wb.pixels + i;
-        if (ris.use_reservoir)
+        if (!wb.nee_weight) {
+        } else if (ris.use_reservoir) {
             ((float *)wb.nee_weight)[slot] = nee_weight_bits<float>(ray.weight, ray.stays);
-        else
+        } else {
             ((double *)wb.nee_weight)[slot] = nee_weight_bits<double>(ray.weight, ray.stays);
+        }
         const int q = queue_append(&wb.counts[1], ray.cast);
         if (q >= 0) {
             wb.q_shadow[2 * (size_t)q] =
@@ -170,14 +172,18 @@ __global__ void __launch_bounds__(kGenerateThreads, 4)
     store_stream_from(wb.rng_state, i, wb.pixels, whole_stream(rng), ps.s156, k0);
 }
 
-__device__ __forceinline__ TracedResults traced_results(const DeviceScene &s, const RisRun &ris, const WaveBuffers &wb,
-                                                        int trace_level, size_t i) {
-    return TracedResults{&s, wb.hits + i * (size_t)wb.n_closest, wb.hit_v + i * (size_t)wb.n_closest, wb.occ + i,
-                         (const char *)wb.nee_weight + i * (ris.use_reservoir ? sizeof(float) : sizeof(double)),
-                         wb.pixels, ris.skip_vis, trace_level, wb.q_winner, wb.counts + 4, (int)i};
+template <bool kWeights>
+__device__ __forceinline__ TracedResults<kWeights> traced_results(const DeviceScene &s, const RisRun &ris,
+                                                                  const WaveBuffers &wb, int trace_level, size_t i) {
+    return TracedResults<kWeights>{
+        &s, wb.hits + i * (size_t)wb.n_closest, wb.hit_v + i * (size_t)wb.n_closest, wb.occ + i,
+        (const char *)wb.nee_weight + i * (ris.use_reservoir ? sizeof(float) : sizeof(double)),
+        wb.pixels, ris.skip_vis, trace_level, wb.q_winner, wb.counts + 4, (int)i};
 }
 
-// The general form of a pixel's resampling: every candidate that is not a light's is replayed.
+// The general form of a pixel's resampling: every candidate that is not a light's is replayed,
+// without stored weights the lights' too.
+template <bool kWeights>
 __device__ __forceinline__ void shade_general(const DeviceScene &s, const CameraD &cam, int frame_index,
                                               const PathRun &pr, const RisRun &ris, const GBufferView &gb,
                                               const ReservoirView &rv, const WaveBuffers &wb, float4 *color,
@@ -191,17 +197,18 @@ __device__ __forceinline__ void shade_general(const DeviceScene &s, const Camera
         load_stream_from(wb.rng_state, i, wb.pixels, pixel_seed(i, frame_index), ps.s156, k0);
     ps.i = i;
     pixel_start_at<true>(s, cam, frame_index, gb, x, y, rng, spill, ps);
-    const TracedResults tr = traced_results(s, ris, wb, trace_level, i);
+    const auto tr = traced_results<kWeights>(s, ris, wb, trace_level, i);
     // past 311 draws the state lives in local memory only: replay instead
     const MtStream *gen_end_ptr = gen_end.k < 312 ? &gen_end : nullptr;
     // the wavefront form runs only for maxDepth 1 and opaque scenes
     const Spec L =
-        path_li<true, TracedResults, true>(s, tr, ps.ray.o, ps.ray.d, true, ps.hit, ps.sc, rng, pr, ris, rv, i, gen_end_ptr, e);
+        path_li<true, TracedResults<kWeights>, true>(s, tr, ps.ray.o, ps.ray.d, true, ps.hit, ps.sc, rng, pr, ris, rv, i, gen_end_ptr, e);
     V3 rgb = spectrum_to_rgb(L, ps.sc.cie);
     if (cam.p.has_params && cam.p.enable_exposure) rgb = rgb * cam.p.exposure_mult;
     color[i] = make_float4(rgb.x, rgb.y, rgb.z, 1.0f);
 }
 
+template <bool kWeights>
 __global__ void __launch_bounds__(256, 2)
     ris_shade_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ CameraD cam, int frame_arg,
                      const __grid_constant__ PathRun pr, const __grid_constant__ RisRun ris,
@@ -211,7 +218,7 @@ __global__ void __launch_bounds__(256, 2)
     if (!tile_pixel(cam.width, cam.height, x, y)) return;
     if (wb.done[(size_t)y * (size_t)cam.width + (size_t)x] & kPixelMiss) return;
     unsigned e = 0;
-    shade_general(s, cam, live_frame(cam, frame_arg), pr, ris, gb, rv, wb, color, trace_level, x, y, e);
+    shade_general<kWeights>(s, cam, live_frame(cam, frame_arg), pr, ris, gb, rv, wb, color, trace_level, x, y, e);
     if (e) atomicOr(err, e);
 }
 
@@ -253,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     uint32_t k0;
     MtStream upd = load_stream_from(wb.rng_state, i, wb.pixels, pixel_seed(i, frame_index), ps.s156, k0);
     upd.spill = spill;
-    const TracedResults tr = traced_results(s, ris, wb, kTraceNoBsdfRays, i);
+    const auto tr = traced_results<true>(s, ris, wb, kTraceNoBsdfRays, i);
     const int N = ris.candidate_count;
     const int n_nee = smaxi(1, N / 2), n_bsdf = smaxi(0, N - n_nee), conn = (done & kPixelConn) ? 1 : 0;
     const int n_total = n_nee + conn + smaxi(0, n_bsdf - conn);
@@ -416,7 +423,7 @@ int launch_ris_shade(const DeviceScene &s, const CameraD &cam, int frame_index, 
     const RisRun ris = ris_run(p);
     // The resampling kernel continues a stream it has not replayed, whose state travels only
     // below draw 312.
-    const bool lean = trace_level == kTraceNoBsdfRays && draws_to_generation_end(p) < 312;
+    const bool lean = wb.nee_weight && trace_level == kTraceNoBsdfRays && draws_to_generation_end(p) < 312;
     if (lean) {
         const bool wide = tune.shade_shape < 2;  // 256 threads per block, else 128
         const int blocks = wide ? tile_blocks<256>(cam.width, cam.height) : tile_blocks<128>(cam.width, cam.height);
@@ -426,8 +433,9 @@ int launch_ris_shade(const DeviceScene &s, const CameraD &cam, int frame_index, 
                                          : ris_resample_kernel<128, 8>;
         k<<<blocks, wide ? 256 : 128, 0, st>>>(s, cam, frame_index, pr, ris, gb, rv, wb, color, err);
     } else {
-        ris_shade_kernel<<<tile_blocks(cam.width, cam.height), 256, 0, st>>>(s, cam, frame_index, pr, ris, gb, rv, wb,
-                                                                             color, trace_level, err);
+        auto k = wb.nee_weight ? ris_shade_kernel<true> : ris_shade_kernel<false>;
+        k<<<tile_blocks(cam.width, cam.height), 256, 0, st>>>(s, cam, frame_index, pr, ris, gb, rv, wb, color,
+                                                              trace_level, err);
     }
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
