@@ -1313,6 +1313,7 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         const int n_nee = std::max(1, p->candidate_count / 2);
         const int n_bsdf = std::max(0, p->candidate_count - n_nee);
         wb.pixels = count;
+        c->have_wave = false;  // the last frame's queues, until this one has run: they may be replaced here
         wb.n_closest = closest_slots(trace_level, n_bsdf);
         wb.n_shadow = n_nee;
         void *q;
