@@ -197,6 +197,13 @@ struct hdr_ctx {
     int32_t rec_frame = 0, graph_frame = 0;
     uint64_t graph_kernels = 0;   // kernel launches one replay of graph_exec makes
     cudaGraphExec_t graph_exec = nullptr;
+    // the memory the recorded kernels read and write: the buffers the recorded passes asked for, and
+    // the scene. hdr_graph_launch refuses once a buffer has been replaced or the scene is gone
+    // (frees counts the frame buffers given back, graph_frees at the last look)
+    std::map<std::string, DevBuf> rec_buffers, graph_buffers;
+    std::weak_ptr<SceneStore> rec_scene, graph_scene;
+    bool rec_has_scene = false, graph_has_scene = false;
+    uint64_t frees = 0, graph_frees = 0;
     int32_t graph_instantiations = 0, graph_updates = 0;
     // hdr_autotune_frame: the wavefront RIS frame in progress searches the trace schedules and
     // resampling launch shapes, reporting into tune_out
@@ -258,19 +265,26 @@ cudaMemPool_t frame_pool(int device) {
 
 void frame_free(hdr_ctx *c, DevBuf &b) {
     if (b.ptr) cudaFreeAsync(b.ptr, c->stream);
+    c->frees += 1;
     c->allocated -= b.bytes;
     b = DevBuf{};
 }
 
 // The light candidates' weights only make a frame faster (ris_path_trace_pass renders without
 // them too), so they give way to a buffer that something cannot do without. True when any were held.
-constexpr const char *kWeightBuffer = "__wave_nee_weight";
+// Those of frames with a reservoir and without are two buffers, so that a frame of the one kind
+// does not replace what a recording of the other uses.
+constexpr const char *kWeightBuffers[] = {"__wave_nee_weight", "__wave_nee_weight_plain"};
 bool give_back(hdr_ctx *c) {
-    auto it = c->buffers.find(kWeightBuffer);
-    if (it == c->buffers.end()) return false;
-    frame_free(c, it->second);
-    c->buffers.erase(it);
-    return true;
+    bool any = false;
+    for (const char *name : kWeightBuffers) {
+        auto it = c->buffers.find(name);
+        if (it == c->buffers.end()) continue;
+        frame_free(c, it->second);
+        c->buffers.erase(it);
+        any = true;
+    }
+    return any;
 }
 bool budget_room(hdr_ctx *c, size_t bytes) {
     auto fits = [&] { return !c->budget || c->allocated + bytes <= c->budget; };
@@ -300,11 +314,17 @@ hdr_status frame_alloc(hdr_ctx *c, DevBuf &b, size_t bytes) {
     return HDR_OK;
 }
 
+// A recorded pass uses this buffer.
+void note_recorded(hdr_ctx *c, const char *name, const DevBuf &b) {
+    if (c->recording) c->rec_buffers[name] = b;
+}
+
 // FrameBuffersMap::Add / AddOrGetPersistent: create (zeroed) or resize keeping
 // the prefix; a same-size request returns the existing buffer untouched.
 hdr_status ensure_buffer(hdr_ctx *c, const char *name, size_t bytes, void **out) {
     auto it = c->buffers.find(name);
     if (it != c->buffers.end() && it->second.bytes == bytes) {
+        note_recorded(c, name, it->second);
         *out = it->second.ptr;
         return HDR_OK;
     }
@@ -333,6 +353,7 @@ hdr_status ensure_buffer(hdr_ctx *c, const char *name, size_t bytes, void **out)
 hdr_status ensure_scratch(hdr_ctx *c, const char *name, size_t bytes, void **out) {
     auto it = c->buffers.find(name);
     if (it != c->buffers.end() && it->second.bytes >= bytes) {
+        note_recorded(c, name, it->second);
         *out = it->second.ptr;
         return HDR_OK;
     }
@@ -388,6 +409,7 @@ hdr_status ensure_batch_scratch(SceneStore *store, const char *name, size_t byte
 void *find_buffer(hdr_ctx *c, const char *name, size_t *bytes) {
     auto it = c->buffers.find(name);
     if (it == c->buffers.end()) return nullptr;
+    note_recorded(c, name, it->second);
     if (bytes) *bytes = it->second.bytes;
     return it->second.ptr;
 }
@@ -417,6 +439,10 @@ hdr_status check_not_recording(const hdr_ctx *c, const char *what) {
 // the first recorded pass fixes that index, the others must give the same one.
 hdr_status record_frame_index(hdr_ctx *c, int32_t frame_index, hdr::CameraD *cam) {
     if (!c->recording) return HDR_OK;
+    if (cam) {  // a pass over the scene
+        c->rec_scene = c->scene_store;
+        c->rec_has_scene = true;
+    }
     if (c->rec_has_frame && c->rec_frame != frame_index)
         return fail(HDR_EINVAL, "recorded passes render one frame index (%d), not %d", c->rec_frame, frame_index);
     c->rec_has_frame = true;
@@ -1350,7 +1376,7 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         // Last, since a frame for which only the weights have no room (a budget, a recording that
         // cannot allocate) renders without them: the same image, its light candidates evaluated
         // a second time after the trace.
-        st = ensure_scratch(c, kWeightBuffer, count * wb.n_shadow * nee_weight_size(p), &q);
+        st = ensure_scratch(c, kWeightBuffers[p->use_reservoir ? 0 : 1], count * wb.n_shadow * nee_weight_size(p), &q);
         if (st != HDR_OK && st != HDR_ENOMEM && !c->recording) return st;
         wb.nee_weight = st == HDR_OK ? q : nullptr;
         if ((st = begin_pass(c, 1)) != HDR_OK) return st;
@@ -2017,6 +2043,7 @@ hdr_status hdr_zero_persistent(hdr_ctx *c) {
     HDR_CUDA(cudaSetDevice(c->device));
     for (const char *name : {"__accum_color", "__ris_reservoir", "__ris_reservoir_prev", "__prev_pos_depth"}) {
         auto it = c->buffers.find(name);
+        if (it != c->buffers.end()) note_recorded(c, name, it->second);
         if (it != c->buffers.end() && it->second.bytes)
             HDR_CUDA(cudaMemsetAsync(it->second.ptr, 0, it->second.bytes, c->stream));
     }
@@ -2491,6 +2518,9 @@ hdr_status hdr_graph_begin(hdr_ctx *c) {
     c->recording = true;
     c->rec_failed = false;
     c->rec_has_frame = false;
+    c->rec_buffers.clear();
+    c->rec_scene.reset();
+    c->rec_has_scene = false;
     c->rec_launches0 = c->launches;
     return HDR_OK;
 }
@@ -2537,6 +2567,25 @@ hdr_status hdr_graph_end(hdr_ctx *c) {
     c->graph_kernels = kernels;
     c->graph_has_frame = c->rec_has_frame;
     c->graph_frame = c->rec_frame;
+    c->graph_buffers.swap(c->rec_buffers);
+    c->graph_scene = c->rec_scene;
+    c->graph_has_scene = c->rec_has_scene;
+    c->graph_frees = c->frees;
+    return HDR_OK;
+}
+
+// Is the memory that the recorded kernels use still theirs?
+static hdr_status check_graph_memory(hdr_ctx *c) {
+    if (c->graph_has_scene && c->graph_scene.expired())
+        return fail(HDR_EINVAL, "the recorded graph renders a scene that has been replaced: record it again");
+    if (c->graph_frees == c->frees) return HDR_OK;
+    for (const auto &kv : c->graph_buffers) {
+        const auto it = c->buffers.find(kv.first);
+        if (it == c->buffers.end() || it->second.ptr != kv.second.ptr || it->second.bytes < kv.second.bytes)
+            return fail(HDR_EINVAL, "the recorded graph uses buffer '%s', which has been replaced: record it again",
+                        kv.first.c_str());
+    }
+    c->graph_frees = c->frees;
     return HDR_OK;
 }
 
@@ -2547,6 +2596,7 @@ hdr_status hdr_graph_launch(hdr_ctx *c, int32_t frame_index) {
     if (!c->graph_exec) return fail(HDR_EINVAL, "no recorded graph (hdr_graph_begin / hdr_graph_end)");
     hdr_status st;
     if ((st = check_cancel(c)) != HDR_OK) return st;
+    if ((st = check_graph_memory(c)) != HDR_OK) return st;
     HDR_CUDA(cudaSetDevice(c->device));
     if (c->graph_has_frame) {  // the frame the recorded passes render, read by their kernels
         set_frame_slot_kernel<<<1, 1, 0, c->stream>>>(c->d_frame_slot, frame_index >= 0 ? frame_index

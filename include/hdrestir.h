@@ -699,6 +699,9 @@ hdr_status hdr_trim_frame_memory(int32_t device, size_t keep_bytes);
  * hdr_autotune_trace, hdr_rng_floats, hdr_graph_launch) fail with HDR_EINVAL and
  * leave the recording intact. A recorded pass that fails marks the recording,
  * and hdr_graph_end then discards it (HDR_EINVAL) and keeps the previous graph.
+ * hdr_graph_launch fails with HDR_EINVAL once a buffer that the recorded passes use
+ * has been replaced (a call with another frame size or candidate count,
+ * hdr_clear_persistent) or the scene they render has been freed.
  * hdr_ctx_destroy drops an unfinished recording. */
 hdr_status hdr_graph_begin(hdr_ctx *ctx);
 hdr_status hdr_graph_end(hdr_ctx *ctx);

@@ -62,7 +62,7 @@ def test_frames_without_room_for_the_weights(scene, form):
             except abi.HdrError:
                 return None, None
             try:
-                return out, ctx.buffer_size("__wave_nee_weight")
+                return out, ctx.buffer_size("__wave_nee_weight" + "_plain" * (not ris["use_reservoir"]))
             except abi.HdrError:
                 return out, 0
 
