@@ -794,6 +794,8 @@ int closest_mode(uint32_t flags, bool sh4, bool links) {
 
 // Bytes per light candidate of WaveBuffers::nee_weight.
 size_t nee_weight_size(const hdr_ris_params *p) { return p->use_reservoir ? sizeof(float) : sizeof(double); }
+// Ray slots of a wavefront frame or batch, numbered in the queues and counted on the device as ints.
+bool slots_fit(size_t slots) { return slots < ((size_t)1 << 31); }
 // Which closest-hit rays the wavefront RIS pass casts (hdr::kTrace*).
 int ris_trace_level(const hdr_ctx *c, const hdr_ris_params *p) {
     if ((p->flags & HDR_RIS_TRACE_ALL_RAYS) || c->scene.bsdf_lights)
@@ -1252,9 +1254,19 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
     // wavefront form: direct light only (no later bounces), no stochastic opacity, no physical
     // sky (its sun technique is served by the one-kernel form only) and no blackbody lights
     // (an extension the wavefront kernels are built without, to keep their registers)
-    const bool wave = p->path.max_depth == 1 && c->scene_opaque && !c->scene.sky && !c->scene.blackbody &&
-                      !(p->flags & HDR_RIS_ONE_KERNEL);
+    bool wave = p->path.max_depth == 1 && c->scene_opaque && !c->scene.sky && !c->scene.blackbody &&
+                !(p->flags & HDR_RIS_ONE_KERNEL);
     const bool spatial = p->spatial_neighbors > 0 && p->use_reservoir;
+    const size_t count = (size_t)cam->width * cam->height;
+    const int n_nee = std::max(1, p->candidate_count / 2), n_bsdf = std::max(0, p->candidate_count - n_nee);
+    const int trace_level = ris_trace_level(c, p);
+    // more ray slots than their numbers hold: the one-kernel form, which has none and gives the same image
+    if (wave && !(slots_fit(count * closest_slots(trace_level, n_bsdf)) && slots_fit(count * n_nee))) {
+        if (spatial || tune || (c->flags & HDR_CTX_RECORD_LIGHTS))
+            return fail(HDR_EINVAL, "%zu pixels with %d candidates need 2^31 ray slots or more, which spatial reuse, "
+                        "autotuning and recorded lights do not work with", count, p->candidate_count);
+        wave = false;
+    }
     if (spatial && !wave)
         return fail(HDR_EINVAL, "spatial reuse runs in the wavefront form only (max_depth 1, opaque scene)");
     if (tune && !wave)
@@ -1262,7 +1274,6 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
                     "no HDR_RIS_ONE_KERNEL)");
     if ((st = check_cancel(c)) != HDR_OK) return st;
     HDR_CUDA(cudaSetDevice(c->device));
-    const size_t count = (size_t)cam->width * cam->height;
     hdr::GBufferView gb;
     if ((st = gbuffer_view(c, count, false, gb)) != HDR_OK) return st;
     void *color = nullptr, *res = nullptr;
@@ -1335,9 +1346,6 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
     }
     if (wave) {
         hdr::WaveBuffers wb{};
-        const int trace_level = ris_trace_level(c, p);
-        const int n_nee = std::max(1, p->candidate_count / 2);
-        const int n_bsdf = std::max(0, p->candidate_count - n_nee);
         wb.pixels = count;
         c->have_wave = false;  // the last frame's queues, until this one has run: they may be replaced here
         wb.n_closest = closest_slots(trace_level, n_bsdf);
@@ -1744,7 +1752,7 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
         total_s += (long long)jobs[(size_t)i].count * jobs[(size_t)i].n_shadow;
         total_w += jobs[(size_t)i].weight_bytes;
     }
-    if (total_c >= (1ll << 31) || total_s >= (1ll << 31))
+    if (!slots_fit((size_t)total_c) || !slots_fit((size_t)total_s))
         return fail(HDR_EINVAL, "batch of %lld closest / %lld shadow ray slots exceeds 2^31", total_c, total_s);
     // the shared queues and result slots belong to the resident scene, whichever ctx leads
     SceneStore *store = lead->scene_store.get();
