@@ -241,10 +241,12 @@ class Context:
         return {"node_quorum": t.node_quorum, "blocks_per_sm": t.blocks_per_sm, "shade_shape": t.shade_shape,
                 "shadow_shape": t.shadow_shape}
 
-    def set_trace_tuning(self, node_quorum: int, blocks_per_sm: int, shade_shape: int = 0,
+    def set_trace_tuning(self, node_quorum: int, blocks_per_sm: int, shade_shape: int | None = None,
                          shadow_shape: int | None = None) -> None:
-        if shadow_shape is None:
-            shadow_shape = self.trace_tuning()["shadow_shape"]
+        """Trace schedule and launch shapes; a shape that is None stays as it is."""
+        now = self.trace_tuning()
+        shade_shape = now["shade_shape"] if shade_shape is None else shade_shape
+        shadow_shape = now["shadow_shape"] if shadow_shape is None else shadow_shape
         t = abi.TraceTuning(int(node_quorum), int(blocks_per_sm), 0.0, int(shade_shape), int(shadow_shape), 0.0)
         abi.check(self._lib.hdr_set_trace_tuning(self._h, C.byref(t)))
 

@@ -192,6 +192,18 @@ int launch_tlas_rebuild(const float *xf, float4 *instances, const float *mesh_ra
 // connection candidate (the path's bounce ray): their weights are the same
 // whatever the rays hit, so those rays are not cast.
 constexpr int kTraceNoBsdfRays = 0, kTraceBounceRay = 1, kTraceAllBsdfRays = 2;
+// Most draws of a pixel up to the end of generation: pixel and lens 4, wavelengths 1, 3 per
+// light candidate, 5 per bounce.
+inline int draws_to_generation_end(const RisParamsD &p) {
+    const int n_nee = p.candidate_count / 2 > 1 ? p.candidate_count / 2 : 1;
+    const int n_bsdf = p.candidate_count > n_nee ? p.candidate_count - n_nee : 0;
+    return 5 + 3 * n_nee + 5 * (n_bsdf + 1);
+}
+// Does ris_resample_kernel serve the frame (else ris_shade_kernel, which has one shape)? It
+// continues a stream it has not replayed, whose state travels only below draw 312.
+inline bool lean_resampling(const RisParamsD &p, const WaveBuffers &wb, int trace_level) {
+    return wb.nee_weight && trace_level == kTraceNoBsdfRays && draws_to_generation_end(p) < 312;
+}
 // The three stages of the wavefront RIS pass on their own (a batch of images
 // runs every image's generate, one trace over their shared queues, then every
 // image's shade). Return the launches, -1 on a launch error.

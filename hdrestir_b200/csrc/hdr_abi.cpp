@@ -1189,7 +1189,8 @@ hdr_status tune_wave_frame(hdr_ctx *c, const hdr::CameraD &cd, int frame_index, 
     hdr::TraceTuning t = c->tune;
     int shade_pick = t.shade_shape;
     float shade_ms = 3.4e38f;
-    for (int shape = 0; shape < hdr::kShadeShapes; ++shape) {
+    const bool lean = hdr::lean_resampling(d, wb, trace_level);  // else the kernel has one shape: timed, not chosen
+    for (int shape = lean ? 0 : shade_pick; shape < (lean ? hdr::kShadeShapes : shade_pick + 1); ++shape) {
         t.shade_shape = shape;
         float ms = 0.0f;
         st = time_best_of_two(

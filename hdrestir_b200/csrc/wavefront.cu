@@ -399,12 +399,6 @@ RisRun ris_run(const RisParamsD &p) {
     ris.reproj = p.reproj;
     return ris;
 }
-// Most draws of a pixel up to the end of generation: pixel and lens 4, wavelengths 1, 3 per
-// light candidate, 5 per bounce.
-int draws_to_generation_end(const RisParamsD &p) {
-    const int n_nee = smaxi(1, p.candidate_count / 2), n_bsdf = smaxi(0, p.candidate_count - n_nee);
-    return 5 + 3 * n_nee + 5 * (n_bsdf + 1);
-}
 }  // namespace
 
 int launch_ris_generate(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
@@ -421,10 +415,7 @@ int launch_ris_shade(const DeviceScene &s, const CameraD &cam, int frame_index, 
                      cudaStream_t st, const TraceTuning &tune) {
     const PathRun pr = path_run(p);
     const RisRun ris = ris_run(p);
-    // The resampling kernel continues a stream it has not replayed, whose state travels only
-    // below draw 312.
-    const bool lean = wb.nee_weight && trace_level == kTraceNoBsdfRays && draws_to_generation_end(p) < 312;
-    if (lean) {
+    if (lean_resampling(p, wb, trace_level)) {
         const bool wide = tune.shade_shape < 2;  // 256 threads per block, else 128
         const int blocks = wide ? tile_blocks<256>(cam.width, cam.height) : tile_blocks<128>(cam.width, cam.height);
         auto k = tune.shade_shape == 0   ? ris_resample_kernel<256, 2>
