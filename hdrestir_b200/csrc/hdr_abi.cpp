@@ -1230,6 +1230,15 @@ hdr_status tune_wave_frame(hdr_ctx *c, const hdr::CameraD &cd, int frame_index, 
 
 }  // namespace
 
+namespace hdr {
+// Bytes a pixel of a wavefront RIS frame over c's scene takes in ray queues, result slots and weights.
+size_t ris_queue_bytes(hdr_ctx *c, const hdr_ris_params *p) {
+    const int n_nee = std::max(1, p->candidate_count / 2), n_bsdf = std::max(0, p->candidate_count - n_nee);
+    std::lock_guard<std::mutex> lock(c->mu);
+    return (size_t)closest_slots(ris_trace_level(c, p), n_bsdf) * 52 + (size_t)n_nee * (33 + nee_weight_size(p));
+}
+}  // namespace hdr
+
 extern "C" {
 
 static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t frame_index,

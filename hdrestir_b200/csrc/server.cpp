@@ -32,6 +32,7 @@
 
 namespace hdr {
 hdr_status set_last_error(hdr_status st, const char *fmt, ...);
+size_t ris_queue_bytes(hdr_ctx *c, const hdr_ris_params *p);
 }
 
 namespace {
@@ -51,16 +52,16 @@ size_t pixels_of(const hdr_job_desc &d) { return (size_t)d.camera.width * (size_
 // Device bytes a job's context allocates, per pixel: GBuffer 96, Color 16,
 // accumulator 16, firefly scratch 16; RIS adds the reservoir (80), the
 // stream state and done flag (49) and its share of the batch's ray queues and
-// result slots (52 per closest-hit slot, 33 per shadow slot). The light candidates' weights
-// (4 or 8 each) stay within the closest-hit slots a default frame is charged for and does not allocate.
+// result slots (52 per closest-hit slot, 33 per shadow slot), which holds the light candidates'
+// weights (4 or 8 each) too where the scene's frames have no closest-hit slots.
+size_t ris_queue_charge(const hdr_ris_params &p) {
+    const int n_nee = std::max(1, p.candidate_count / 2);
+    return (size_t)(1 + std::max(0, p.candidate_count - n_nee)) * 52 + (size_t)n_nee * 33;
+}
 size_t job_bytes(const hdr_job_desc &d) {
     const size_t px = pixels_of(d);
     size_t per = 96 + 16 + 16 + (d.firefly ? 16 : 0);
-    if (d.pipeline == HDR_JOB_RIS) {
-        const int n_nee = std::max(1, d.ris.candidate_count / 2);
-        const int n_closest = 1 + std::max(0, d.ris.candidate_count - n_nee);
-        per += (d.ris.use_reservoir ? 80 : 0) + 49 + (size_t)n_closest * 52 + (size_t)n_nee * 33;
-    }
+    if (d.pipeline == HDR_JOB_RIS) per += (d.ris.use_reservoir ? 80 : 0) + 49 + ris_queue_charge(d.ris);
     return px * per + (1u << 20);
 }
 
@@ -240,6 +241,12 @@ hdr_status hdr_server_submit(hdr_server *sv, const hdr_job_desc *job, int64_t *j
     if (sv->budget && j->bytes > sv->budget)
         return hdr::set_last_error(HDR_ENOMEM, "job needs about %zu bytes, above the %zu-byte budget", j->bytes,
                                    sv->budget);
+    // where they have, the weights come on top (a job that fits without them is not refused for them)
+    if (job->pipeline == HDR_JOB_RIS) {
+        const size_t queues = hdr::ris_queue_bytes(sv->scenes[(size_t)job->scene], &job->ris);
+        const size_t charged = ris_queue_charge(job->ris);
+        j->bytes += pixels_of(*job) * (queues > charged ? queues - charged : 0);
+    }
     *job_id = j->id;
     sv->queued.push_back(std::move(j));
     return HDR_OK;
