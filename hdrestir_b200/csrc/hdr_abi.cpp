@@ -1544,15 +1544,41 @@ hdr_status hdr_scene_set_instance_transforms(hdr_ctx *c, const float *transforms
         xf = store->xf_staging;
     }
     hdr::DeviceScene &s = c->scene;
-    const int launched = hdr::launch_tlas_rebuild(
-        xf, const_cast<float4 *>(s.instances), store->mesh_ranges, store->inst_bounds, num_instances,
-        const_cast<float4 *>(s.tlas_nodes), store->tlas_capacity, const_cast<int *>(s.tlas_inst), store->tlas_stack,
-        num_instances + 2, store->tlas_info, c->stream);
-    if (launched < 0) {
+    auto failed_launch = [c] {
         c->has_scene = false;
         return fail(HDR_ECUDA, "TLAS rebuild launch: %s", cudaGetErrorString(cudaGetLastError()));
-    }
+    };
+    int launched = hdr::launch_instance_update(xf, const_cast<float4 *>(s.instances), store->mesh_ranges,
+                                               store->inst_bounds, num_instances, c->stream);
+    if (launched < 0) return failed_launch();
     c->launches += (uint64_t)launched;
+    std::vector<float> b9, records;
+    if (store->sh4) {
+        b9.resize((size_t)num_instances * 9);
+        records.resize((size_t)num_instances * 32);
+        HDR_CUDA(cudaMemcpyAsync(b9.data(), store->inst_bounds, b9.size() * sizeof(float), cudaMemcpyDeviceToHost,
+                                 c->stream));
+        HDR_CUDA(cudaMemcpyAsync(records.data(), s.instances, records.size() * sizeof(float), cudaMemcpyDeviceToHost,
+                                 c->stream));
+        HDR_CUDA(cudaStreamSynchronize(c->stream));
+    }
+    launched = hdr::launch_tlas_build(store->inst_bounds, num_instances, const_cast<float4 *>(s.tlas_nodes),
+                                      store->tlas_capacity, const_cast<int *>(s.tlas_inst), store->tlas_stack,
+                                      num_instances + 2, store->tlas_info, c->stream);
+    if (launched < 0) return failed_launch();
+    c->launches += (uint64_t)launched;
+    // The SAH trees' top level over the moved instances' world boxes, on the host while the device
+    // builds its TLAS, with as many opened nodes as there are instances: 3.98 ms a call for 2001
+    // instances, 0.45 for 201. After the TLAS and with 1024 opened nodes, as an upload has them, it
+    // took 6.24 and 1.34; closest hits then take 0 and 2 % longer than after an upload (21
+    // instances: 5 %).
+    bool sh4_built = false;
+    if (store->sh4) {
+        std::vector<float> b6((size_t)num_instances * 6);
+        for (int i = 0; i < num_instances; ++i)
+            for (int k = 0; k < 6; ++k) b6[6 * (size_t)i + k] = b9[9 * (size_t)i + k];
+        sh4_built = hdr::rebuild_shadow_tlas(b6.data(), records.data(), num_instances, store->sh4_host);
+    }
     int info[4] = {};
     HDR_CUDA(cudaMemcpyAsync(info, store->tlas_info, sizeof(info), cudaMemcpyDeviceToHost, c->stream));
     HDR_CUDA(cudaStreamSynchronize(c->stream));
@@ -1564,23 +1590,15 @@ hdr_status hdr_scene_set_instance_transforms(hdr_ctx *c, const float *transforms
     }
     s.proper_boxes = (store->blas_proper && !info[3]) ? 1 : 0;
     s.shallow = (store->max_blas_depth + info[1] + 4 <= hdr::kShallowStack) ? 1 : 0;
-    if (store->sh4) {  // the shadow BVH's TLAS over the moved instances' world boxes
-        std::vector<float> b9((size_t)num_instances * 9), b6((size_t)num_instances * 6),
-            records((size_t)num_instances * 32);
-        HDR_CUDA(cudaMemcpyAsync(b9.data(), store->inst_bounds, b9.size() * sizeof(float), cudaMemcpyDeviceToHost,
-                                 c->stream));
-        HDR_CUDA(cudaMemcpyAsync(records.data(), s.instances, records.size() * sizeof(float), cudaMemcpyDeviceToHost,
-                                 c->stream));
+    if (store->sh4) {
         // closest-hit tie-breaks follow the rebuilt reference TLAS's instance order
         std::vector<int> tlas_inst((size_t)num_instances), rank;
         HDR_CUDA(cudaMemcpyAsync(tlas_inst.data(), s.tlas_inst, tlas_inst.size() * sizeof(int),
                                  cudaMemcpyDeviceToHost, c->stream));
         HDR_CUDA(cudaStreamSynchronize(c->stream));
-        for (int i = 0; i < num_instances; ++i)
-            for (int k = 0; k < 6; ++k) b6[6 * (size_t)i + k] = b9[9 * (size_t)i + k];
         hdr::shadow_ranks(tlas_inst, num_instances, rank);
-        hdr::ShadowBvh &sb = store->sh4_host;
-        if (hdr::rebuild_shadow_tlas(b6.data(), records.data(), sb)) {
+        const hdr::ShadowBvh &sb = store->sh4_host;
+        if (sh4_built) {
             HDR_CUDA(cudaMemcpyAsync(const_cast<float4 *>(s.sh4_nodes), sb.nodes.data(),
                                      (size_t)sb.tlas_capacity * hdr::kSh4NodeFloats * sizeof(float),
                                      cudaMemcpyHostToDevice, c->stream));

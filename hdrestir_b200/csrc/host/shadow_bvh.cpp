@@ -420,7 +420,7 @@ struct TopLeafCode {
 
 }  // namespace
 
-bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, ShadowBvh &b) {
+bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, int opened_refs, ShadowBvh &b) {
     const size_t n_inst = b.inst_root.size();
     std::fill(b.mesh_world.begin(), b.mesh_world.end(), -1);
     std::vector<TopRef> refs;
@@ -453,7 +453,7 @@ bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, Sh
         }
     }
     std::make_heap(heap.begin(), heap.end(), smaller);
-    const size_t limit = refs.size() + (size_t)kSh4OpenedRefs;
+    const size_t limit = refs.size() + (size_t)std::min(opened_refs, kSh4OpenedRefs);
     while (!heap.empty() && refs.size() + 3 <= limit) {
         std::pop_heap(heap.begin(), heap.end(), smaller);
         const int at = heap.back();
@@ -580,7 +580,7 @@ bool build_shadow_bvh(const hdr_scene_desc &desc, const FlatScene &flat, ShadowB
     }
     shadow_ranks(flat.tlas_inst, n_inst, out.inst_rank);
     // not an error when it does not fit: the reference trees serve these queries too
-    out.ok = rebuild_shadow_tlas(flat.inst_bounds.data(), flat.instances.data(), out);
+    out.ok = rebuild_shadow_tlas(flat.inst_bounds.data(), flat.instances.data(), kSh4OpenedRefs, out);
     return true;
 }
 

@@ -74,10 +74,11 @@ bool build_shadow_bvh(const hdr_scene_desc &desc, const FlatScene &flat, ShadowB
 void shadow_ranks(const std::vector<int> &tlas_inst, int num_instances, std::vector<int> &rank);
 
 // Rebuilds the top-level tree over instances that moved: `inst_bounds` (6 floats each, the
-// world boxes) and `inst_records` (32 floats each, the inverse transform first). Reads the
+// world boxes) and `inst_records` (32 floats each, the inverse transform first), with at most
+// opened_refs leaves from opened instances (no more than kSh4OpenedRefs). Reads the
 // BLAS nodes, inst_root and inst_mesh of `b`, and writes its mesh_world, the first nodes of
 // b.nodes and b.tlas_depth; returns false when the tree does not fit the reserved room or the
 // stack bound.
-bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, ShadowBvh &b);
+bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, int opened_refs, ShadowBvh &b);
 
 }  // namespace hdr

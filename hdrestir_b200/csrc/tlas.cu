@@ -152,17 +152,20 @@ __global__ void __launch_bounds__(256) tlas_build_kernel(const float *__restrict
 
 }  // namespace
 
-int launch_tlas_rebuild(const float *xf, float4 *instances, const float *mesh_ranges, float *bounds, int n,
-                        float4 *tlas_nodes, int cap_nodes, int *tlas_inst, int4 *stack, int cap_stack, int *info,
-                        cudaStream_t st) {
-    if (n <= 0) return 0;
+int launch_instance_update(const float *xf, float4 *instances, const float *mesh_ranges, float *bounds, int n,
+                           cudaStream_t st) {
     instance_update_kernel<<<(n + 127) / 128, 128, 0, st>>>(xf, instances, mesh_ranges, bounds, n);
+    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
+}
+
+int launch_tlas_build(const float *bounds, int n, float4 *tlas_nodes, int cap_nodes, int *tlas_inst, int4 *stack,
+                      int cap_stack, int *info, cudaStream_t st) {
     const size_t smem = (size_t)n * kInstSmemBytes;
     const int staged = smem <= (size_t)kTlasSmemBytes ? 1 : 0;
     if (staged) cudaFuncSetAttribute(tlas_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     tlas_build_kernel<<<1, 256, staged ? smem : 0, st>>>(bounds, n, tlas_nodes, cap_nodes, tlas_inst, stack,
                                                          cap_stack, info, staged);
-    return cudaPeekAtLastError() == cudaSuccess ? 2 : -1;
+    return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
 }
 
 }  // namespace hdr
