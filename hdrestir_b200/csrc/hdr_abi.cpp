@@ -1568,19 +1568,30 @@ hdr_status hdr_scene_set_instance_transforms(hdr_ctx *c, const float *transforms
     if (launched < 0) return failed_launch();
     c->launches += (uint64_t)launched;
     // The SAH trees' top level over the moved instances' world boxes, on the host while the device
-    // builds its TLAS, with as many opened nodes as there are instances: 3.98 ms a call for 2001
-    // instances, 0.45 for 201. After the TLAS and with 1024 opened nodes, as an upload has them, it
-    // took 6.24 and 1.34; closest hits then take 0 and 2 % longer than after an upload (21
-    // instances: 5 %).
+    // builds its TLAS: 3.92 ms a call for 2001 instances, 0.53 for 201 (6.2 and 1.34 one after
+    // the other, with a wait for every copy).
     bool sh4_built = false;
     if (store->sh4) {
         std::vector<float> b6((size_t)num_instances * 6);
         for (int i = 0; i < num_instances; ++i)
             for (int k = 0; k < 6; ++k) b6[6 * (size_t)i + k] = b9[9 * (size_t)i + k];
-        sh4_built = hdr::rebuild_shadow_tlas(b6.data(), records.data(), num_instances, store->sh4_host);
+        sh4_built = hdr::rebuild_shadow_tlas(b6.data(), records.data(), store->sh4_host);
     }
+    // host copies of what the device built, and what goes back: alive to the end of the call
     int info[4] = {};
+    std::vector<int> tlas_inst, rank, inst_leaf;
+    std::vector<float> nodes;
     HDR_CUDA(cudaMemcpyAsync(info, store->tlas_info, sizeof(info), cudaMemcpyDeviceToHost, c->stream));
+    if (store->sh4) {
+        tlas_inst.resize((size_t)num_instances);
+        HDR_CUDA(cudaMemcpyAsync(tlas_inst.data(), s.tlas_inst, tlas_inst.size() * sizeof(int),
+                                 cudaMemcpyDeviceToHost, c->stream));
+        if (store->ref_links) {
+            nodes.resize(8 * (size_t)store->tlas_capacity);
+            HDR_CUDA(cudaMemcpyAsync(nodes.data(), s.tlas_nodes, nodes.size() * sizeof(float), cudaMemcpyDeviceToHost,
+                                     c->stream));
+        }
+    }
     HDR_CUDA(cudaStreamSynchronize(c->stream));
     store->wide_stale = true;
     if (info[2] || store->max_blas_depth + info[1] + 4 > hdr::kTraceStack) {
@@ -1592,21 +1603,16 @@ hdr_status hdr_scene_set_instance_transforms(hdr_ctx *c, const float *transforms
     s.shallow = (store->max_blas_depth + info[1] + 4 <= hdr::kShallowStack) ? 1 : 0;
     if (store->sh4) {
         // closest-hit tie-breaks follow the rebuilt reference TLAS's instance order
-        std::vector<int> tlas_inst((size_t)num_instances), rank;
-        HDR_CUDA(cudaMemcpyAsync(tlas_inst.data(), s.tlas_inst, tlas_inst.size() * sizeof(int),
-                                 cudaMemcpyDeviceToHost, c->stream));
-        HDR_CUDA(cudaStreamSynchronize(c->stream));
         hdr::shadow_ranks(tlas_inst, num_instances, rank);
         const hdr::ShadowBvh &sb = store->sh4_host;
         if (sh4_built) {
             HDR_CUDA(cudaMemcpyAsync(const_cast<float4 *>(s.sh4_nodes), sb.nodes.data(),
-                                     (size_t)sb.tlas_capacity * hdr::kSh4NodeFloats * sizeof(float),
+                                     (size_t)sb.tlas_nodes * hdr::kSh4NodeFloats * sizeof(float),
                                      cudaMemcpyHostToDevice, c->stream));
             HDR_CUDA(cudaMemcpyAsync(const_cast<int *>(s.sh4_mesh_world), sb.mesh_world.data(),
                                      sb.mesh_world.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
             HDR_CUDA(cudaMemcpyAsync(const_cast<int *>(s.sh4_inst_rank), rank.data(), rank.size() * sizeof(int),
                                      cudaMemcpyHostToDevice, c->stream));
-            HDR_CUDA(cudaStreamSynchronize(c->stream));  // host buffers
         } else {
             store->sh4 = false;  // too deep for the shadow walk's stack: the reference trees serve shadow rays
         }
@@ -1614,20 +1620,11 @@ hdr_status hdr_scene_set_instance_transforms(hdr_ctx *c, const float *transforms
     // the reference TLAS changed on the device: the instances' leaves are found again in it (the
     // triangles' still hold); if that fails, closest hits go back to the reference walk
     if (store->ref_links && store->sh4) {
-        std::vector<float> nodes(8 * (size_t)store->tlas_capacity);
-        std::vector<int> tlas_inst((size_t)num_instances), inst_leaf;
-        HDR_CUDA(cudaMemcpyAsync(nodes.data(), s.tlas_nodes, nodes.size() * sizeof(float), cudaMemcpyDeviceToHost,
-                                 c->stream));
-        HDR_CUDA(cudaMemcpyAsync(tlas_inst.data(), s.tlas_inst, tlas_inst.size() * sizeof(int),
-                                 cudaMemcpyDeviceToHost, c->stream));
-        HDR_CUDA(cudaStreamSynchronize(c->stream));
         store->ref_links = tlas_links(nodes.data(), (size_t)store->tlas_capacity, tlas_inst.data(), tlas_inst.size(),
                                       num_instances, inst_leaf);
-        if (store->ref_links) {
+        if (store->ref_links)
             HDR_CUDA(cudaMemcpyAsync(const_cast<int *>(s.ref_inst_leaf), inst_leaf.data(),
                                      inst_leaf.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-            HDR_CUDA(cudaStreamSynchronize(c->stream));  // host buffers
-        }
     } else {
         store->ref_links = false;
     }
@@ -1638,7 +1635,7 @@ hdr_status hdr_scene_set_instance_transforms(hdr_ctx *c, const float *transforms
     fill_desc_copies(s, store->desc_dev, copies, store->sh4);
     HDR_CUDA(cudaMemcpyAsync(const_cast<hdr::DeviceScene *>(store->desc_dev), copies, sizeof(copies),
                              cudaMemcpyHostToDevice, c->stream));
-    HDR_CUDA(cudaStreamSynchronize(c->stream));  // `copies` is a host stack buffer
+    HDR_CUDA(cudaStreamSynchronize(c->stream));  // the host buffers above
     return HDR_OK;
 }
 

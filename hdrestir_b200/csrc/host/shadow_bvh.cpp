@@ -55,18 +55,37 @@ inline void grow(float *lo, float *hi, const float *a, const float *b) {
     }
 }
 
+// x, y, z and an unused lane
+typedef float F4 __attribute__((vector_size(16)));
+typedef int I4 __attribute__((vector_size(16)));
+inline F4 load3(const float *v) { return F4{v[0], v[1], v[2], 0.0f}; }
+struct Box4 {
+    F4 lo{FLT_MAX, FLT_MAX, FLT_MAX, 0.0f}, hi{-FLT_MAX, -FLT_MAX, -FLT_MAX, 0.0f};
+    void grow(F4 a, F4 b) {
+        lo = a < lo ? a : lo;
+        hi = hi < b ? b : hi;
+    }
+    float half_area() const {
+        const F4 d = hi - lo;
+        return (d[0] < 0.0f || d[1] < 0.0f || d[2] < 0.0f) ? 0.0f : d[0] * d[1] + d[1] * d[2] + d[2] * d[0];
+    }
+};
+
 // Binned SAH (16 bins per axis over the centroid bounds), leaves of at most
 // max_leaf primitives. The primitives themselves are partitioned, so every node reads a
 // consecutive range; order[] is the resulting leaf order. Empty bins cost nothing (most
 // nodes hold a few primitives), and the two halves of a large node are built at the same
 // time: the tree does not depend on how many threads there are, only the place of a node in
-// the array does. 522,242 triangles on 8 cores: 460 ms with one thread and leaves of four
-// triangles before, 130 ms now.
+// the array does. A box is one register pair, and only bins that hold something are swept: a
+// top level of 3,024 leaves, built again whenever instances move, 3.3 -> 2.2 ms on one core, 1.7
+// on several. All trees of 523 thousand triangles on 8 cores: 0.43 s with one thread and leaves
+// of four triangles before, 0.24 s now.
 class SahBuilder {
   public:
     SahBuilder(const std::vector<PrimBox> &prims, int max_leaf, std::vector<BNode> &nodes)
         : refs_(prims.size()), nodes_(nodes), max_leaf_(max_leaf) {
-        for (size_t i = 0; i < prims.size(); ++i) refs_[i] = {prims[i], (int)i};
+        for (size_t i = 0; i < prims.size(); ++i)
+            refs_[i] = {load3(prims[i].lo), load3(prims[i].hi), load3(prims[i].c), (int)i};
         nodes_.assign(std::max<size_t>(1, 2 * prims.size()), BNode());
     }
     void build(std::vector<int> &order) {
@@ -77,13 +96,13 @@ class SahBuilder {
     }
 
   private:
-    static constexpr int kBins = 16, kParallelPrims = 4096, kParallelDepth = 4;
+    static constexpr int kBins = 16, kParallelPrims = 512, kParallelDepth = 4;
     struct Ref {
-        PrimBox box;
+        F4 lo, hi, c;
         int index;
     };
     struct Bin {
-        float lo[3], hi[3];
+        F4 lo, hi;
         int count;
     };
     struct Task {
@@ -120,81 +139,81 @@ class SahBuilder {
 
     // The node's bounds, and where its primitives are parted (-1: it is a leaf).
     int split(const Task &t) {
-        float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        float clo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, chi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+        Box4 box, centres;
         for (int i = t.start; i < t.end; ++i) {
-            const PrimBox &p = refs_[(size_t)i].box;
-            grow(lo, hi, p.lo, p.hi);
-            grow(clo, chi, p.c, p.c);
+            const Ref &p = refs_[(size_t)i];
+            box.grow(p.lo, p.hi);
+            centres.grow(p.c, p.c);
         }
         BNode &nd = nodes_[(size_t)t.node];
-        std::memcpy(nd.lo, lo, sizeof(lo));
-        std::memcpy(nd.hi, hi, sizeof(hi));
+        for (int k = 0; k < 3; ++k) nd.lo[k] = box.lo[k], nd.hi[k] = box.hi[k];
         if (t.end - t.start <= max_leaf_) {
             nd.first = t.start;
             nd.count = t.end - t.start;
             return -1;
         }
-        Bin bins[3][kBins];
-        float scale[3];
-        for (int ax = 0; ax < 3; ++ax) {
-            for (Bin &b : bins[ax]) b.count = 0;
-            const float extent = chi[ax] - clo[ax];
-            scale[ax] = extent > 0.0f ? kBins / extent : 0.0f;
-        }
-        auto bin_of = [&](const PrimBox &p, int ax) {
-            return std::min(kBins - 1, std::max(0, (int)((p.c[ax] - clo[ax]) * scale[ax])));
+        const F4 clo = centres.lo, extent = centres.hi - clo;
+        const F4 scale = extent > 0.0f ? (float)kBins / extent : F4{};
+        auto bins_of = [&](const Ref &p) {
+            const I4 b = __builtin_convertvector((p.c - clo) * scale, I4);
+            const I4 from0 = b > 0 ? b : I4{};
+            return from0 < kBins - 1 ? from0 : I4{} + (kBins - 1);
         };
+        struct {
+            Bin bin[kBins];
+            unsigned used = 0;  // bit b: bin b holds a primitive
+        } axis[3];
         for (int i = t.start; i < t.end; ++i) {
-            const PrimBox &p = refs_[(size_t)i].box;
+            const Ref &p = refs_[(size_t)i];
+            const I4 at = bins_of(p);
             for (int ax = 0; ax < 3; ++ax) {
                 if (!(scale[ax] > 0.0f)) continue;
-                Bin &b = bins[ax][bin_of(p, ax)];
-                if (b.count++ == 0) {
-                    std::memcpy(b.lo, p.lo, sizeof(b.lo));
-                    std::memcpy(b.hi, p.hi, sizeof(b.hi));
+                Bin &b = axis[ax].bin[at[ax]];
+                if (axis[ax].used >> at[ax] & 1u) {
+                    b.lo = p.lo < b.lo ? p.lo : b.lo;
+                    b.hi = b.hi < p.hi ? p.hi : b.hi;
+                    ++b.count;
                 } else {
-                    grow(b.lo, b.hi, p.lo, p.hi);
+                    axis[ax].used |= 1u << at[ax];
+                    b.lo = p.lo, b.hi = p.hi;
+                    b.count = 1;
                 }
             }
         }
         float best = FLT_MAX;
         int best_axis = -1, best_bin = 0;
         for (int ax = 0; ax < 3; ++ax) {
-            if (!(scale[ax] > 0.0f)) continue;
-            const Bin *bin = bins[ax];
-            float r_area[kBins];
-            int r_count[kBins];
-            float alo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, ahi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+            // the splits above each bin that holds something, but the highest: from the top what lies
+            // above them, then from below
+            int held[kBins], n_held = 0;
+            for (unsigned left = axis[ax].used; left; left &= left - 1) held[n_held++] = __builtin_ctz(left);
+            float area[kBins];
+            int count[kBins];
+            Box4 above, below;
             int acc = 0;
-            for (int b = kBins - 1; b > 0; --b) {
-                acc += bin[b].count;
-                if (bin[b].count) {
-                    grow(alo, ahi, bin[b].lo, bin[b].hi);
-                    r_area[b] = half_area(alo, ahi);
-                } else {
-                    r_area[b] = b < kBins - 1 ? r_area[b + 1] : 0.0f;
-                }
-                r_count[b] = acc;
+            for (int k = n_held - 1; k > 0; --k) {
+                const Bin &bin = axis[ax].bin[held[k]];
+                acc += bin.count;
+                above.grow(bin.lo, bin.hi);
+                area[k] = above.half_area();
+                count[k] = acc;
             }
-            for (int k = 0; k < 3; ++k) alo[k] = FLT_MAX, ahi[k] = -FLT_MAX;
             acc = 0;
-            for (int b = 0; b < kBins - 1; ++b) {
-                if (!bin[b].count) continue;  // the split before it again
-                acc += bin[b].count;
-                grow(alo, ahi, bin[b].lo, bin[b].hi);
-                if (!r_count[b + 1]) continue;
-                const float cost = half_area(alo, ahi) * (float)acc + r_area[b + 1] * (float)r_count[b + 1];
+            for (int k = 0; k + 1 < n_held; ++k) {
+                const Bin &bin = axis[ax].bin[held[k]];
+                acc += bin.count;
+                below.grow(bin.lo, bin.hi);
+                const float cost = below.half_area() * (float)acc + area[k + 1] * (float)count[k + 1];
                 if (cost < best) {
                     best = cost;
                     best_axis = ax;
-                    best_bin = b + 1;
+                    best_bin = held[k] + 1;
                 }
             }
         }
         if (best_axis >= 0) {
             const int m = (int)(std::partition(refs_.begin() + t.start, refs_.begin() + t.end,
-                                               [&](const Ref &r) { return bin_of(r.box, best_axis) < best_bin; }) -
+                                               [&](const Ref &r) { return bins_of(r)[best_axis] < best_bin; }) -
                                 refs_.begin());
             if (m > t.start && m < t.end) return m;
         }
@@ -380,12 +399,6 @@ bool identity_inverse(const float *m) {
     return true;
 }
 
-// A leaf of the top-level tree: an instance, or a node or triangle leaf inside an opened one.
-struct TopRef {
-    PrimBox box;
-    int code;
-};
-
 struct BlasLeafCode {
     const std::vector<BNode> &bn;
     const std::vector<int> &order;
@@ -413,55 +426,30 @@ struct BlasLeafCode {
 struct TopLeafCode {
     const std::vector<BNode> &bn;
     const std::vector<int> &order;
-    const std::vector<TopRef> &refs;
+    const std::vector<ShadowRef> &refs;
     int operator()(int b) const { return refs[(size_t)order[(size_t)bn[(size_t)b].first]].code; }
     bool triangles(int b) const { return (*this)(b) < 0; }
 };
 
-}  // namespace
-
-bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, int opened_refs, ShadowBvh &b) {
-    const size_t n_inst = b.inst_root.size();
-    std::fill(b.mesh_world.begin(), b.mesh_world.end(), -1);
-    std::vector<TopRef> refs;
-    auto make_ref = [](const float *lo, const float *hi, int code) {
-        TopRef r;
-        for (int k = 0; k < 3; ++k) {
-            r.box.lo[k] = lo[k];
-            r.box.hi[k] = hi[k];
-            r.box.c[k] = 0.5f * (lo[k] + hi[k]);
-        }
-        r.code = code;
-        return r;
-    };
-    // the nodes inside opened instances, largest box on top
+// The opened instances' refs replaced by the nodes inside them, the largest box first.
+void open_instances(const std::vector<float> &nodes, const std::vector<int> &opened, std::vector<ShadowRef> &refs) {
     auto smaller = [&](int a, int c) {
-        return half_area(refs[(size_t)a].box.lo, refs[(size_t)a].box.hi) <
-               half_area(refs[(size_t)c].box.lo, refs[(size_t)c].box.hi);
+        return half_area(refs[(size_t)a].lo, refs[(size_t)a].hi) < half_area(refs[(size_t)c].lo, refs[(size_t)c].hi);
     };
-    std::vector<int> heap;
-    for (size_t i = 0; i < n_inst; ++i) {
-        if (b.inst_root[i] < 0) continue;
-        if (!encodable(inst_bounds + 6 * i, inst_bounds + 6 * i + 3)) return false;
-        int &world = b.mesh_world[(size_t)b.inst_mesh[i]];
-        const bool open = world < 0 && identity_inverse(inst_records + 32 * i);
-        refs.push_back(make_ref(inst_bounds + 6 * i, inst_bounds + 6 * i + 3,
-                                open ? b.inst_root[i] : (kSh4InstBit | (int)i)));
-        if (open) {
-            world = (int)i;
-            heap.push_back((int)refs.size() - 1);
-        }
-    }
+    std::vector<int> heap = opened;
     std::make_heap(heap.begin(), heap.end(), smaller);
-    const size_t limit = refs.size() + (size_t)std::min(opened_refs, kSh4OpenedRefs);
+    const size_t limit = refs.size() + (size_t)kSh4OpenedRefs;
     while (!heap.empty() && refs.size() + 3 <= limit) {
         std::pop_heap(heap.begin(), heap.end(), smaller);
         const int at = heap.back();
         heap.pop_back();
-        const Node4 node = load_node(b.nodes, refs[(size_t)at].code);
+        const Node4 node = load_node(nodes, refs[(size_t)at].code);
         int pos = at;  // the first child takes the opened node's place
         for (int k = 0; k < node.children; ++k) {
-            const TopRef child = make_ref(node.lo[k], node.hi[k], node.entry[k]);
+            ShadowRef child;
+            std::memcpy(child.lo, node.lo[k], sizeof(child.lo));
+            std::memcpy(child.hi, node.hi[k], sizeof(child.hi));
+            child.code = node.entry[k];
             if (pos < (int)refs.size())
                 refs[(size_t)pos] = child;
             else
@@ -473,11 +461,61 @@ bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, in
             pos = (int)refs.size();
         }
     }
+}
+
+}  // namespace
+
+bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, ShadowBvh &b) {
+    const size_t n_inst = b.inst_root.size();
+    std::fill(b.mesh_world.begin(), b.mesh_world.end(), -1);
+    std::vector<ShadowRef> refs;
+    auto make_ref = [](const float *lo, const float *hi, int code) {
+        ShadowRef r;
+        std::memcpy(r.lo, lo, sizeof(r.lo));
+        std::memcpy(r.hi, hi, sizeof(r.hi));
+        r.code = code;
+        return r;
+    };
+    std::vector<int> opened;  // positions in refs of the opened instances
+    for (size_t i = 0; i < n_inst; ++i) {
+        if (b.inst_root[i] < 0) continue;
+        if (!encodable(inst_bounds + 6 * i, inst_bounds + 6 * i + 3)) return false;
+        int &world = b.mesh_world[(size_t)b.inst_mesh[i]];
+        const bool open = world < 0 && identity_inverse(inst_records + 32 * i);
+        refs.push_back(make_ref(inst_bounds + 6 * i, inst_bounds + 6 * i + 3,
+                                open ? b.inst_root[i] : (kSh4InstBit | (int)i)));
+        if (open) {
+            world = (int)i;
+            opened.push_back((int)refs.size() - 1);
+        }
+    }
+    // An identity instance's nodes stand where they stood: moves that open the same instances again
+    // take the leaves of the last time.
+    const size_t n_base = refs.size();
+    if (!b.opened.empty() && opened == b.opened) {
+        for (size_t k = 0; k < opened.size(); ++k) refs[(size_t)opened[k]] = b.opened_refs[k];
+        refs.insert(refs.end(), b.opened_refs.begin() + (ptrdiff_t)opened.size(), b.opened_refs.end());
+    } else {
+        open_instances(b.nodes, opened, refs);
+        b.opened = opened;
+        b.opened_refs.clear();
+        for (int at : opened) b.opened_refs.push_back(refs[(size_t)at]);
+        b.opened_refs.insert(b.opened_refs.end(), refs.begin() + (ptrdiff_t)n_base, refs.end());
+    }
     std::vector<float> top;
     b.tlas_depth = 0;
     if (!refs.empty()) {
         std::vector<PrimBox> prims;
-        for (const TopRef &r : refs) prims.push_back(r.box);
+        prims.reserve(refs.size());
+        for (const ShadowRef &r : refs) {
+            PrimBox p;
+            for (int k = 0; k < 3; ++k) {
+                p.lo[k] = r.lo[k];
+                p.hi[k] = r.hi[k];
+                p.c[k] = 0.5f * (r.lo[k] + r.hi[k]);
+            }
+            prims.push_back(p);
+        }
         std::vector<BNode> bn;
         std::vector<int> order;
         build_binary(prims, 1, bn, order);
@@ -492,6 +530,7 @@ bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, in
         b.tlas_depth = 1;
     }
     std::memcpy(b.nodes.data(), top.data(), top.size() * sizeof(float));
+    b.tlas_nodes = (int)(top.size() / kSh4NodeFloats);
     // a walk holds at most 3 entries per level it has descended, the end marker, one in hand, and one
     // that leads back to the world ray
     return 3 + 3 * (b.tlas_depth + b.blas_depth) <= kSh4Stack;
@@ -580,7 +619,7 @@ bool build_shadow_bvh(const hdr_scene_desc &desc, const FlatScene &flat, ShadowB
     }
     shadow_ranks(flat.tlas_inst, n_inst, out.inst_rank);
     // not an error when it does not fit: the reference trees serve these queries too
-    out.ok = rebuild_shadow_tlas(flat.inst_bounds.data(), flat.instances.data(), kSh4OpenedRefs, out);
+    out.ok = rebuild_shadow_tlas(flat.inst_bounds.data(), flat.instances.data(), out);
     return true;
 }
 

@@ -50,6 +50,12 @@ namespace hdr {
 
 struct FlatScene;
 
+// A leaf of the top-level tree: an instance, or a node or triangle leaf inside an opened one.
+struct ShadowRef {
+    float lo[3], hi[3];
+    int code;
+};
+
 struct ShadowBvh {
     std::vector<float> nodes;
     std::vector<float> tris;
@@ -57,7 +63,10 @@ struct ShadowBvh {
     std::vector<int> inst_mesh;   // per instance: its mesh
     std::vector<int> inst_rank;   // per instance: its position in the reference TLAS's leaf order
     std::vector<int> mesh_world;  // per mesh: the instance whose nodes are opened, -1 = none
+    std::vector<int> opened;      // the opened instances, by their place among those with triangles
+    std::vector<ShadowRef> opened_refs;  // the leaves in their places, then the other ones inside them
     int tlas_capacity = 0;        // nodes reserved for the top-level tree at the front of `nodes`
+    int tlas_nodes = 0;           // and those it takes
     int tlas_depth = 0, blas_depth = 0;
     bool ok = false;              // false: not built (the scene is walked with the reference trees)
 };
@@ -74,11 +83,10 @@ bool build_shadow_bvh(const hdr_scene_desc &desc, const FlatScene &flat, ShadowB
 void shadow_ranks(const std::vector<int> &tlas_inst, int num_instances, std::vector<int> &rank);
 
 // Rebuilds the top-level tree over instances that moved: `inst_bounds` (6 floats each, the
-// world boxes) and `inst_records` (32 floats each, the inverse transform first), with at most
-// opened_refs leaves from opened instances (no more than kSh4OpenedRefs). Reads the
-// BLAS nodes, inst_root and inst_mesh of `b`, and writes its mesh_world, the first nodes of
-// b.nodes and b.tlas_depth; returns false when the tree does not fit the reserved room or the
+// world boxes) and `inst_records` (32 floats each, the inverse transform first). Reads the
+// BLAS nodes, inst_root and inst_mesh of `b`, and writes its mesh_world, opened, opened_refs, the
+// first nodes of b.nodes and b.tlas_depth; returns false when the tree does not fit the reserved room or the
 // stack bound.
-bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, int opened_refs, ShadowBvh &b);
+bool rebuild_shadow_tlas(const float *inst_bounds, const float *inst_records, ShadowBvh &b);
 
 }  // namespace hdr
