@@ -200,7 +200,7 @@ struct HitId {
 
 // The triangle field of a wavefront hit slot: the index, and in the four bits above it
 // (the upload limits a scene to 2^27 triangles) how many units in the last place beyond
-// t the SAH walk found no other hit (Closest4Walk::bound).
+// t the reference's walk has no hit before it (Closest4Walk::bound).
 __device__ __forceinline__ int hit_pack(int tri, int bound_ulps) { return tri | (bound_ulps << 27); }
 __device__ __forceinline__ int hit_tri(int packed) { return packed & 0x07ffffff; }
 __device__ __forceinline__ int hit_bound_ulps(int packed) { return packed >> 27; }
@@ -786,17 +786,17 @@ __device__ bool trace_ray_wide(const DeviceScene &s, V3 o, V3 d, float t_limit, 
 namespace hdr {
 
 // The check of a closest hit found on the 4-wide SAH trees (DeviceScene::sh4_closest
-// == 2). The reference's walk (scene.cpp:414-510, bvh.cpp:243-305) skips a node only
-// when its slab test fails or its entry distance exceeds the running closest t. The
-// SAH walk reports `bound` (Closest4Walk::bound): no hit of the scene but this one lies
-// in [t, bound), so the running t does not drop below `bound` before the hit's triangle
-// is tested. Hence, if every box on the way from the TLAS root down to the instance's
-// leaf, and from the instance's BLAS root down to the triangle's leaf (object-space
-// ray, BLAS thresholds), passes the reference's slab test with an entry distance no
-// farther than `bound`, the reference walk tests the triangle and takes it: the same
-// IntersectTriangle arithmetic gives the same t, and the SAH walk breaks ties in the
-// reference's walk order. A hit that grazes a box the reference's rounding rejects
-// fails the check.
+// == 2). The reference's walk (scene.cpp:414-510, bvh.cpp:243-305) visits left children
+// first and skips a node only when its slab test fails or its entry distance exceeds the
+// running closest t. The SAH walk reports `bound` (Closest4Walk::bound): no hit that the
+// reference's walk meets before this one lies in [t, bound), so the running t does not drop
+// below `bound` before the hit's triangle is tested. Hence, if every box on the way from the
+// TLAS root down to the instance's leaf, and from the instance's BLAS root down to the
+// triangle's leaf (object-space ray, BLAS thresholds), passes the reference's slab test with
+// an entry distance no farther than `bound`, the reference walk tests the triangle and takes
+// it: the same IntersectTriangle arithmetic gives the same t, and the SAH walk breaks ties in
+// the reference's walk order. A hit that grazes a box the reference's rounding rejects fails
+// the check.
 //
 // Only the two leaves are tested. Every node's box is the exact union of its
 // children's, and the rounded products (bound - o) * inv are monotone in the bound:

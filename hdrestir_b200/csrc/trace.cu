@@ -298,7 +298,11 @@ __global__ void __launch_bounds__(kTraceThreads, kMinBlocks) trace_both4_kernel(
 // entry whose hit ref_reaches cannot vouch for walks the reference's trees here. Few do (of
 // 500,000 random rays the unchecked walk answers 19 differently among coplanar boxes, none over
 // the terrain), so they get no list and no kernel of their own: the two kernels took 208 us of
-// the four rounds of a 256 x 256 path-traced box, this one takes 23. A miss needs no check: the SAH trees' boxes hold every triangle, so
+// the four rounds of a 256 x 256 path-traced box, this one takes 23. Surfaces within a few units
+// in the last place of each other reject more: a room's walls four times over, 0 to 3 units
+// apart, 1080p: RIS with all rays 7.65 ms (6.84 with the list), path tracing at depth 4 6.0 (7.4);
+// walls twice over are no slower than with it. Walking a block's rejected entries side by side
+// was slower still (8.46). A miss needs no check: the SAH trees' boxes hold every triangle, so
 // the reference walk finds no hit either.
 __global__ void __launch_bounds__(256) check_closest_kernel(const __grid_constant__ DeviceScene s,
                                                             const float4 *__restrict__ q, const int *count,
