@@ -50,35 +50,6 @@ __device__ __forceinline__ bool same_bits(float4 a, float4 b) {
            __float_as_int(a.z) == __float_as_int(b.z) && __float_as_int(a.w) == __float_as_int(b.w);
 }
 
-// ApplyFireflySuppression's body for pixel (x, y): neighbours earlier in
-// row-major order come from `prev` (when given), later ones (and the pixel
-// itself, which a clamped coordinate at the border can name) from `orig`.
-__device__ __forceinline__ float4 firefly_pixel(const float4 *__restrict__ orig, const float4 *prev, int x, int y,
-                                                int width, int height) {
-    const size_t p = (size_t)y * width + x;
-    float4 c = orig[p];
-    const float lum = lum4(c);
-    float max_n = 0.0f;
-    for (int dy = -1; dy <= 1; ++dy) {
-        for (int dx = -1; dx <= 1; ++dx) {
-            if (dx == 0 && dy == 0) continue;
-            const int nx = sclampi(x + dx, 0, width - 1);
-            const int ny = sclampi(y + dy, 0, height - 1);
-            const size_t q = (size_t)ny * width + nx;
-            const float4 v = (prev && q < p) ? prev[q] : orig[q];
-            max_n = smaxf(max_n, lum4(v));
-        }
-    }
-    const float thr = max_n * 4.0f + 0.5f;
-    if (lum > thr && lum > 0.0f) {
-        const float scale = thr / lum;
-        c.x *= scale;
-        c.y *= scale;
-        c.z *= scale;
-    }
-    return c;
-}
-
 // A tile of kTileW x kTileH pixels per block: a thread has kRows rows of one column, a warp
 // kRows rows. The luminances of the tile and of the two pixels around it are in shared memory: a
 // pixel's neighbours, and theirs for the in-place check, are clamped coordinates of the frame,
@@ -204,29 +175,67 @@ __global__ void __launch_bounds__(kTileThreads)
     }
 }
 
-// The row-major in-place clamp, exactly, by one block. Pixel (x, y) depends on its earlier
-// neighbours (x-1, y), (x-1, y-1), (x, y-1), (x+1, y-1) (or on itself, at the
-// border), and all of them lie on earlier anti-diagonals t = x + 2y. So the
-// block walks t = 0 .. (w-1) + 2(h-1), computes every pixel of one diagonal in
-// parallel from the final values of earlier ones (in `plane`) and the
-// unclamped values of later ones (in `orig`), and meets at a barrier before the
-// next diagonal. Bounded: w + 2h - 2 steps, each at most min(h, w/2 + 1) pixels.
-__device__ __noinline__ void firefly_sequential(const float4 *orig, float4 *plane, int width, int height) {
-    const int t_end = (width - 1) + 2 * (height - 1);
-    for (int t = 0; t <= t_end; ++t) {
-        // y with 0 <= t - 2y <= width - 1 and 0 <= y <= height - 1
-        const int y_lo = smaxi(0, (t - (width - 1) + 1) / 2);
-        const int y_hi = smini(height - 1, t / 2);
-        for (int y = y_lo + (int)threadIdx.x; y <= y_hi; y += (int)blockDim.x) {
-            const int x = t - 2 * y;
-            plane[(size_t)y * width + x] = firefly_pixel(orig, plane, x, y, width, height);
-        }
-        __syncthreads();
-    }
-}
-
 __device__ __forceinline__ float4 mean_of(float4 a, float inv_n) {
     return make_float4(a.x * inv_n, a.y * inv_n, a.z * inv_n, a.w * inv_n);
+}
+
+// The row-major in-place clamp, exactly, with the sum and the mean in the colour's place, by one
+// block of 1024 threads. Pixel (x, y) depends on its earlier neighbours (x-1, y), (x-1, y-1),
+// (x, y-1), (x+1, y-1), so a thread walks a row two pixels behind the row above, with a barrier
+// after each step, and the rows pass their luminances on in shared memory: the clamped one of a
+// pixel when it is clamped, the unclamped one four steps earlier, when the row above comes to need
+// it (at time t thread k is at x and reads x-1 .. x+1 of k-1, which clamps x+2, and of k+1, which
+// publishes x+2: rings of four have the slots apart). Rows are taken kWalkRows at a time: thread 0
+// publishes the last row of the rows before, kept in last_row, the thread past the last row the
+// unclamped row below. Bounded: w + 2 kWalkRows + 6 steps for each kWalkRows rows.
+//
+// Uncoalesced by its nature (a warp's lanes are in 32 rows): what bounds it is the count of
+// accesses, three loads and two stores a pixel: 1.43, 9.55 and 35.3 ms for a frame of 640 x 360,
+// 1920 x 1080 and 3840 x 2160 (1.64, 10.8 and 47.0 with the eight neighbours' colours from memory
+// and the sum and mean in a pass of this block's own).
+constexpr int kWalkRows = 1022;
+__device__ __noinline__ void firefly_sequential(float4 *color, float *last_row, float4 *accum, int width, int height,
+                                                float inv_n) {
+    __shared__ float unclamped[4][1024], clamped[4][1024];
+    const int k = threadIdx.x;
+    for (int y0 = 0; y0 < height; y0 += kWalkRows) {
+        const int rows = smini(kWalkRows, height - y0), y = y0 - 1 + k;
+        const bool own = k >= 1 && k <= rows, ahead = k >= 1 && k <= rows + 1 && y < height;
+        const size_t row = (size_t)smaxi(y, 0) * width;
+        const int steps = width + 4 + 2 * (rows + 1);
+        for (int t = 0; t < steps; ++t) {
+            const int x = t - 4 - 2 * k;
+            if (ahead && x + 4 >= 0 && x + 4 < width) unclamped[x & 3][k] = lum4(color[row + x + 4]);
+            if (x >= 0 && x < width && k == 0 && y0 > 0) clamped[x & 3][0] = last_row[x];
+            if (x >= 0 && x < width && own) {
+                const float4 c = color[row + x], b = accum[row + x];
+                const float lum = lum4(c);
+                const int l = (x - 1) & 3, m = x & 3, r = (x + 1) & 3;
+                const bool left = x > 0, right = x + 1 < width, up = y > 0, down = y + 1 < height;
+                // (a clamped coordinate at the border names the pixel itself)
+                float max_n = left && right && up && down ? 0.0f : smaxf(0.0f, lum);
+                if (left) max_n = smaxf(max_n, clamped[l][k]);
+                if (right) max_n = smaxf(max_n, unclamped[r][k]);
+                if (up) {
+                    if (left) max_n = smaxf(max_n, clamped[l][k - 1]);
+                    max_n = smaxf(max_n, clamped[m][k - 1]);
+                    if (right) max_n = smaxf(max_n, clamped[r][k - 1]);
+                }
+                if (down) {
+                    if (left) max_n = smaxf(max_n, unclamped[l][k + 1]);
+                    max_n = smaxf(max_n, unclamped[m][k + 1]);
+                    if (right) max_n = smaxf(max_n, unclamped[r][k + 1]);
+                }
+                const float4 f = firefly_clamp(c, lum, max_n * 4.0f + 0.5f);
+                const float4 a = make_float4(b.x + f.x, b.y + f.y, b.z + f.z, b.w + f.w);
+                clamped[m][k] = lum4(f);
+                if (k == rows) last_row[x] = lum4(f);
+                accum[row + x] = a;
+                color[row + x] = mean_of(a, inv_n);
+            }
+            __syncthreads();
+        }
+    }
 }
 
 // The mean, and the sums in their place (kParity; else sums is accum itself). From the last
@@ -240,14 +249,7 @@ __global__ void __launch_bounds__(1024, 2) mean_kernel(float4 *sums, float4 *acc
     if (frame_slot) inv_n = 1.0f / (float)(*frame_slot + 1);
     const size_t count = (size_t)width * height;
     if (kParity && *changed) {  // the same for every thread
-        if (blockIdx.x != 0) return;
-        firefly_sequential(out, sums, width, height);
-        for (size_t p = threadIdx.x; p < count; p += blockDim.x) {
-            const float4 c = sums[p], b = accum[p];
-            const float4 a = make_float4(b.x + c.x, b.y + c.y, b.z + c.z, b.w + c.w);
-            accum[p] = a;
-            out[p] = mean_of(a, inv_n);
-        }
+        if (blockIdx.x == 0) firefly_sequential(out, (float *)sums, accum, width, height, inv_n);
         return;
     }
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) {
