@@ -89,13 +89,13 @@ struct SceneStore {
     float *xf_staging = nullptr;    // 16 floats per instance
     int4 *tlas_stack = nullptr;     // num_instances + 2 entries
     int *tlas_info = nullptr;       // 4 ints
-    // shadow-ray BVH (host/shadow_bvh.h): present when sh4 is true; the TLAS part is
+    // 4-wide SAH trees (host/shadow_bvh.h): present when sh4 is true; the top-level tree is
     // rebuilt on the host when instances move
     bool sh4 = false;
-    // the reference trees' parent links for exact SAH closest hits (closest_mode 2); they
-    // describe the uploaded TLAS, so moving instances on the device clears this
+    // the leaves of the reference's trees are known for the check of closest hits (closest_mode
+    // 2); moving instances finds the instances' again
     bool ref_links = false;
-    // its host copy, from which hdr_scene_set_instance_transforms rebuilds the top-level tree
+    // the SAH trees' host copy, from which hdr_scene_set_instance_transforms rebuilds the top-level tree
     // (nodes, roots and mesh table; the triangles are dropped after the upload)
     hdr::ShadowBvh sh4_host;
     // the scene's arrays by DeviceScene field name, for hdr_scene_array
@@ -684,8 +684,8 @@ namespace {
 // per TLAS node its parent, per instance its TLAS leaf, per BLAS node (all meshes,
 // mesh-local indices) its parent, per triangle record its mesh-local leaf. Only
 // nodes a walk can reach are linked (-1 elsewhere). Needs the host-built trees.
-// The check's path records: per TLAS node and per BLAS node, 8 floats (32 B, one
-// sector): the node's box min, its parent's index bits (-1 at a root), its box max, 0.
+// Where the check of closest hits (closest_mode 2) finds a hit's boxes in the reference's trees:
+// each instance's TLAS leaf, and each triangle record's BLAS leaf, counted from its mesh's root.
 struct RefLinks {
     std::vector<int> inst_leaf, tri_leaf;
 };

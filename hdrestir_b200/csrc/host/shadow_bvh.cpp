@@ -595,7 +595,7 @@ bool build_shadow_bvh(const hdr_scene_desc &desc, const FlatScene &flat, ShadowB
         Collapser col{bn, out.nodes, 0};
         int root = 0;
         const size_t tri_base = out.tris.size() / kTriGeoFloats;
-        if (tri_base + nt >= ((size_t)1 << 27)) {  // leaf entries: (first << 4) | ... fits 31 bits
+        if (tri_base + nt >= ((size_t)1 << 27)) {  // leaf entries: (first << 2) | ... fits 29 bits
             err = "too many triangles for the shadow BVH encoding";
             return false;
         }

@@ -1,24 +1,23 @@
-// Shadow-ray BVH (no reference counterpart): a second acceleration structure
-// over the same triangles and instances, used only for the query "is there a
-// hit nearer than the light" (the visibility test of _evaluateLightSample,
-// ris_direct_light_integrator.cpp:628-658, and of the MIS integrator's NEE,
-// mis_direct_light_integrator.cpp:140-151).
+// 4-wide SAH trees (no reference counterpart): a second acceleration structure over the same
+// triangles and instances, for the query "is there a hit nearer than the light" (the visibility
+// test of _evaluateLightSample, ris_direct_light_integrator.cpp:628-658, and of the MIS
+// integrator's NEE, mis_direct_light_integrator.cpp:140-151) and for closest hits.
 //
-// The answer of that query does not depend on the tree: the reference walks its
+// The answer of the first query does not depend on the tree: the reference walks its
 // midpoint-split trees and compares the closest hit with the light distance,
 // and a hit exists below the limit exactly when some triangle test (the same
 // IntersectTriangle arithmetic in the same instance space) returns one. So this
 // structure is built for speed: binned-SAH binary trees collapsed to 4 children
 // per node, each node holding its children's boxes (tested together, before
-// descending), triangles in leaf order. Closest hits keep walking the
-// reference-order trees, whose tie-breaks they need.
+// descending), triangles in leaf order.
 //
 // The same trees answer closest-hit queries with the reference's result: every
 // triangle record carries its index in the reference's BLAS triangle order, and
 // every instance its position in the reference TLAS's leaf order; among hits at
 // equal distance the walk keeps the smallest (instance position, triangle
 // index), which is the one the reference's left-first walks find first
-// (bvh.cpp:262-304, scene.cpp:414-510, strict `<` on t).
+// (bvh.cpp:262-304, scene.cpp:414-510, strict `<` on t). Whether the reference's own
+// rounded box tests let it reach that hit is checked afterwards (ref_reaches, device/traverse.cuh).
 //
 // Records and entries: device/sh4_layout.h. Children stand in the order an any-hit walk tries
 // them: triangles first, then the smaller box first (a small box is cheap to finish
