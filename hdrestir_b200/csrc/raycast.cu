@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(256) raycast_kernel(const __grid_constant__ De
     const RayF ray = centre_ray(cam, live_frame(cam, frame_arg), x, y, i);
     unsigned e = 0;
     HitId hid;
-    const bool has = trace_ray<false>(s, ray.o, ray.d, 0.0f, hid, e);
+    const bool has = s.wide ? trace_ray_wide<false>(s, ray.o, ray.d, 0.0f, hid, e)
+                            : trace_ray_binary<false>(s, ray.o, ray.d, 0.0f, hid, e);
     write_pixel(s, gb, aov, i, ray, has, hid);
     if (e) atomicOr(err, e);
 }
