@@ -436,10 +436,11 @@ __global__ void __launch_bounds__(kTraceThreads) trace_shadow_kernel(DeviceScene
 int launch_wave_trace(const DeviceScene &s, WaveBuffers wb, const TraceTuning &tune, unsigned *err, cudaStream_t st,
                       cudaEvent_t *ev_begin, cudaEvent_t *ev_end) {
     auto mark = [&](cudaEvent_t *ev, int k) { return !ev || cudaEventRecord(ev[k], st) == cudaSuccess; };
-    const int most = tune.sm_count * tune.blocks_per_sm;
+    const bool refill = (tune.mode & kTraceLanePerRay) == 0;
+    // a lane that keeps its ray has its share of the queue fixed by the grid: smaller shares
+    const int most = tune.sm_count * tune.blocks_per_sm * (refill ? 1 : 2);
     const int cgrid = grid_for(most, wb.closest_slots, kTraceThreads);
     const int sgrid = grid_for(most, wb.shadow_slots, kTraceThreads);
-    const bool refill = (tune.mode & kTraceLanePerRay) == 0;
     const bool phased = refill && (tune.mode & kTraceUnphased) == 0;
     const bool shallow = s.shallow && (tune.mode & kTraceSplitStack) == 0;
     const bool both = s.sh4 && s.sh4_closest && wb.closest_slots > 0 && !ev_begin;  // not timed one by one
