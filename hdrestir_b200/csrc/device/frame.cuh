@@ -100,8 +100,8 @@ struct WaveBuffers {
     float *hit_v;         // pixels * n_closest
     unsigned char *occ;   // n_shadow planes of pixels
     // n_shadow planes of pixels: each light candidate's resampling weight if its shadow ray is
-    // unoccluded (float with a reservoir, double without; nee_weight_bits); nullptr: no room for
-    // them, the shade kernel evaluates the candidates again
+    // unoccluded (float with a reservoir, double without; nee_weight_bits); nullptr: no use or no
+    // room for them, the shade kernel evaluates the candidates again
     void *nee_weight;
     uint4 *rng_state;     // 3 planes of pixels: stream state at the end of candidate generation
                           // (store_stream_from)
@@ -199,6 +199,15 @@ inline int draws_to_generation_end(const RisParamsD &p) {
     const int n_nee = p.candidate_count / 2 > 1 ? p.candidate_count / 2 : 1;
     const int n_bsdf = p.candidate_count > n_nee ? p.candidate_count - n_nee : 0;
     return 5 + 3 * n_nee + 5 * (n_bsdf + 1);
+}
+// Can any pixel's resampling read stored weights? With a reservoir only one whose stream is below
+// draw 312 at the end of generation (ris_direct_li): no fewer draws than the pixel's two, the
+// wavelength, those of every light candidate and one per bounce.
+inline bool weights_read(const DeviceScene &s, const RisParamsD &p) {
+    const int n_nee = p.candidate_count / 2 > 1 ? p.candidate_count / 2 : 1;
+    const int n_bsdf = p.candidate_count > n_nee ? p.candidate_count - n_nee : 1;
+    const int per_light = s.num_lights <= 0 ? 0 : (s.nee_draws > 0 ? s.nee_draws : 1);
+    return !p.use_reservoir || 3 + n_nee * per_light + n_bsdf < 312;
 }
 // Does ris_resample_kernel serve the frame (else ris_shade_kernel, which has one shape)? It
 // continues a stream it has not replayed, whose state travels only below draw 312.

@@ -439,10 +439,10 @@ struct RisNeeRay {  // a light candidate as the generate kernel leaves it
 // _evaluateLightSample, :628-673): the values ris_nee_candidate computes after the trace.
 // A candidate that the early-outs drop weighs 0 whatever its densities are, unless the
 // light's density is a NaN (an environment with an infinite texel) or its square overflows (mis
-// is then undefined): only then are they evaluated.
+// is then undefined): only then are they evaluated. weigh: the weight is wanted.
 __device__ __forceinline__ RisNeeRay ris_nee_ray(const DeviceScene &s, const Surface &sf, int li,
                                                  const LightSampleD &ls, const RisStrategy &strat,
-                                                 const SpectralCtx &sc) {
+                                                 const SpectralCtx &sc, bool weigh) {
     RisNeeRay r;
     const float n_l = dot(sf.sn, ls.dir);
     const float dist2 = ls.dist * ls.dist;
@@ -456,7 +456,7 @@ __device__ __forceinline__ RisNeeRay ris_nee_ray(const DeviceScene &s, const Sur
     r.limit = ls.dist - 1e-3f;
     r.weight = 0.0;
     r.stays = false;
-    if (dropped && isfinite(p_nee * p_nee)) return r;
+    if (!weigh || (dropped && isfinite(p_nee * p_nee))) return r;
     const V3 wo = -sf.ray_d;
     const float mis = delta ? 1.0f
                             : power_heuristic3(p_nee, strat.n_nee, 0.0f, strat.n_sky,

@@ -1394,9 +1394,11 @@ static hdr_status ris_path_trace_pass(hdr_ctx *c, const hdr_camera *cam, int32_t
         // Last, since a frame for which only the weights have no room (a budget, a recording that
         // cannot allocate) renders without them: the same image, its light candidates evaluated
         // a second time after the trace.
-        st = ensure_scratch(c, kWeightBuffers[p->use_reservoir ? 0 : 1], count * wb.n_shadow * nee_weight_size(p), &q);
-        if (st != HDR_OK && st != HDR_ENOMEM && !c->recording) return st;
-        wb.nee_weight = st == HDR_OK ? q : nullptr;
+        if (hdr::weights_read(c->scene, d)) {
+            st = ensure_scratch(c, kWeightBuffers[p->use_reservoir ? 0 : 1], count * wb.n_shadow * nee_weight_size(p), &q);
+            if (st != HDR_OK && st != HDR_ENOMEM && !c->recording) return st;
+            wb.nee_weight = st == HDR_OK ? q : nullptr;
+        }
         if ((st = begin_pass(c, 1)) != HDR_OK) return st;
         const bool timed = timing_on(c);
         if (timed)
@@ -1716,7 +1718,7 @@ hdr_status prepare_ris_job(hdr_ctx *c, const hdr_camera *cam, int32_t frame_inde
     j.trace_level = ris_trace_level(c, p);
     j.n_closest = closest_slots(j.trace_level, std::max(0, p->candidate_count - n_nee));
     j.n_shadow = n_nee;
-    j.weight_bytes = (j.count * j.n_shadow * nee_weight_size(p) + 15) & ~(size_t)15;
+    j.weight_bytes = hdr::weights_read(c->scene, d) ? (j.count * j.n_shadow * nee_weight_size(p) + 15) & ~(size_t)15 : 0;
     if ((st = ensure_buffer(c, "__wave_rng", j.count * 48, &q)) != HDR_OK) return st;
     j.rng_state = (uint4 *)q;
     if ((st = ensure_buffer(c, "__wave_done", j.count, &q)) != HDR_OK) return st;
@@ -1822,7 +1824,7 @@ hdr_status hdr_ris_path_trace_batch(hdr_ctx *const *ctxs, int32_t n, const hdr_c
         wb.hits = all.hits + base_c[(size_t)i];
         wb.hit_v = all.hit_v + base_c[(size_t)i];
         wb.occ = all.occ + base_s[(size_t)i];
-        wb.nee_weight = weights;
+        wb.nee_weight = j.weight_bytes ? weights : nullptr;
         if (weights) weights += j.weight_bytes;
         wb.rng_state = j.rng_state;
         wb.done = j.done;

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kGenerateThreads, 4)
         ray.weight = 0.0;
         const bool proposed = propose_candidate(s, ps.hit.position, rng, li, ls);
         if (wb.nee_light) wb.nee_light[i * (size_t)wb.n_shadow + j] = proposed ? li : -1;
-        if (proposed) ray = ris_nee_ray(s, sf, li, ls, strat, ps.sc);
+        if (proposed) ray = ris_nee_ray(s, sf, li, ls, strat, ps.sc, wb.nee_weight != nullptr);
         const size_t slot = (size_t)j * wb.pixels + i;
         if (!wb.nee_weight) {
         } else if (ris.use_reservoir) {
