@@ -79,7 +79,7 @@ constexpr int kPixelConnNan = 4;  // and its pdf squared overflows: its weight i
 // Shape: four blocks of 128 (128 registers, nothing spilled). Five (96 registers): 1.45, 0.115,
 // 0.416 ms; six (80): 1.41, 0.117, 0.415.
 constexpr int kGenerateThreads = 128;
-template <class Rng>  // MtShort where draws_to_generation_end is at most 155
+template <class Rng, bool kWeights>  // MtShort where draws_to_generation_end is at most 155
 __global__ void __launch_bounds__(kGenerateThreads, 4)
     ris_generate_kernel(const __grid_constant__ DeviceScene s, const __grid_constant__ CameraD cam, int frame_arg,
                         const __grid_constant__ PathRun pr, const __grid_constant__ RisRun ris,
@@ -133,13 +133,13 @@ __global__ void __launch_bounds__(kGenerateThreads, 4)
         ray.weight = 0.0;
         const bool proposed = propose_candidate(s, ps.hit.position, rng, li, ls);
         if (wb.nee_light) wb.nee_light[i * (size_t)wb.n_shadow + j] = proposed ? li : -1;
-        if (proposed) ray = ris_nee_ray(s, sf, li, ls, strat, ps.sc, wb.nee_weight != nullptr);
+        if (proposed) ray = ris_nee_ray(s, sf, li, ls, strat, ps.sc, kWeights);
         const size_t slot = (size_t)j * wb.pixels + i;
-        if (!wb.nee_weight) {
-        } else if (ris.use_reservoir) {
-            ((float *)wb.nee_weight)[slot] = nee_weight_bits<float>(ray.weight, ray.stays);
-        } else {
-            ((double *)wb.nee_weight)[slot] = nee_weight_bits<double>(ray.weight, ray.stays);
+        if (kWeights) {
+            if (ris.use_reservoir)
+                ((float *)wb.nee_weight)[slot] = nee_weight_bits<float>(ray.weight, ray.stays);
+            else
+                ((double *)wb.nee_weight)[slot] = nee_weight_bits<double>(ray.weight, ray.stays);
         }
         const int q = queue_append(&wb.counts[1], ray.cast);
         if (q >= 0) {
@@ -404,7 +404,9 @@ RisRun ris_run(const RisParamsD &p) {
 int launch_ris_generate(const DeviceScene &s, const CameraD &cam, int frame_index, const RisParamsD &p,
                         GBufferView gb, WaveBuffers wb, float4 *color, int trace_level, unsigned *err,
                         cudaStream_t st) {
-    auto k = draws_to_generation_end(p) <= 155 ? ris_generate_kernel<MtShort> : ris_generate_kernel<MtStream>;
+    const bool few = draws_to_generation_end(p) <= 155;
+    auto k = wb.nee_weight ? (few ? ris_generate_kernel<MtShort, true> : ris_generate_kernel<MtStream, true>)
+                           : (few ? ris_generate_kernel<MtShort, false> : ris_generate_kernel<MtStream, false>);
     k<<<tile_blocks<kGenerateThreads>(cam.width, cam.height), kGenerateThreads, 0, st>>>(
         s, cam, frame_index, path_run(p), ris_run(p), gb, wb, color, trace_level, err);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
