@@ -398,15 +398,14 @@ struct Sh4LocalStack {
 // `<`. The nearest hit child is taken into hand, the others are pushed as they stand
 // (sorting them too saves 1 % of the node steps).
 //
-// second_t is the nearest hit that the reference's walk meets before the closest one, as far as
-// it lies within 2^-18 of it: of two hits that close, the order of the reference's trees tells
-// which comes first. Boxes are culled 2^-18 of the way beyond the closest t, so every triangle
-// hit up to 15 units in the last place (less than 2^-19) beyond it has been tested: bound() is
-// the distance below which the reference's walk has no hit when it comes to the closest one's
-// triangle. A surface that coincides with the closest one and comes later leaves the bound as it
-// is; with any coinciding surface lowering it, the check rejected the hits on coincident walls
-// (65 boxes twice over, 1080p: RIS with all rays 3.00 -> 2.05 ms, path tracing at depth 4 1.75 ->
-// 1.21, primary rays 0.38 -> 0.15).
+// second_t is the nearest hit seen beyond the closest one's distance. Boxes are culled 2^-18
+// of the way beyond the closest t, so every triangle hit up to 15 units in the last place
+// (less than 2^-19) beyond it has been tested: bound() is the distance below which the
+// reference's walk has no hit when it comes to the closest one's triangle. Hits at the very
+// distance do not lower it, for the closest one is the first of them in that walk's order. (With
+// no slack left for a hit that another surface coincides with, the check rejected the hits on
+// coincident walls: 65 boxes twice over, 1080p: RIS with all rays 3.00 -> 2.05 ms, path tracing
+// at depth 4 1.75 -> 1.22, primary rays 0.38 -> 0.15.)
 constexpr float kSh4CullPast = 1.0f + 3.814697265625e-06f;
 constexpr int kSh4BoundUlps = 15;
 
@@ -475,23 +474,22 @@ struct Closest4Walk : Walk4Base<Stk, Src> {
             const int rec = first + q;
             float t, u, v;
             if (!tri_test(B::oo, B::od, s.sh4_tris + 3 * (size_t)rec, t, u, v)) continue;
-            bool better = t < best_t;
-            if (fmaxf(t, best_t) <= fminf(t, best_t) * kSh4CullPast && found()) {
+            if (t > best_t) {
+                second_t = fminf(second_t, t);
+                continue;
+            }
+            if (t == best_t && found()) {
                 const int ra = __ldg(&s.sh4_inst_rank[rec_inst(s, rec, cur_inst)]);
                 const int rb = __ldg(&s.sh4_inst_rank[rec_inst(s, best_rec, best_inst)]);
-                const bool first = ra < rb || (ra == rb && rec_tri(s, rec) < rec_tri(s, best_rec));
-                if (t == best_t)
-                    better = first;
-                else if (better != first)  // the farther of the two is met first
-                    second_t = better ? best_t : fminf(second_t, t);
+                if (!(ra < rb || (ra == rb && rec_tri(s, rec) < rec_tri(s, best_rec)))) continue;
+            } else {
+                second_t = best_t;
             }
-            if (better) {
-                best_t = t;
-                best_u = u;
-                best_v = v;
-                best_rec = rec;
-                best_inst = cur_inst;
-            }
+            best_t = t;
+            best_u = u;
+            best_v = v;
+            best_rec = rec;
+            best_inst = cur_inst;
         }
         B::next();
     }

@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kTraceThreads, kMinBlocks) trace_both4_kernel(
 // the terrain), so they get no list and no kernel of their own: the two kernels took 208 us of
 // the four rounds of a 256 x 256 path-traced box, this one takes 23. Surfaces within a few units
 // in the last place of each other reject more: a room's walls four times over, 0 to 3 units
-// apart, 1080p: RIS with all rays 7.65 ms (6.84 with the list), path tracing at depth 4 6.0 (7.4);
+// apart, 1080p: RIS with all rays 7.5 ms (6.85 with the list), path tracing at depth 4 5.95 (7.4);
 // walls twice over are no slower than with it. Walking a block's rejected entries side by side
 // was slower still (8.46). A miss needs no check: the SAH trees' boxes hold every triangle, so
 // the reference walk finds no hit either.
