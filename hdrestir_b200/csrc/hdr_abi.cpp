@@ -335,6 +335,7 @@ hdr_status ensure_buffer(hdr_ctx *c, const char *name, size_t bytes, void **out)
     hdr_status st = frame_alloc(c, nb, bytes);
     if (st != HDR_OK) return st;
     if (bytes) HDR_CUDA(cudaMemsetAsync(nb.ptr, 0, bytes, c->stream));
+    it = c->buffers.find(name);  // (again: making room may have given it back)
     if (it != c->buffers.end()) {
         const size_t keep = std::min(bytes, it->second.bytes);
         if (keep) HDR_CUDA(cudaMemcpyAsync(nb.ptr, it->second.ptr, keep, cudaMemcpyDeviceToDevice, c->stream));
@@ -2163,6 +2164,10 @@ hdr_status hdr_upscale(hdr_ctx *c, const char *name, int32_t components, int32_t
     DevBuf nb;
     hdr_status st = frame_alloc(c, nb, (size_t)dst_w * dst_h * components * sizeof(float));
     if (st != HDR_OK) return st;
+    if ((it = c->buffers.find(name)) == c->buffers.end()) {  // given back to make room
+        frame_free(c, nb);
+        return fail(HDR_ENOMEM, "no room to upscale '%s'", name);
+    }
     if (hdr::launch_upscale((const float *)it->second.ptr, (float *)nb.ptr, components, src_w, src_h, dst_w, dst_h,
                             c->tune.sm_count, c->stream) < 0) {
         frame_free(c, nb);

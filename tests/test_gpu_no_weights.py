@@ -80,3 +80,29 @@ def test_frames_without_room_for_the_weights(scene, form):
         assert np.array_equal(a.view(np.uint8 if a.dtype == np.uint8 else np.uint32)[~nan],
                               b.view(np.uint8 if b.dtype == np.uint8 else np.uint32)[~nan])
     assert any(np.nan_to_num(np.abs(a[:, :3])).sum() > 0 for a in want if a.ndim == 2)
+
+
+def test_replacing_the_weights_themselves_when_they_give_way():
+    """A buffer of that name whose larger replacement only fits once the old one is given back."""
+    from hdrestir_b200.context import Context
+    sc, cam = SCENES["boxes"](48, 40)
+    ris = dict(candidate_count=16, use_reservoir=True, max_depth=1)
+    done = 0
+    for budget in np.linspace(2 << 20, 6 << 20, 60).astype(int):
+        with Context(device=0, hbm_budget=int(budget)) as ctx:
+            try:
+                ctx.upload_scene(sc)
+                ctx.raycast(cam, 0)
+                ctx.ris_path_trace(cam, 0, **ris)
+                held = ctx.buffer_size("__wave_nee_weight")
+            except abi.HdrError:
+                continue
+            try:
+                ctx.upload("__wave_nee_weight", np.zeros(held + 4096, np.uint8))
+                done += 1
+                assert ctx.buffer_size("__wave_nee_weight") == held + 4096
+            except abi.HdrError:
+                pass
+            ctx.ris_path_trace(cam, 1, **ris)
+            ctx.synchronize()
+    assert done > 0
